@@ -717,8 +717,13 @@ int decode_planned(const pkv_decode_plan* plan, const void* q, const void* kc, c
     st = launch_tma_cluster<T>(a, plan->cluster, static_cast<cudaStream_t>(stream), &launched);
     if (st != PKV_OK || launched) return st;
   }
+  // Work units, or their upper bound when the plan was made on the device.  The TMA kernel turns them into
+  // resident blocks of warps itself; the kernels that give a unit a whole block (and stride over the rest) are
+  // capped at four blocks per SM when the count is only a bound.  (Capping the UNITS at that number, whatever
+  // the kernel, leaves a device-made plan on 148 of the 444 resident blocks of the TMA kernel: a step of 22
+  // layers over 128 sequences of 650 keys, 32 query / 4 kv heads, took 809 us that way and takes 432.)
   long long blocks = static_cast<long long>(plan->n_items) * plan->kv_heads;
-  if (!plan->exact && blocks > persistent_grid()) blocks = persistent_grid();
+  if (!plan->exact && !tma_path<T>(a) && blocks > persistent_grid()) blocks = persistent_grid();
   if (blocks > 0x7fffffffll) blocks = 0x7fffffffll;
   return launch_decode<T>(a, static_cast<int>(blocks), static_cast<cudaStream_t>(stream), (plan->reserved & 1) != 0);
 }
