@@ -42,6 +42,7 @@ struct StepPackArgs {
   int tables_cap;
   int32_t* table_offset;    // [n_slices] at most
   int32_t* counts;          // [4] = n_tokens, n_seqs, n_table, status bits
+  int hash_log2;            // places of the row table: 1 << hash_log2 >= 2 n_slices
 };
 
 // Exclusive scan of three values per item over up to kMaxSlices items held kPerThread per thread.
@@ -83,44 +84,78 @@ __device__ __forceinline__ void block_scan3(int (&a)[kPerThread], int (&b)[kPerT
   tot[0] = warp_tot[32][0]; tot[1] = warp_tot[32][1]; tot[2] = warp_tot[32][2];
 }
 
+// Sequences of the step by row: an open-addressing table in shared memory, row -> first slice that names it.
+// Twice as many places as slices (a power of two), multiplicative hashing, linear probing.
+__device__ __forceinline__ uint32_t hash_row(int row, int hash_log2) {
+  return (static_cast<uint32_t>(row) * 2654435769u) >> (32 - hash_log2);
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+// One cluster of blocks.  The tables' updates and the outputs are dealt over all of them; the numbering
+// of the sequences (a look-up per slice and three scans) is done by every block for itself, which costs no
+// more than handing it over would.  Latency is all there is to it: a step of 128 sequences moves 30 KB.
+// Finding a slice's sequence by walking the slices before it made this launch 42 us for 128 decode slices
+// (one block, two walks of up to n_slices dependent steps); with the table and one slice per warp it is 8.
 __global__ void __launch_bounds__(kThreads, 1) step_pack_kernel(const StepPackArgs a) {
   extern __shared__ int32_t sm[];
-  int32_t* s_row = sm;                        // [kMaxSlices] row of slice i (-1: invalid)
-  int32_t* s_tok = sm + kMaxSlices;           // first packed token of slice i
-  int32_t* s_idx = sm + 2 * kMaxSlices;       // step-local sequence number of slice i
-  int32_t* s_off = sm + 3 * kMaxSlices;       // where its table starts in `tables` (of its first appearance)
+  int32_t* s_row = sm;                        // [n_slices] row of slice i (-1: invalid)
+  int32_t* s_start = s_row + a.n_slices;      // its first position
+  int32_t* s_len = s_start + a.n_slices;      // its length
+  int32_t* s_nb = s_len + a.n_slices;         // blocks in its row's table
+  int32_t* s_tok = s_nb + a.n_slices;         // first packed token of slice i
+  int32_t* s_idx = s_tok + a.n_slices;        // step-local sequence number of slice i
+  int32_t* s_off = s_idx + a.n_slices;        // where its table starts in `tables` (-1 - that: not its first appearance)
+  int32_t* h_row = s_off + a.n_slices;        // [1 << hash_log2] row held by a place (-1: free)
+  int32_t* h_first = h_row + (1 << a.hash_log2);
   __shared__ int warp_tot[33][3];
-  __shared__ int s_status;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_status = 0;
+  const int n_blocks = gridDim.x, rank = blockIdx.x;      // one cluster: the grid is the cluster
+  const int gtid = rank * kThreads + tid, gthreads = n_blocks * kThreads;
+  for (int i = tid; i < (1 << a.hash_log2); i += kThreads) { h_row[i] = -1; h_first[i] = 0x7fffffff; }
   // No early release of the dependents: the kernels behind this one read the arrays it writes before
   // their own griddepcontrol.wait (they treat the step's index arrays as complete from the start).
   pdl_wait();
+  if (gtid == 0) a.counts[3] = 0;
 
   // ---- 0. bring the resident tables up to date: releases first, then appended blocks ----
-  for (int u = tid; u < a.n_updates; u += kThreads) {
+  bool bad_row = false;
+  for (int u = gtid; u < a.n_updates; u += gthreads) {
     const int row = a.updates[3 * u], idx = a.updates[3 * u + 1];
-    if (row < 0 || row >= a.max_rows) { atomicOr(&s_status, kStBadRow); continue; }
+    if (row < 0 || row >= a.max_rows) { bad_row = true; continue; }
     if (idx < 0) a.seq_nblocks[row] = 0;
   }
-  __syncthreads();
-  for (int u = tid; u < a.n_updates; u += kThreads) {
+  // ---- 1. slices -> shared memory, and the first slice of each row ----
+  for (int i = tid; i < a.n_slices; i += kThreads) {
+    int row = a.slices[3 * i];
+    s_start[i] = a.slices[3 * i + 1];
+    s_len[i] = max(a.slices[3 * i + 2], 0);
+    if (row < 0 || row >= a.max_rows) { bad_row = true; row = -1; }
+    s_row[i] = row;
+  }
+  cluster_barrier();                                        // releases, the zeroed status; this block's table and slices
+  for (int u = gtid; u < a.n_updates; u += gthreads) {
     const int row = a.updates[3 * u], idx = a.updates[3 * u + 1], blk = a.updates[3 * u + 2];
     if (row < 0 || row >= a.max_rows || idx < 0) continue;
-    if (idx >= a.table_stride) { atomicOr(&s_status, kStBadRow); continue; }
+    if (idx >= a.table_stride) { bad_row = true; continue; }
     a.seq_tables[static_cast<size_t>(row) * a.table_stride + idx] = blk;
     atomicMax(&a.seq_nblocks[row], idx + 1);
   }
-  __threadfence_block();
-  __syncthreads();
-
-  // ---- 1. slices -> shared memory ----
+  if (bad_row) atomicOr(&a.counts[3], kStBadRow);
   for (int i = tid; i < a.n_slices; i += kThreads) {
-    int row = a.slices[3 * i];
-    if (row < 0 || row >= a.max_rows) { atomicOr(&s_status, kStBadRow); row = -1; }
-    s_row[i] = row;
+    const int row = s_row[i];
+    if (row < 0) continue;
+    uint32_t h = hash_row(row, a.hash_log2);
+    for (;;) {                                              // ends: there are more places than rows
+      const int seen = atomicCAS(&h_row[h], -1, row);
+      if (seen == -1 || seen == row) break;
+      h = (h + 1) & ((1u << a.hash_log2) - 1);
+    }
+    atomicMin(&h_first[h], i);
   }
-  __syncthreads();
+  cluster_barrier();                                        // the updated tables, everywhere
 
   // ---- 2. first appearance of each slice's sequence, then three exclusive scans ----
   int v_len[kPerThread], v_uniq[kPerThread], v_nb[kPerThread], first[kPerThread];
@@ -131,12 +166,15 @@ __global__ void __launch_bounds__(kThreads, 1) step_pack_kernel(const StepPackAr
     first[k] = i;
     if (i < a.n_slices && s_row[i] >= 0) {
       const int row = s_row[i];
-      for (int j = 0; j < i; ++j)
-        if (s_row[j] == row) { first[k] = j; break; }
-      v_len[k] = max(a.slices[3 * i + 2], 0);
+      uint32_t h = hash_row(row, a.hash_log2);
+      while (h_row[h] != row) h = (h + 1) & ((1u << a.hash_log2) - 1);
+      first[k] = h_first[h];
+      v_len[k] = s_len[i];
+      const int nb = __ldcg(a.seq_nblocks + row);           // written by any block of the cluster
+      s_nb[i] = nb;
       if (first[k] == i) {
         v_uniq[k] = 1;
-        v_nb[k] = a.seq_nblocks[row];
+        v_nb[k] = nb;
       }
     }
   }
@@ -157,49 +195,52 @@ __global__ void __launch_bounds__(kThreads, 1) step_pack_kernel(const StepPackAr
     const int i = tid * kPerThread + k;
     if (i < a.n_slices && first[k] != i) {   // a later slice of a sequence takes its first slice's number
       s_idx[i] = s_idx[first[k]];
-      s_off[i] = s_off[first[k]];
+      s_off[i] = -1;
     }
   }
   const int n_tokens = tot[0], n_seqs = tot[1], n_table = tot[2];
-  if (n_tokens > a.tokens_cap) atomicOr(&s_status, kStTokensCap);
-  if (n_table > a.tables_cap) atomicOr(&s_status, kStTablesCap);
-  __syncthreads();
   const bool fits = n_tokens <= a.tokens_cap && n_table <= a.tables_cap;
+  __syncthreads();
 
-  // ---- 3. outputs: a warp per slice ----
+  // ---- 3. outputs: a warp per slice, dealt over the cluster ----
+  bool beyond = false;
   if (fits) {
-    for (int i = warp; i < a.n_slices; i += kThreads / 32) {
+    for (int i = warp * n_blocks + rank; i < a.n_slices; i += n_blocks * (kThreads / 32)) {
       const int row = s_row[i];
       if (row < 0) continue;
-      const int start = a.slices[3 * i + 1], len = max(a.slices[3 * i + 2], 0);
-      const int nb = a.seq_nblocks[row];
+      const int start = s_start[i], len = s_len[i], nb = s_nb[i];
       const int32_t* tbl = a.seq_tables + static_cast<size_t>(row) * a.table_stride;
       const int base = s_tok[i], idx = s_idx[i], off = s_off[i];
-      bool first_here = true;
-      for (int j = 0; j < i; ++j)           // warp-uniform; S is small
-        if (s_row[j] == row) { first_here = false; break; }
-      if (first_here) {
+      if (off >= 0) {
         if (lane == 0) a.table_offset[idx] = off;
-        for (int b = lane; b < nb; b += 32) a.tables[off + b] = tbl[b];
+        for (int b0 = lane; b0 < nb; b0 += 128) {           // four entries in flight per lane
+          int32_t e[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) e[u] = b0 + 32 * u < nb ? __ldcg(tbl + b0 + 32 * u) : 0;
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (b0 + 32 * u < nb) a.tables[off + b0 + 32 * u] = e[u];
+        }
       }
       for (int t = lane; t < len; t += 32) {
         const int pos = start + t;
         const int bi = pos / a.block_size;
         int slot = 0;
-        if (pos < 0 || bi >= nb) atomicOr(&s_status, kStPosBeyondTable);
-        else slot = tbl[bi] * a.block_size + (pos - bi * a.block_size);
+        if (pos < 0 || bi >= nb) beyond = true;
+        else slot = __ldcg(tbl + bi) * a.block_size + (pos - bi * a.block_size);
         a.positions[base + t] = pos;
         a.token_seq[base + t] = idx;
         a.slots[base + t] = slot;
       }
     }
   }
-  __syncthreads();
-  if (tid == 0) {
+  if (beyond) atomicOr(&a.counts[3], kStPosBeyondTable);
+  if (gtid == 0) {
     a.counts[0] = n_tokens;
     a.counts[1] = n_seqs;
     a.counts[2] = n_table;
-    a.counts[3] = s_status;
+    const int st = (n_tokens > a.tokens_cap ? kStTokensCap : 0) | (n_table > a.tables_cap ? kStTablesCap : 0);
+    if (st) atomicOr(&a.counts[3], st);
   }
 }
 
@@ -227,15 +268,33 @@ extern "C" int pkv_step_pack_device(const int32_t* d_updates, int n_updates, con
   a.max_rows = max_rows; a.table_stride = table_stride; a.block_size = block_size;
   a.slots = d_slots; a.token_seq = d_token_seq; a.positions = d_positions; a.tokens_cap = tokens_cap;
   a.tables = d_tables; a.tables_cap = tables_cap; a.table_offset = d_table_offset; a.counts = d_counts;
-  constexpr int smem = 4 * kMaxSlices * static_cast<int>(sizeof(int32_t));
+  a.hash_log2 = 5;
+  while ((1 << a.hash_log2) < 2 * n_slices) ++a.hash_log2;
+  const size_t smem = sizeof(int32_t) * (7 * static_cast<size_t>(n_slices) + 2 * (static_cast<size_t>(1) << a.hash_log2));
+  constexpr int kMaxSmem = static_cast<int>(sizeof(int32_t)) * (7 * kMaxSlices + 4 * kMaxSlices);
   static thread_local int configured_device = -1;
   int dev = 0;
   cudaGetDevice(&dev);
   if (configured_device != dev) {
-    const cudaError_t e = cudaFuncSetAttribute(step_pack_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return fail(PKV_E_CUDA, "%s: cannot reserve %d bytes of shared memory: %s", fn, smem, cudaGetErrorString(e));
+    const cudaError_t e = cudaFuncSetAttribute(step_pack_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+    if (e != cudaSuccess) return fail(PKV_E_CUDA, "%s: cannot reserve %d bytes of shared memory: %s", fn, kMaxSmem, cudaGetErrorString(e));
     configured_device = dev;
   }
-  launch_pdl(step_pack_kernel, dim3(1), dim3(kThreads), smem, static_cast<cudaStream_t>(stream), a);
+  // Enough blocks that every slice gets a warp of its own, up to the largest portable cluster.
+  const int blocks = n_slices <= 32 && n_updates <= 2 * kThreads ? 1 : n_slices <= 64 ? 2 : n_slices <= 128 ? 4 : 8;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = blocks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, step_pack_kernel, a);
   return check_launch("step_pack_kernel");
 }

@@ -128,3 +128,26 @@ def test_problems_are_reported_in_the_status_word(pkv, torch_cuda):
         packer.pack([(7, 0, 1)], check=True)              # no such row
     assert packer.pack([], check=True) == 0
     assert packer.counts.cpu().numpy().tolist() == [0, 0, 0, 0]
+
+
+@pytest.mark.parametrize("n_slices", [1, 31, 32, 33, 64, 65, 128, 129, 1025, 4096])
+def test_slice_counts_around_the_launch_shapes(pkv, orc, torch_cuda, n_slices):
+    """One, two, four and eight blocks, the largest step, and the row table's collisions: rows are
+    spread over a large store and a third of the slices return to a sequence seen before."""
+    rng = np.random.default_rng(n_slices)
+    bs, max_rows = 16, 50000
+    packer = pkv.DeviceStepPacker(max_rows, 40, bs, max_tokens=4 * n_slices, max_table_entries=40 * n_slices)
+    distinct = max(1, (2 * n_slices) // 3)
+    rows = rng.choice(max_rows, size=distinct, replace=False)
+    tables = {int(r): rng.integers(0, 9999, size=int(rng.integers(1, 41))).astype(np.int32) for r in rows}
+    for r, t in tables.items():
+        packer.set_table(r, t)
+    picks = np.concatenate([rows, rng.choice(rows, size=n_slices - distinct)])
+    rng.shuffle(picks)
+    slices = []
+    for r in picks:
+        cap = tables[int(r)].size * bs
+        n = int(rng.integers(1, 5))
+        slices.append((int(r), int(rng.integers(0, cap - n + 1)), n))
+    n = packer.pack(slices)
+    check(packer, oracle_pack(orc, tables, slices, bs), n)
