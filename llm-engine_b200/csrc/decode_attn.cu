@@ -99,199 +99,237 @@ struct RouteArgs {
   int* dims;        // [4] out: runs, 128-row tiles of the longest run, prefill work items, decode tokens
 };
 
-__device__ void route_phase(const int* __restrict__ token_pos, int n, const RouteArgs& r, int* sm_scan, int* sm_misc) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  auto is_start = [&](int t) {
-    return t == 0 || r.token_seq[t] != r.token_seq[t - 1] || token_pos[t] != token_pos[t - 1] + 1;
-  };
-  // 1. running maximum of the start indices = first token of each token's run
-  int carry = 0;
-  for (int base = 0; base < n; base += kPlanThreads) {
-    const int t = base + tid;
-    int v = (t < n && is_start(t)) ? t : -1;
+// Inclusive scans over the block's threads, one value each (sum, or maximum).  `sm` holds one word per
+// warp and is free for the next scan only after another barrier; *total receives the block's result.
+struct ScanSum { static __device__ __forceinline__ int id() { return 0; } static __device__ __forceinline__ int op(int a, int b) { return a + b; } };
+struct ScanMax { static __device__ __forceinline__ int id() { return -1; } static __device__ __forceinline__ int op(int a, int b) { return max(a, b); } };
+template <typename Op>
+__device__ __forceinline__ int warp_scan(int v, int lane) {
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int x = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o) v = max(v, x);
-    }
-    if (lane == 31) sm_scan[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-      int a = sm_scan[lane];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int x = __shfl_up_sync(0xffffffffu, a, o);
-        if (lane >= o) a = max(a, x);
-      }
-      sm_scan[lane] = a;
-    }
-    __syncthreads();
-    v = max(v, max(warp ? sm_scan[warp - 1] : -1, carry));
-    if (t < n) r.run_start[t] = v;
-    carry = max(carry, sm_scan[kPlanThreads / 32 - 1]);
-    __syncthreads();
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v = Op::op(v, x);
   }
-  // 2. the last token of a run stores the run's length at its first token
-  for (int t = tid; t < n; t += kPlanThreads) {
-    if (t == n - 1 || is_start(t + 1)) {
-      const int rs = r.run_start[t];
-      r.run_len[rs] = t - rs + 1;
-    }
-  }
-  if (tid == 0) { sm_misc[0] = 0; sm_misc[1] = 0; sm_misc[2] = 0; }   // runs so far, longest run, decode tokens
+  return v;
+}
+template <typename Op>
+__device__ __forceinline__ int block_scan(int v, int* sm, int* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  v = warp_scan<Op>(v, lane);
+  if (lane == 31) sm[warp] = v;
   __syncthreads();
-  // 3. effective lengths and the records of the long runs, in packed order
-  for (int base = 0; base < n; base += kPlanThreads) {
-    const int t = base + tid;
-    int flag = 0, len = 0;
-    if (t < n) {
-      const int rs = r.run_start[t];
-      len = r.run_len[rs];
-      const bool long_run = len >= r.min_run;
-      r.eff_len[t] = long_run ? 0 : max(token_pos[t], 0) + 1;
-      flag = (long_run && rs == t) ? 1 : 0;
-      if (!long_run) atomicAdd(&sm_misc[2], 1);
-    }
-    int sc = flag;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int x = __shfl_up_sync(0xffffffffu, sc, o);
-      if (lane >= o) sc += x;
-    }
-    if (lane == 31) sm_scan[warp] = sc;
-    __syncthreads();
-    if (warp == 0) {
-      int a = sm_scan[lane];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int x = __shfl_up_sync(0xffffffffu, a, o);
-        if (lane >= o) a += x;
-      }
-      sm_scan[lane] = a;
-    }
-    __syncthreads();
-    if (flag) {
-      const int i = sm_misc[0] + (warp ? sm_scan[warp - 1] : 0) + sc - 1;
-      r.q_start[i] = t;
-      r.q_len[i] = len;
-      r.ctx_len[i] = max(token_pos[t], 0);
-      r.tbl_off[i] = r.table_offset[r.token_seq[t]];
-      atomicMax(&sm_misc[1], len);
-    }
-    __syncthreads();
-    if (tid == 0) sm_misc[0] += sm_scan[kPlanThreads / 32 - 1];
-    __syncthreads();
-  }
-  if (tid == 0) {
-    const int tiles = (sm_misc[1] + 127) / 128;
-    r.dims[0] = sm_misc[0];
-    r.dims[1] = tiles;
-    r.dims[2] = sm_misc[0] * tiles * r.q_heads;
-    r.dims[3] = sm_misc[2];
-  }
-  __syncthreads();
+  const int w = warp_scan<Op>(sm[lane], lane);        // every warp scans the 32 warp totals for itself: one barrier
+  const int before = __shfl_sync(0xffffffffu, w, max(warp - 1, 0));
+  *total = __shfl_sync(0xffffffffu, w, 31);
+  return warp ? Op::op(before, v) : v;
 }
 
+// One block: all of it is latency (a step of 600 tokens reads 5 KB), so a step of up to kPlanThreads
+// tokens keeps everything a token needs in its thread's registers and run lengths in shared memory, and
+// every scan costs one barrier.
+// (The kernel it replaces made one histogram per chunk candidate and five passes with three to five barriers
+// each: 6.8 us for 48 tokens, 7.9 us for 620.)
 template <bool ROUTE>
-__global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __restrict__ token_pos, int n_tokens,
-                                                                    int kv_heads, long long extra_budget,
-                                                                    int wave_ctas, int forced_chunk,
-                                                                    PlanHeader* header, TokSplit* tok_split,
-                                                                    int* counters, WorkItem* items, const RouteArgs route) {
-  __shared__ unsigned long long sm_items[kNumChunkCandidates];
-  __shared__ int sm_chunk;
-  __shared__ int sm_scan_items[kPlanThreads / 32], sm_scan_parts[kPlanThreads / 32];
-  __shared__ int sm_carry_items, sm_carry_parts;
-  __shared__ int sm_misc[4];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if constexpr (ROUTE) route_phase(token_pos, n_tokens, route, sm_scan_items, sm_misc);
+__global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __restrict__ token_pos, int n_tokens, int max_shares,
+                                                                    int forced_chunk, int kv_heads, PlanHeader* header,
+                                                                    TokSplit* tok_split, int* counters, WorkItem* items,
+                                                                    const RouteArgs r) {
+  extern __shared__ int sm_first[];                       // [max_shares + 1] first item of every share
+  __shared__ int sm_scan[8][kPlanThreads / 32];
+  __shared__ int sm_len[kPlanThreads];                    // run lengths of a step of up to kPlanThreads tokens
+  __shared__ int sm_start[kPlanThreads + 1];              // ... and whether a run starts at a token
+  __shared__ int sm_misc[4];                              // long runs, longest of them, tokens of none
+  const int tid = threadIdx.x;
+  const bool small = n_tokens <= kPlanThreads;
+  // the next launch on the stream is the prefill kernel, which waits for this one before it reads anything
+  if constexpr (ROUTE) pdl_launch_dependents();
+  if (tid < 4) sm_misc[tid] = 0;
+  for (int i = tid; i <= max_shares; i += kPlanThreads) sm_first[i] = 0x7fffffff;
+  if (tid == 0) sm_start[n_tokens < kPlanThreads ? n_tokens : kPlanThreads] = 1;
+  pdl_wait();
+  if (tid == 0) counters[0] = 0;
+
   // keys the decode path handles for token t: position + 1, or 0 for a token the router gave to the prefill kernel
+  int my_len = 0;                                          // of token tid, when the step is small
+  if constexpr (ROUTE) {
+    auto is_start = [&](int t) {
+      return t == 0 || r.token_seq[t] != r.token_seq[t - 1] || token_pos[t] != token_pos[t - 1] + 1;
+    };
+    if (small) {
+      const int t = tid;
+      int pos = 0, seq = -1;
+      bool start = false;
+      if (t < n_tokens) {
+        pos = token_pos[t];
+        seq = r.token_seq[t];
+        start = t == 0 || r.token_seq[t - 1] != seq || token_pos[t - 1] + 1 != pos;
+        sm_start[t] = start;
+      }
+      int tot;
+      const int rs = block_scan<ScanMax>(start ? t : -1, sm_scan[0], &tot);
+      if (t < n_tokens && sm_start[t + 1]) sm_len[rs] = t - rs + 1;   // the run's last token
+      __syncthreads();
+      int flag = 0, len = 0;
+      if (t < n_tokens) {
+        len = sm_len[rs];
+        const bool long_run = len >= r.min_run;
+        my_len = long_run ? 0 : max(pos, 0) + 1;
+        flag = long_run && start;
+      }
+      const int i = block_scan<ScanSum>(flag, sm_scan[1], &tot) - 1;
+      if (flag) {
+        r.q_start[i] = t;
+        r.q_len[i] = len;
+        r.ctx_len[i] = max(pos, 0);
+        r.tbl_off[i] = r.table_offset[seq];
+        atomicMax(&sm_misc[1], len);
+      }
+      const int n_dec = __syncthreads_count(my_len > 0);
+      if (tid == 0) { sm_misc[0] = tot; sm_misc[2] = n_dec; }
+    } else {
+      // 1. running maximum of the start indices = first token of each token's run
+      int carry = -1;
+      for (int base = 0; base < n_tokens; base += kPlanThreads) {
+        const int t = base + tid;
+        int tot;
+        const int v = max(block_scan<ScanMax>((t < n_tokens && is_start(t)) ? t : -1, sm_scan[0], &tot), carry);
+        if (t < n_tokens) r.run_start[t] = v;
+        carry = max(carry, tot);
+        __syncthreads();
+      }
+      // 2. the last token of a run stores the run's length at its first token
+      for (int t = tid; t < n_tokens; t += kPlanThreads) {
+        if (t == n_tokens - 1 || is_start(t + 1)) {
+          const int rs = r.run_start[t];
+          r.run_len[rs] = t - rs + 1;
+        }
+      }
+      __syncthreads();
+      // 3. effective lengths and the records of the long runs, in packed order
+      int runs = 0;
+      for (int base = 0; base < n_tokens; base += kPlanThreads) {
+        const int t = base + tid;
+        int flag = 0, len = 0, eff = 0;
+        if (t < n_tokens) {
+          const int rs = r.run_start[t];
+          len = r.run_len[rs];
+          const bool long_run = len >= r.min_run;
+          eff = long_run ? 0 : max(token_pos[t], 0) + 1;
+          r.eff_len[t] = eff;
+          flag = long_run && rs == t;
+        }
+        int tot;
+        const int i = runs + block_scan<ScanSum>(flag, sm_scan[1], &tot) - 1;
+        if (flag) {
+          r.q_start[i] = t;
+          r.q_len[i] = len;
+          r.ctx_len[i] = max(token_pos[t], 0);
+          r.tbl_off[i] = r.table_offset[r.token_seq[t]];
+          atomicMax(&sm_misc[1], len);
+        }
+        runs += tot;
+        const int n_dec = __syncthreads_count(eff > 0);
+        if (tid == 0) { sm_misc[0] = runs; sm_misc[2] += n_dec; }
+      }
+    }
+  } else {
+    if (tid < n_tokens) my_len = max(token_pos[tid], 0) + 1;
+  }
   auto length_of = [&](int t) {
-    if constexpr (ROUTE) return route.eff_len[t];
+    if (small) return my_len;
+    if constexpr (ROUTE) return r.eff_len[t];
     return max(token_pos[t], 0) + 1;
   };
-  if (tid < kNumChunkCandidates) sm_items[tid] = 0ull;
-  if (tid == 0) { sm_carry_items = 0; sm_carry_parts = 0; }
-  __syncthreads();
-  {
-    unsigned long long loc[kNumChunkCandidates];
-#pragma unroll
-    for (int j = 0; j < kNumChunkCandidates; ++j) loc[j] = 0ull;
-    for (int t = tid; t < n_tokens; t += kPlanThreads) {
-      const int L = length_of(t);
-#pragma unroll
-      for (int j = 0; j < kNumChunkCandidates; ++j) loc[j] += static_cast<unsigned>((L + (kMinChunk << j) - 1) / (kMinChunk << j));
-    }
-#pragma unroll
-    for (int j = 0; j < kNumChunkCandidates; ++j) {
-      unsigned long long v = loc[j];
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0 && v) atomicAdd(&sm_items[j], v);
-    }
-  }
-  __syncthreads();
-  if (tid == 0) {
-    long long items_at[kNumChunkCandidates];
-    for (int j = 0; j < kNumChunkCandidates; ++j) items_at[j] = static_cast<long long>(sm_items[j]);
-    sm_chunk = choose_chunk(items_at, n_tokens, kv_heads, extra_budget, wave_ctas, forced_chunk);
-  }
-  __syncthreads();
-  const int chunk = sm_chunk;
 
+  // padded keys of the whole step -> how it is cut
+  long long total = 0;
+  long long my_begin = 0;                                  // where token tid begins in the laid-out step, when it is small
+  if (small) {
+    int tot;
+    const int p = share_padded(my_len) / kShareSlab;       // scanned in slabs: 32 bits hold 2^36 keys
+    my_begin = static_cast<long long>(block_scan<ScanSum>(p, sm_scan[2], &tot) - p) * kShareSlab;
+    total = static_cast<long long>(tot) * kShareSlab;
+  } else {
+    long long loc = 0;
+    for (int t = tid; t < n_tokens; t += kPlanThreads) loc += share_padded(length_of(t));
+    for (int o = 16; o > 0; o >>= 1) loc += __shfl_xor_sync(0xffffffffu, loc, o);
+    __shared__ long long sm_tot[kPlanThreads / 32];
+    if ((tid & 31) == 0) sm_tot[tid >> 5] = loc;
+    __syncthreads();
+    for (int w = 0; w < kPlanThreads / 32; ++w) total += sm_tot[w];
+  }
+  const ShareRule rule = share_rule(total, max_shares, forced_chunk);
+
+  int n_items = 0, n_parts = 0;
+  long long carry_begin = 0;
   for (int base = 0; base < n_tokens; base += kPlanThreads) {
     const int t = base + tid;
-    int L = 0, ns = 0;
-    if (t < n_tokens) {
-      L = length_of(t);
-      ns = L == 0 ? 0 : (chunk > 0 ? (L + chunk - 1) / chunk : 1);
+    const int L = t < n_tokens ? length_of(t) : 0;
+    const int padded = share_padded(L);
+    int tot;
+    long long begin = my_begin;
+    if (!small) {
+      const int p = padded / kShareSlab;
+      begin = carry_begin + static_cast<long long>(block_scan<ScanSum>(p, sm_scan[2], &tot) - p) * kShareSlab;
+      carry_begin += static_cast<long long>(tot) * kShareSlab;
+    }
+    int ns = 0;
+    ShareCut cut{0, 0};
+    if (L > 0) {
+      if (rule.per > 0) {
+        cut = share_cuts(begin, padded, rule.per);
+        ns = cut.n + 1;
+      } else {
+        ns = rule.chunk > 0 ? (L + rule.chunk - 1) / rule.chunk : 1;
+      }
     }
     const int np = ns > 1 ? ns : 0;
-    // inclusive scans of ns and np across the block
-    int si = ns, sp = np;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int a = __shfl_up_sync(0xffffffffu, si, o), b = __shfl_up_sync(0xffffffffu, sp, o);
-      if (lane >= o) { si += a; sp += b; }
-    }
-    if (lane == 31) { sm_scan_items[warp] = si; sm_scan_parts[warp] = sp; }
-    __syncthreads();
-    if (warp == 0) {
-      int a = sm_scan_items[lane], b = sm_scan_parts[lane];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int x = __shfl_up_sync(0xffffffffu, a, o), y = __shfl_up_sync(0xffffffffu, b, o);
-        if (lane >= o) { a += x; b += y; }
-      }
-      sm_scan_items[lane] = a;
-      sm_scan_parts[lane] = b;
-    }
-    __syncthreads();
-    const int item0 = sm_carry_items + (warp ? sm_scan_items[warp - 1] : 0) + si - ns;
-    const int part0 = sm_carry_parts + (warp ? sm_scan_parts[warp - 1] : 0) + sp - np;
+    int tot_items, tot_parts;
+    const int item0 = n_items + block_scan<ScanSum>(ns, sm_scan[3], &tot_items) - ns;
+    const int part0 = n_parts + block_scan<ScanSum>(np, sm_scan[4], &tot_parts) - np;
     if (t < n_tokens) {
       tok_split[t] = TokSplit{part0, ns};
       for (int s = 0; s < ns; ++s) {
-        const int b = chunk > 0 ? s * chunk : 0;
-        const int len = chunk > 0 ? min(chunk, L - b) : L;
-        items[item0 + s] = WorkItem{t, b, len, ns > 1 ? part0 + s : -1};
+        int b, e;                                          // first key, end
+        if (rule.per > 0) {
+          const long long at = s ? cut.first + static_cast<long long>(s - 1) * rule.per : begin;
+          b = static_cast<int>(at - begin);
+          e = s < cut.n ? static_cast<int>(cut.first + static_cast<long long>(s) * rule.per - begin) : L;
+          atomicMin(&sm_first[share_of(at, rule.per, rule.n_shares)], item0 + s);
+        } else {
+          b = s * rule.chunk;
+          e = s + 1 < ns ? b + rule.chunk : L;
+        }
+        items[item0 + s] = WorkItem{t, b, e - b, ns > 1 ? part0 + s : -1};
       }
     }
-    __syncthreads();
-    if (tid == 0) {
-      sm_carry_items += sm_scan_items[kPlanThreads / 32 - 1];
-      sm_carry_parts += sm_scan_parts[kPlanThreads / 32 - 1];
-    }
-    __syncthreads();
+    n_items += tot_items;
+    n_parts += tot_parts;
+    if (!small) __syncthreads();                           // the scans' words, before the next round
   }
-  for (int i = tid; i < n_tokens * kv_heads; i += kPlanThreads) counters[i] = 0;
+  if (rule.n_shares > 0) {
+    __syncthreads();
+    int* first = reinterpret_cast<int*>(items + n_items);
+    for (int s = tid; s <= rule.n_shares; s += kPlanThreads) first[s] = s < rule.n_shares ? min(sm_first[s], n_items) : n_items;
+  }
   if (tid == 0) {
     header->magic = kPlanMagic;
-    header->n_items = sm_carry_items;
-    header->chunk = chunk;
+    header->n_items = n_items;
+    header->chunk = rule.per > 0 ? rule.per : rule.chunk;
     header->n_tokens = n_tokens;
-    header->n_parts = sm_carry_parts;
+    header->n_parts = n_parts;
     header->kv_heads = kv_heads;
-    header->pad[0] = header->pad[1] = 0;
+    header->n_shares = rule.n_shares;
+    header->pad = 0;
+  }
+  if constexpr (ROUTE) {
+    if (tid == 0) {
+      const int tiles = (sm_misc[1] + 127) / 128;
+      r.dims[0] = sm_misc[0];
+      r.dims[1] = tiles;
+      r.dims[2] = sm_misc[0] * tiles * r.q_heads;
+      r.dims[3] = sm_misc[2];
+    }
   }
 }
 
@@ -578,6 +616,7 @@ void fill_args(DecodeArgs& a, const void* q, const void* kc, const void* vc, con
   a.n_peers = 0; a.my_rank = 0; a.epoch = 0;
   a.new_k = nullptr; a.new_v = nullptr; a.slots = nullptr;
   a.host_err = nullptr;
+  a.wait_last = 0;
   a.pool_rows = 1ull << 30;
 }
 
@@ -603,6 +642,12 @@ int persistent_grid() {
   return sms * 4;
 }
 
+// Warps the attention kernel of this geometry keeps resident: what a step's keys are shared out over.
+int decode_workers(int q_heads, int kv_heads, int head_dim) {
+  (void)q_heads; (void)kv_heads;
+  return persistent_sms() * (head_dim == 128 ? 8 : 12);
+}
+
 // Budget of extra items for this workspace: what fits, capped by the target grid.
 int plan_budget(int n_tokens, int q_heads, int kv_heads, int head_dim, size_t workspace_bytes, WsLayout* w) {
   const int fit = ws_extra_for_bytes(n_tokens, q_heads, kv_heads, head_dim, workspace_bytes, max_extra(kv_heads));
@@ -622,21 +667,18 @@ int plan_device(const int* token_pos, int n_tokens, int q_heads, int kv_heads, i
   if (budget < 0)
     return fail(PKV_E_WORKSPACE, "pkv_decode_plan_device: workspace of %zu bytes cannot hold the plan for %d tokens", workspace_bytes, n_tokens);
   char* base = static_cast<char*>(workspace);
-  if (route)
-    decode_plan_kernel<true><<<1, kPlanThreads, 0, stream>>>(
-        token_pos, n_tokens, kv_heads, budget, tuning().wave_ctas, tuning().forced_chunk,
-        reinterpret_cast<PlanHeader*>(base), reinterpret_cast<TokSplit*>(base + w.off_tok),
-        reinterpret_cast<int*>(base + w.off_cnt), reinterpret_cast<WorkItem*>(base + w.off_items), *route);
-  else
-    decode_plan_kernel<false><<<1, kPlanThreads, 0, stream>>>(
-        token_pos, n_tokens, kv_heads, budget, tuning().wave_ctas, tuning().forced_chunk,
-        reinterpret_cast<PlanHeader*>(base), reinterpret_cast<TokSplit*>(base + w.off_tok),
-        reinterpret_cast<int*>(base + w.off_cnt), reinterpret_cast<WorkItem*>(base + w.off_items), RouteArgs{});
+  const int max_shares = max_shares_for(w.cap_extra < budget ? w.cap_extra : budget, decode_workers(q_heads, kv_heads, head_dim) / kv_heads);
+  const size_t smem = sizeof(int) * static_cast<size_t>(max_shares + 1);
+  auto kern = route ? decode_plan_kernel<true> : decode_plan_kernel<false>;
+  launch_pdl(kern, dim3(1), dim3(kPlanThreads), smem, stream, token_pos, n_tokens, max_shares, tuning().forced_chunk, kv_heads,
+             reinterpret_cast<PlanHeader*>(base), reinterpret_cast<TokSplit*>(base + w.off_tok),
+             reinterpret_cast<int*>(base + w.off_cnt), reinterpret_cast<WorkItem*>(base + w.off_items),
+             route ? *route : RouteArgs{});
   int st = check_launch("decode_plan_kernel");
   if (st != PKV_OK) return st;
   plan->n_tokens = n_tokens; plan->q_heads = q_heads; plan->kv_heads = kv_heads; plan->head_dim = head_dim;
   plan->chunk = -1;                      // decided on the device
-  plan->n_items = n_tokens + budget;     // upper bound
+  plan->n_items = n_tokens + budget;     // upper bound, of the items and of the shares
   plan->exact = 0;
   plan->reserved = 1;                    // tokens may have been split: run the merge
   return PKV_OK;
@@ -658,7 +700,7 @@ template <typename T>
 int decode_planned(const pkv_decode_plan* plan, const void* q, const void* kc, const void* vc, const int* bt,
                    const int* to, const int* ts, const int* tp, void* out, int block_size, float scale,
                    void* workspace, size_t workspace_bytes, pkv_stream stream, const PeerSetup* peers = nullptr,
-                   const FusedAppend* app = nullptr, bool may_allocate = true) {
+                   const FusedAppend* app = nullptr, bool may_allocate = true, bool wait_last = false) {
   const char* fn = peers ? "pkv_decode_attn_planned_peer" : (app ? "pkv_append_decode_attn_planned" : "pkv_decode_attn_planned");
   if (!plan) return fail(PKV_E_ARG, "%s: null plan", fn);
   if (plan->n_tokens <= 0) return PKV_OK;
@@ -676,6 +718,7 @@ int decode_planned(const pkv_decode_plan* plan, const void* q, const void* kc, c
   fill_args(a, q, kc, vc, bt, to, ts, tp, out, plan->n_tokens, plan->q_heads, plan->kv_heads, plan->head_dim, block_size, scale);
   attach_workspace(a, workspace, w);
   a.host_err = error_mirror(may_allocate);
+  a.wait_last = wait_last ? 1 : 0;
   if (plan->num_blocks > 0) a.pool_rows = static_cast<unsigned long long>(plan->num_blocks) * block_size;
   if (peers) {
     if constexpr (sizeof(T) != 2) return fail(PKV_E_UNSUPPORTED, "%s: the head-sharded exchange is for 16-bit outputs", fn);
@@ -820,14 +863,19 @@ int mixed_attn(const void* q, const void* kc, const void* vc, const int* bt, con
   st = plan_device(tp, n_tokens, q_heads, kv_heads, head_dim, workspace, dec_bytes, static_cast<cudaStream_t>(stream), &plan, &r);
   if (st != PKV_OK) return st;
   plan.num_blocks = num_blocks > 0 ? num_blocks : 0;
-  // decode tokens (and short runs) through the decode kernels; tokens of long runs are in no work item
-  st = decode_planned<T>(&plan, q, kc, vc, bt, to, ts, tp, out, block_size, scale, workspace, dec_bytes, stream);
-  if (st != PKV_OK) return st;
-  // the long runs through the tensor-core kernel, whose item counts come from the router
+  // The long runs through the tensor-core kernel, whose item counts come from the router; then decode tokens
+  // and short runs through the decode kernels (tokens of long runs are in no work item).  The prefill kernel
+  // lets the launch behind it start as soon as it has itself seen the plan complete, and the decode kernel,
+  // which shares no output with it, runs next to it (DecodeArgs::wait_last).  One after the other, a step of
+  // two 300-token chunks and 20 decode tokens took 42 us a layer.
   const int max_runs = n_tokens / min_run;
-  if constexpr (!IsF32<T>::value)
+  if constexpr (!IsF32<T>::value) {
     st = prefill_launch<T>(q, kc, vc, bt, r.tbl_off, r.q_start, r.q_len, r.ctx_len, out, n_tokens, max_runs, n_tokens,
                            q_heads, kv_heads, head_dim, block_size, num_blocks, scale, stream, r.dims, true);
+    if (st != PKV_OK) return st;
+  }
+  st = decode_planned<T>(&plan, q, kc, vc, bt, to, ts, tp, out, block_size, scale, workspace, dec_bytes, stream, nullptr, nullptr,
+                         true, true);
   return st;
 }
 
@@ -877,19 +925,30 @@ static int plan_host_image(const char* fn, const int* h_token_pos, int n_tokens,
   const int budget = plan_budget(n_tokens, q_heads, kv_heads, head_dim, workspace_bytes, &w);
   if (budget < 0) return fail(PKV_E_WORKSPACE, "%s: workspace of %zu bytes cannot hold the plan for %d tokens", fn, workspace_bytes, n_tokens);
 
-  long long items_at[kNumChunkCandidates] = {0};
+  long long total = 0;
+  int max_len = 0;
   for (int t = 0; t < n_tokens; ++t) {
     if (h_token_pos[t] < 0) return fail(PKV_E_ARG, "%s: token %d has negative position %d", fn, t, h_token_pos[t]);
-    const int L = h_token_pos[t] + 1;
-    for (int j = 0; j < kNumChunkCandidates; ++j) items_at[j] += (L + (kMinChunk << j) - 1) / (kMinChunk << j);
+    total += share_padded(h_token_pos[t] + 1);
+    max_len = std::max(max_len, h_token_pos[t] + 1);
   }
-  const int chunk = choose_chunk(items_at, n_tokens, kv_heads, budget, tuning().wave_ctas, tuning().forced_chunk);
+  const int max_shares = max_shares_for(budget, decode_workers(q_heads, kv_heads, head_dim) / kv_heads);
+  const ShareRule rule = share_rule(total, max_shares, tuning().forced_chunk);
+  const int chunk = rule.chunk;
   long long n_items = n_tokens;
-  if (chunk > 0) {
+  if (rule.per > 0) {
+    long long begin = 0;
+    for (int t = 0; t < n_tokens; ++t) {
+      const int padded = share_padded(h_token_pos[t] + 1);
+      n_items += share_cuts(begin, padded, rule.per).n;
+      begin += padded;
+    }
+  } else if (chunk > 0) {
     n_items = 0;
     for (int t = 0; t < n_tokens; ++t) n_items += (h_token_pos[t] + chunk) / chunk;
   }
-  const size_t image = w.off_items + sizeof(WorkItem) * static_cast<size_t>(n_items);
+  const size_t table = rule.n_shares > 0 ? sizeof(int) * static_cast<size_t>(rule.n_shares + 1) : 0;
+  const size_t image = w.off_items + sizeof(WorkItem) * static_cast<size_t>(n_items) + table;
   if (image > staging_bytes) return fail(PKV_E_WORKSPACE, "%s: staging buffer of %zu bytes is smaller than the %zu-byte plan image", fn, staging_bytes, image);
 
   char* img = static_cast<char*>(h_staging);
@@ -898,38 +957,61 @@ static int plan_host_image(const char* fn, const int* h_token_pos, int n_tokens,
   TokSplit* tsp = reinterpret_cast<TokSplit*>(img + w.off_tok);
   WorkItem* it = reinterpret_cast<WorkItem*>(img + w.off_items);
   int ni = 0, np = 0;
-  // Longest first: full-size chunks, then the ragged tails in decreasing length, so
-  // that dealing the list round-robin gives every worker about the same number of
-  // keys and the short units land at the end of the launch.  (Handing units out
-  // dynamically through an atomic counter was measured and was no faster.)
-  for (int t = 0; t < n_tokens; ++t) {
-    const int L = h_token_pos[t] + 1;
-    const int ns = chunk > 0 ? (L + chunk - 1) / chunk : 1;
-    tsp[t] = TokSplit{np, ns};
-    if (ns > 1) np += ns;
-    if (chunk > 0)
-      for (int s = 0; s + 1 < ns || (s < ns && L - s * chunk == chunk); ++s)
-        it[ni++] = WorkItem{t, s * chunk, chunk, ns > 1 ? tsp[t].part_base + s : -1};
+  if (rule.per > 0) {
+    int* first = reinterpret_cast<int*>(it + n_items);
+    long long begin = 0;
+    int share = -1;                                   // last share that has an item
+    for (int t = 0; t < n_tokens; ++t) {
+      const int L = h_token_pos[t] + 1;
+      const ShareCut cut = share_cuts(begin, share_padded(L), rule.per);
+      const int ns = cut.n + 1;
+      tsp[t] = TokSplit{np, ns};
+      for (int s = 0; s < ns; ++s) {
+        const long long at = s ? cut.first + static_cast<long long>(s - 1) * rule.per : begin;
+        const int b = static_cast<int>(at - begin);
+        const int e = s < cut.n ? static_cast<int>(cut.first + static_cast<long long>(s) * rule.per - begin) : L;
+        for (const int sh = share_of(at, rule.per, rule.n_shares); share < sh;) first[++share] = ni;
+        it[ni++] = WorkItem{t, b, e - b, ns > 1 ? np + s : -1};
+      }
+      if (ns > 1) np += ns;
+      begin += share_padded(L);
+    }
+    while (share < rule.n_shares) first[++share] = ni;
+  } else {
+    // Longest first: full-size chunks, then the ragged tails in decreasing length, so
+    // that dealing the list round-robin gives every worker about the same number of
+    // keys and the short units land at the end of the launch.  (Handing units out
+    // dynamically through an atomic counter was measured and was no faster.)
+    for (int t = 0; t < n_tokens; ++t) {
+      const int L = h_token_pos[t] + 1;
+      const int ns = chunk > 0 ? (L + chunk - 1) / chunk : 1;
+      tsp[t] = TokSplit{np, ns};
+      if (ns > 1) np += ns;
+      if (chunk > 0)
+        for (int s = 0; s + 1 < ns || (s < ns && L - s * chunk == chunk); ++s)
+          it[ni++] = WorkItem{t, s * chunk, chunk, ns > 1 ? tsp[t].part_base + s : -1};
+    }
+    const int n_full = ni;
+    for (int t = 0; t < n_tokens; ++t) {
+      const int L = h_token_pos[t] + 1;
+      const int ns = tsp[t].nsplits;
+      const int b = chunk > 0 ? (ns - 1) * chunk : 0;
+      const int len = L - b;
+      if (chunk > 0 && len == chunk) continue;  // already listed as a full chunk
+      it[ni++] = WorkItem{t, b, len, ns > 1 ? tsp[t].part_base + ns - 1 : -1};
+    }
+    std::stable_sort(it + n_full, it + ni, [](const WorkItem& x, const WorkItem& y) { return x.kv_len > y.kv_len; });
   }
-  const int n_full = ni;
-  for (int t = 0; t < n_tokens; ++t) {
-    const int L = h_token_pos[t] + 1;
-    const int ns = tsp[t].nsplits;
-    const int b = chunk > 0 ? (ns - 1) * chunk : 0;
-    const int len = L - b;
-    if (chunk > 0 && len == chunk) continue;  // already listed as a full chunk
-    it[ni++] = WorkItem{t, b, len, ns > 1 ? tsp[t].part_base + ns - 1 : -1};
-  }
-  std::stable_sort(it + n_full, it + ni, [](const WorkItem& x, const WorkItem& y) { return x.kv_len > y.kv_len; });
+  hd->n_shares = rule.n_shares;
+  hd->chunk = rule.per > 0 ? rule.per : chunk;
   hd->magic = kPlanMagic;
   hd->n_items = ni;
-  hd->chunk = chunk;
   hd->n_tokens = n_tokens;
   hd->n_parts = np;
   hd->kv_heads = kv_heads;
   *image_bytes = image;
   plan->n_tokens = n_tokens; plan->q_heads = q_heads; plan->kv_heads = kv_heads; plan->head_dim = head_dim;
-  plan->chunk = chunk;
+  plan->chunk = hd->chunk;
   plan->n_items = ni;
   plan->exact = 1;
   plan->reserved = np > 0 ? 1 : 0;       // whether any token was split (the merge kernel is skipped otherwise)
@@ -944,8 +1026,6 @@ static int plan_host_image(const char* fn, const int* h_token_pos, int n_tokens,
       int cs = static_cast<int>(std::min<long long>(8, resident / pairs));
       if (tuning().cluster_size >= 2 && tuning().cluster_size < cs) cs = tuning().cluster_size;
       while (cs > 2 && !cluster_size_ok(cs)) --cs;       // 8, 4, 3 or 2 blocks: what the landing areas are sized for
-      int max_len = 0;
-      for (int t = 0; t < n_tokens; ++t) max_len = std::max(max_len, h_token_pos[t] + 1);
       if ((max_len + 4 * cs - 1) / (4 * cs) <= tuning().cluster_max_keys) plan->cluster = cs;
     }
   }

@@ -73,6 +73,10 @@ struct DecodeArgs {
   const void* new_v;
   const int* slots;
   unsigned int* host_err;   // pinned host word that also receives a give-up (null: none)
+  // 1: the launch before this one on the stream let it start only after everything this launch reads was
+  // complete, and writes nothing that it reads or writes (the prefill kernel of a mixed step): wait for it
+  // before leaving instead of before loading.
+  int wait_last;
   unsigned long long pool_rows;   // slots the K/V tensor maps cover (the pool size when the caller gave it, else a bound)
 };
 

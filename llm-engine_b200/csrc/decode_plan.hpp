@@ -5,16 +5,20 @@
 // A decode step is a ragged batch: token t attends L_t = token_pos[t] + 1 keys and
 // L_t can differ by 64x inside one batch.  One thread block per (token, kv head)
 // would leave the GPU waiting for the longest sequence, so each token's key range
-// is cut into chunks of `chunk` keys; a work item is (token, first key, key count).
-// Tokens that fit one chunk write their output directly; the others write one
-// partial (running max, denominator, unnormalised accumulator) per chunk, and the
-// thread block that finishes a token's last outstanding chunk merges them.
+// is cut; a work item is (token, first key, key count).  Tokens that stay whole write
+// their output directly; the others write one partial (running max, denominator,
+// unnormalised accumulator) per item, and a second kernel merges them.
+//
+// Two ways to cut (ShareRule below): steps with enough keys are laid end to end and cut
+// into equal SHARES, one per resident warp and kv head, so that every warp reads the same
+// number of keys and a token has a partial per warp that touches it and no more; small
+// steps are cut token by token into chunks.
 //
 // Workspace layout (every region 256-byte aligned):
 //   header | tok_split[n_tokens] | counters[n_tokens*kv_heads] | items[cap_items]
 //          | part_ml[cap_parts*q_heads*2] | part_acc[cap_parts*q_heads*head_dim]
-// The first four regions up to items[n_items] form the "plan image" that the host
-// planner uploads in one copy.
+// The first four regions up to items[n_items] (and, behind the items of a plan with shares,
+// the first item of every share) form the "plan image" that the host planner uploads in one copy.
 #pragma once
 
 #include <cstddef>
@@ -39,7 +43,8 @@ struct PlanHeader {
   int n_tokens;
   int n_parts;
   int kv_heads;
-  int pad[2];
+  int n_shares;  // 0: units are dealt one by one; otherwise int first_item[n_shares + 1] follows the items
+  int pad;
 };
 
 struct WorkItem {
@@ -107,7 +112,67 @@ inline int ws_extra_for_bytes(int n_tokens, int q_heads, int kv_heads, int head_
   return lo;
 }
 
-// Chunk rule.  items_at[j] = sum over tokens of ceil(L_t / (64 << j)).
+// ---- shares -----------------------------------------------------------------------
+// The tokens' histories, each rounded up to whole slabs, are laid end to end; share j is the
+// stretch [j * per, (j + 1) * per).  A token is cut at every multiple of `per` that lies more
+// than a slab inside it on both sides, and an item belongs to the share its first key falls
+// into, give or take that slab: shares stay within a slab of `per`, no piece of a cut token is
+// a lone slab, and every share but possibly the last begins with exactly one item.
+//
+// Cutting every token into chunks of its own (256 keys and up, dealt round-robin) gave a step of
+// 256 sequences x 128-8,192 keys on 4 kv heads 1,440 items a kv head for 444 warps: a third more
+// or less work on some warps and 1,100 partials, where shares give each warp the same 1,145 keys
+// and 650 partials.
+constexpr int kShareSlab = 32;
+// Below this many keys a share the tokens are cut one by one into chunks of this length instead:
+// equal shares would cut short tokens that need no merge at all when left whole.
+constexpr int kMinShareKeys = 128;
+
+PKV_HD inline int share_padded(int len) { return (len + kShareSlab - 1) & ~(kShareSlab - 1); }
+
+struct ShareCut {
+  long long first;   // first cut, in the laid-out coordinate (valid when n > 0)
+  int n;             // cuts: the token has n + 1 items
+};
+// Cuts of a token that begins at `begin` and is `padded` keys long (> 0).
+PKV_HD inline ShareCut share_cuts(long long begin, int padded, int per) {
+  ShareCut c;
+  c.first = ((begin + kShareSlab) / per + 1) * per;
+  const long long end = begin + padded - kShareSlab;    // cuts lie strictly below
+  c.n = end > c.first ? static_cast<int>((end - 1 - c.first) / per) + 1 : 0;
+  return c;
+}
+// Share of the item that begins at `item_begin` (a last token of one slab would otherwise open a share of its own).
+PKV_HD inline int share_of(long long item_begin, int per, int n_shares) {
+  const long long s = (item_begin + kShareSlab) / per;
+  return static_cast<int>(s < n_shares ? s : n_shares - 1);
+}
+
+struct ShareRule {
+  int per;        // keys per share (a multiple of the slab), or 0: cut token by token
+  int n_shares;
+  int chunk;      // per == 0: keys per chunk, 0 = tokens are not cut
+};
+// total: padded keys of the step; max_shares: warps per kv head (0: the workspace has no room for splits).
+PKV_HD inline ShareRule share_rule(long long total, int max_shares, int forced_chunk) {
+  ShareRule r{0, 0, 0};
+  if (max_shares <= 0) return r;
+  if (forced_chunk > 0 && total / forced_chunk <= max_shares) { r.chunk = forced_chunk; return r; }
+  if (total < static_cast<long long>(max_shares) * kMinShareKeys) { r.chunk = kMinShareKeys; return r; }
+  const long long per = ((total + max_shares - 1) / max_shares + kShareSlab - 1) / kShareSlab * kShareSlab;
+  if (per > 0x40000000) return r;
+  r.per = static_cast<int>(per);
+  r.n_shares = static_cast<int>((total + r.per - 1) / r.per);
+  return r;
+}
+// Shares a workspace with room for `extra` items beyond one per token takes: the items, their
+// partials and the table behind the items.
+PKV_HD inline int max_shares_for(int extra, int workers_per_kv_head) {
+  const int fit = (extra - 2) / 5 * 4;
+  return fit < workers_per_kv_head ? (fit > 0 ? fit : 0) : workers_per_kv_head;
+}
+
+// Chunk rule of the shared-prefix planner, and of the cluster form's offer.  items_at[j] = sum over tokens of ceil(L_t / (64 << j)).
 //   1. take the smallest chunk >= 256 keys whose item count stays within the
 //      budget (one item per token plus `extra_budget`): the most parallelism the
 //      workspace and the target grid allow, without paying a partial per 16 KB;

@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(&kmap) : "memory");
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(&vmap) : "memory");
   }
-  bool waited = false;
+  bool waited = !CLUSTER && !FUSED_APPEND && a.wait_last != 0;
   // Cluster launches: this warp's one unit, from the token's position alone (a step constant).
   int c_token = 0, c_kvh = 0, c_begin = 0, c_len = 0, c_nsplits = 1, c_split = 0;
   uint32_t c_rank = 0, c_size = 1;
@@ -172,12 +172,37 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
       asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
     }
   }
+  // Units of this warp: one item each (item, kv head) dealt round-robin, or, when the plan has shares, all the
+  // items of a (share, kv head) one after the other.  The issue side and the math side walk the same list,
+  // each with a cursor of its own.
+  const int n_shares = (CLUSTER || TOK > 1 || a.direct) ? 0 : a.header->n_shares;
   const int n_items = CLUSTER ? 0 : (TOK > 1 ? a.n_shared : (a.direct ? a.n_tokens : a.header->n_items));
-  const int total = CLUSTER ? (c_len > 0 ? 1 : 0) : n_items * a.kv_heads;
+  const int total = CLUSTER ? (c_len > 0 ? 1 : 0) : (n_shares > 0 ? n_shares : n_items) * a.kv_heads;
   const int gw = CLUSTER ? 0 : blockIdx.x * WARPS + warp, GW = CLUSTER ? 1 : gridDim.x * WARPS;
+  const int* share_first = CLUSTER || TOK > 1 || a.direct ? nullptr : reinterpret_cast<const int*>(a.items + n_items);
+  struct Cursor { int u, item, end, kvh; };
+  auto next_unit = [&](Cursor& x) -> bool {
+    if constexpr (CLUSTER) {             // at most one unit
+      x.kvh = c_kvh;
+      return ++x.u < total;
+    }
+    ++x.item;
+    while (x.item >= x.end) {
+      x.u += GW;
+      if (x.u >= total) { x.u = total; x.item = x.end = 0; return false; }
+      x.item = x.u / a.kv_heads;
+      x.kvh = x.u - x.item * a.kv_heads;
+      x.end = x.item + 1;
+      if (n_shares > 0) {
+        x.end = __ldg(share_first + x.item + 1);
+        x.item = __ldg(share_first + x.item);
+      }
+    }
+    return true;
+  };
 
   // ---------------------------- issue side ----------------------------
-  int iu = gw - GW;             // unit the issue pointer is in (advanced before first use)
+  Cursor ic{gw - GW, 0, 0, 0};  // unit the issue pointer is in (advanced before first use)
   int i_nslabs = 0, i_slab = 0, i_kvbeg = 0, i_len = 0, i_x0 = 0;
   const int* i_tbl = nullptr;
   int i_ent = 0, i_ent_base = -64;   // this lane's block-table entry for box i_ent_base + lane
@@ -186,9 +211,8 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
   // Issues the next slab of this warp's unit sequence, if there is one.
   auto issue_next = [&]() -> bool {
     while (i_slab >= i_nslabs) {
-      iu += GW;
-      if (iu >= total) { iu = total; return false; }
-      const int item = iu / a.kv_heads, kvh = CLUSTER ? c_kvh : iu - item * a.kv_heads;
+      if (!next_unit(ic)) return false;
+      const int item = ic.item, kvh = ic.kvh;
       int token, part;
       if constexpr (CLUSTER) {
         token = c_token;
@@ -266,8 +290,9 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
   // ---------------------------- math side -----------------------------
   const int mi = lane >> 3, r8 = lane & 7;
   bool more = true;
-  for (int cu = gw; cu < total; cu += GW) {
-    const int item = cu / a.kv_heads, kvh = CLUSTER ? c_kvh : cu - item * a.kv_heads;
+  Cursor mc{gw - GW, 0, 0, 0};
+  while (next_unit(mc)) {
+    const int item = mc.item, kvh = mc.kvh;
     int token, kv_begin, kv_len, part;
     int toks[TOK], parts[TOK], n_tok = 1;
     if constexpr (CLUSTER) {
@@ -463,7 +488,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
       ++n_consumed;
     }
     if constexpr (!CLUSTER) {
-      if (!ok) return;  // this warp has copies in flight only into its own ring; nothing else depends on it
+      if (!ok) break;   // this warp has copies in flight only into its own ring; nothing else depends on it
     }                   // (in a cluster the warp stays for the barriers; its give-up is on record)
 
     while (more && n_issued - n_consumed < NSTAGES) more = issue_next();  // keep loads flowing through the finish
@@ -527,6 +552,9 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
         }
       }
     }
+  }
+  if constexpr (!CLUSTER && !FUSED_APPEND) {
+    if (a.wait_last) pdl_wait();       // this launch's completion has to imply the previous one's
   }
   if constexpr (CLUSTER) {
     if (c_nsplits > 1) {               // the same for every thread of the cluster

@@ -273,8 +273,11 @@ __global__ void __launch_bounds__(kThreads, 2)
   tc_fence_after();
   const uint32_t tmem = tmem_base_slot;
 
-  pdl_launch_dependents();
+  // In a mixed step (a.dims) the launch behind this one is the decode kernel, which does not wait for this
+  // one before it reads the router's plan: it may start only once the plan is complete.
+  if (a.dims == nullptr) pdl_launch_dependents();
   pdl_wait();
+  if (a.dims != nullptr) pdl_launch_dependents();
 
   // Order in which the (sequence, query tile) groups are handed out: longest key range first, so that
   // the launch ends on its shortest items and the blocks finish together (with the natural order the

@@ -1,0 +1,116 @@
+"""The split-K work list (csrc/decode_plan.hpp): every token's keys exactly once, partial slots distinct, shares
+that cover the items in order and hold about the same number of keys.  The host planner is read back from
+its image; the device planner has to produce the same integers."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+SLAB, MIN_SHARE = 32, 128
+
+
+def align256(n):
+    return (n + 255) // 256 * 256
+
+
+def host_image(pkv, pos, qh, kvh, hd, ws_bytes=None):
+    L = pkv.lib()
+    pos = np.ascontiguousarray(pos, dtype=np.int32)
+    nstage = L.pkv_decode_plan_staging_bytes(pos.size, kvh)
+    staging = np.zeros(nstage, dtype=np.uint8)
+    plan, image = pkv._lib.DecodePlan(), C.c_size_t(0)
+    ws = ws_bytes or L.pkv_decode_workspace_bytes(pos.size, qh, kvh, hd)
+    st = L.pkv_decode_plan_host_image(pos.ctypes.data, pos.size, qh, kvh, hd, staging.ctypes.data, nstage, ws, C.byref(plan), C.byref(image))
+    assert st == 0, L.pkv_last_error()
+    return staging[:image.value], plan
+
+
+def read(image, n, kvh):
+    """(header, splits, items, first item of every share) of a plan image."""
+    words = image.view(np.int32)
+    header = words[:8]
+    o = 256
+    splits = words[o // 4:o // 4 + 2 * n].reshape(n, 2)
+    o = align256(align256(o + 8 * n) + 4 * n * kvh)
+    items = words[o // 4:o // 4 + 4 * header[1]].reshape(-1, 4)
+    first = words[o // 4 + 4 * header[1]:][:header[6] + 1] if header[6] else None
+    return header, splits, items, first
+
+
+def check(image, pos, kvh):
+    n = len(pos)
+    header, splits, items, first = read(image, n, kvh)
+    assert header[3] == n and header[5] == kvh
+    seen = np.zeros(header[4], dtype=int)
+    for t in range(n):
+        mine = items[items[:, 0] == t]
+        assert len(mine) == splits[t, 1]
+        mine = mine[np.argsort(mine[:, 1])]
+        at = 0
+        for s, (_, b, ln, part) in enumerate(mine):
+            assert b == at and ln > 0 and (b % SLAB == 0)
+            assert part == (splits[t, 0] + s if len(mine) > 1 else -1)
+            if part >= 0:
+                seen[part] += 1
+            at += ln
+        assert at == pos[t] + 1
+    assert (seen == 1).all()
+    if first is not None:
+        per, n_shares = header[2], header[6]
+        assert first[0] == 0 and first[-1] == header[1] and (np.diff(first) >= 0).all() and (np.diff(first)[:-1] > 0).all()
+        padded = [sum(-(-x // SLAB) * SLAB for x in items[first[s]:first[s + 1], 2]) for s in range(n_shares)]
+        assert max(padded) <= per + 2 * SLAB and min(padded[:-1], default=per) >= per - 2 * SLAB
+        assert items[:, 2].min() > 0 and all(x > SLAB for t in range(n) if splits[t, 1] > 1 for x in items[items[:, 0] == t, 2])
+    return header
+
+
+STEPS = {
+    "one": [0], "one long": [70000], "slab edges": [30, 31, 32, 33, 63, 64, 65, 95, 96, 127, 128] * 40,
+    "small": [5, 300, 17, 129, 1500], "equal": [4095] * 256, "short": [99] * 1500, "single keys": [0] * 2500,
+    "ragged": np.random.default_rng(3).integers(0, 8192, size=256), "last token of one slab": [127] * 3551 + [31],
+}
+
+
+@pytest.mark.parametrize("kvh", [1, 2, 4, 8])
+@pytest.mark.parametrize("name", sorted(STEPS))
+def test_host_plan_covers_every_key_once(pkv, name, kvh):
+    pos = np.asarray(STEPS[name], dtype=np.int32)
+    for hd in (64, 128):
+        check(host_image(pkv, pos, 4 * kvh, kvh, hd)[0], pos, kvh)
+
+
+@pytest.mark.parametrize("extra", [0, 1, 2, 3, 7, 40, 200])
+def test_small_workspaces_take_fewer_shares(pkv, extra):
+    """The partials (2 * extra slots) and the share table stay inside what the workspace was sized for."""
+    pos, qh, kvh, hd = np.random.default_rng(4).integers(0, 4096, size=60).astype(np.int32), 8, 2, 64
+    n = pos.size
+    off_items = align256(align256(256 + 8 * n) + 4 * n * kvh)
+    ml = align256(off_items + 16 * (n + extra))
+    total = align256(align256(ml + 8 * 2 * extra * qh) + 4 * 2 * extra * qh * hd)
+    image, plan = host_image(pkv, pos, qh, kvh, hd, total)
+    header = check(image, pos, kvh)
+    assert header[4] <= 2 * extra and image.size <= ml
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", sorted(STEPS))
+def test_device_plan_is_the_host_plan(pkv, torch_cuda, name):
+    """Same cuts, slots and shares, around the 1,024 tokens one pass of the planner block takes (chunked steps
+    list the same items in another order)."""
+    torch = torch_cuda
+    pos = np.asarray(STEPS[name], dtype=np.int32)
+    for n in sorted({pos.size, min(pos.size, 1024), min(pos.size, 1025)}):
+        p = np.ascontiguousarray(pos[:n])
+        plan = pkv.DecodePlan(n, 32, 4, 64)
+        plan.workspace.random_(0, 255)
+        plan.build_device(torch.from_numpy(p).cuda())
+        torch.cuda.synchronize()
+        got = read(plan.workspace.cpu().numpy(), n, 4)
+        image, _ = host_image(pkv, p, 32, 4, 64)
+        want = read(image, n, 4)
+        check(plan.workspace.cpu().numpy(), p, 4)
+        assert got[0].tolist() == want[0].tolist() and (got[1][:, 1] == want[1][:, 1]).all()
+        key = lambda items: sorted(map(tuple, items.tolist()))
+        assert key(got[2]) == key(want[2])
+        if want[3] is not None:
+            assert (got[3] == want[3]).all() and (got[2] == want[2]).all()
