@@ -88,7 +88,7 @@ constexpr int kPlanThreads = 1024;
 struct RouteArgs {
   const int* token_seq;
   const int* table_offset;
-  int min_run, q_heads;
+  int min_run;
   int* run_start;   // [n_tokens] scratch: first token of the run a token belongs to
   int* run_len;     // [n_tokens] scratch: length of a run, stored at its first token
   int* eff_len;     // [n_tokens] out
@@ -96,13 +96,13 @@ struct RouteArgs {
   int* q_len;
   int* ctx_len;
   int* tbl_off;
-  int* dims;        // [4] out: runs, 128-row tiles of the longest run, prefill work items, decode tokens
+  int* dims;        // [4] out: runs, tokens of the longest, tokens of none
 };
 
 // Inclusive scans over the block's threads, one value each (sum, or maximum).  `sm` holds one word per
 // warp and is free for the next scan only after another barrier; *total receives the block's result.
-struct ScanSum { static __device__ __forceinline__ int id() { return 0; } static __device__ __forceinline__ int op(int a, int b) { return a + b; } };
-struct ScanMax { static __device__ __forceinline__ int id() { return -1; } static __device__ __forceinline__ int op(int a, int b) { return max(a, b); } };
+struct ScanSum { static __device__ __forceinline__ int op(int a, int b) { return a + b; } };
+struct ScanMax { static __device__ __forceinline__ int op(int a, int b) { return max(a, b); } };
 template <typename Op>
 __device__ __forceinline__ int warp_scan(int v, int lane) {
 #pragma unroll
@@ -324,11 +324,10 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
   }
   if constexpr (ROUTE) {
     if (tid == 0) {
-      const int tiles = (sm_misc[1] + 127) / 128;
       r.dims[0] = sm_misc[0];
-      r.dims[1] = tiles;
-      r.dims[2] = sm_misc[0] * tiles * r.q_heads;
-      r.dims[3] = sm_misc[2];
+      r.dims[1] = sm_misc[1];
+      r.dims[2] = sm_misc[2];
+      r.dims[3] = 0;
     }
   }
 }
@@ -849,7 +848,7 @@ int mixed_attn(const void* q, const void* kc, const void* vc, const int* bt, con
   char* rbase = static_cast<char*>(workspace) + dec_bytes;
   RouteArgs r;
   r.token_seq = ts; r.table_offset = to;
-  r.min_run = min_run; r.q_heads = q_heads;
+  r.min_run = min_run;
   r.run_start = reinterpret_cast<int*>(rbase + rl.off_start);
   r.run_len = reinterpret_cast<int*>(rbase + rl.off_len);
   r.eff_len = reinterpret_cast<int*>(rbase + rl.off_eff);

@@ -3,10 +3,14 @@
 //
 // llm-engine has no prefill kernel (src/kernels/attention_prefill.cu:1 is a stub):
 // every prompt token goes through the decode kernel and re-reads its whole history.
-// Here a work item is 128 consecutive tokens of one sequence's chunk for one query
-// head; its keys are walked in tiles of 64, so S = Q K^T and O = P V are dense
-// 128 x 64 x 64 contractions issued as tcgen05.mma with the accumulators in tensor
-// memory.  The result it must agree with is ref::paged_attention_head
+// Here a work item is up to 128 (token, query head) rows that share a kv head: the
+// heads of a GQA group side by side for 128 / heads consecutive tokens of one sequence's
+// chunk (16 tokens x 8 heads, 18 x 7, 128 x 1).  Its keys are walked in tiles of 64, so
+// S = Q K^T and O = P V are dense 128 x 64 x 64 contractions issued as tcgen05.mma with
+// the accumulators in tensor memory.  Few tokens per tile is what keeps the work close to
+// the causal triangle: a tile computes every key up to its last token's for all its rows,
+// so 128-token tiles of one head spend 64 keys a row on average above the diagonal (and a
+// whole tile on a chunk of 17 tokens), 16-token tiles 8.  The result it must agree with is ref::paged_attention_head
 // (include/engine/ops.h:87-111) applied to every (token, head) of the chunk.
 //
 // Thread blocks are persistent, two per SM: each takes items until none are left --
@@ -83,7 +87,8 @@ constexpr int kSmemTotal = kSmemOnes + kKBytes + 1024;       // 105 KB: two bloc
 constexpr int kThreads = 192, kProducerWarp = 4, kMmaWarp = 5;   // warps 0-3: softmax, one thread per row of the tile
 constexpr uint32_t kTmemCols = 256;                          // two blocks per SM share the 512 columns
 constexpr uint32_t kTmemS = 0, kTmemO = 128, kTmemL = 192;   // S0 @0, S1 @64, O @128 (64) with the row sums right behind (16)
-constexpr int kMaxRanked = 256;       // launches of up to this many (sequence, tile) groups hand them out longest first
+constexpr int kBuckets = 128;
+constexpr int kMaxRankedSeqs = 256;   // launches of up to this many sequences hand their tiles out longest first
 constexpr float kRescaleThreshold = 8.f;                     // in log2 units: P stays below 2^8
 
 struct PrefillArgs {
@@ -94,16 +99,19 @@ struct PrefillArgs {
   const int* ctx_len;
   void* out;
   int q_heads, kv_heads, group;
+  int pack, tile_tokens, head_tiles;   // query heads per tile, tokens per tile, q_heads / pack
+  uint32_t by_pack;                    // (row * by_pack) >> 16 == row / pack for row < 128
+  uint32_t by_tile_tokens;             // umulhi(x, by_tile_tokens) == x / tile_tokens for 0 <= x < 2^25 (8 <= tile_tokens <= 128)
   int block_size, bs_log2;
   float scale;
-  // persistent scheduling: items = sequences x query-tile slots x heads, handed out by a ticket counter
+  // persistent scheduling: items = query tiles x head tiles, handed out by a ticket counter
   // (ticket == nullptr: dealt in a fixed order instead)
   unsigned int* ticket;
   unsigned int* done;
-  int n_items, n_qtiles_max, n_seqs;
-  // When non-null, { n_seqs, n_qtiles_max, n_items } are read from this device array instead (written
-  // by an earlier kernel on the stream: the mixed-step router decides on the device which runs of
-  // tokens are prefill chunks); the three fields above are then upper bounds that sized the grid.
+  int n_seqs, max_q_len;
+  // When non-null, { n_seqs, max_q_len } are read from this device array instead (written by an earlier
+  // kernel on the stream: the mixed-step router decides on the device which runs of tokens are prefill
+  // chunks); the two fields above are then upper bounds that sized the grid.
   const int* dims;
   unsigned int* host_err;   // pinned host word that also receives a give-up (null: none)
 };
@@ -213,7 +221,7 @@ __device__ __forceinline__ void give_up(unsigned int* host_err) {
 // from shared memory once the item's Q tile barrier has completed.
 struct ItemDesc {
   int n_kt;        // key tiles; -1: no more items
-  int head, row0, rows_here, kv_total, limit0;   // limit0 = last visible key position of row 0
+  int head, row0, rows_here, kv_total, limit0;   // first head and token, rows that are stored, keys, last visible key of the first token
   int pad[2];
 };
 
@@ -256,14 +264,19 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
     mbar_fence_init();
   }
+  // rows past pack x tile_tokens are never fetched: zero, so that they cost no rescale
+  for (int i = a.pack * a.tile_tokens * 8 + threadIdx.x; i < kQTile * 8; i += kThreads) {
+    *reinterpret_cast<uint4*>(base_ptr + kSmemQ + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+    *reinterpret_cast<uint4*>(base_ptr + kSmemQ + kQBytes + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+  }
   if (threadIdx.x < kKTile) {
     // the tile of ones that makes columns 64..79 of every P V product the row sums of P
     const uint32_t one2 = pack2<T>(1.f, 1.f);
     unsigned char* orow = base_ptr + kSmemOnes + threadIdx.x * 128;
 #pragma unroll
     for (int ch = 0; ch < 8; ++ch) *reinterpret_cast<uint4*>(orow + ch * 16) = make_uint4(one2, one2, one2, one2);
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   }
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_base_slot)), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
@@ -279,39 +292,45 @@ __global__ void __launch_bounds__(kThreads, 2)
   pdl_wait();
   if (a.dims != nullptr) pdl_launch_dependents();
 
-  // Order in which the (sequence, query tile) groups are handed out: longest key range first, so that
-  // the launch ends on its shortest items and the blocks finish together (with the natural order the
-  // last blocks ran up to a tenth of the launch alone).  Every block ranks the groups itself, once:
-  // a few hundred comparisons per thread for up to kMaxRanked groups; larger launches keep the
-  // natural order, whose tail matters less the more items there are.
-  __shared__ int s_key[kMaxRanked];
-  __shared__ short s_order[kMaxRanked];
+  // Query tiles are handed out longest key range first, so that the launch ends on its shortest items and the
+  // blocks finish together (configuration 4: 515 us for four layers sequence by sequence, 486 us this way).
+  // The lengths of a sequence's tiles are an arithmetic series, so nothing has to be sorted: lengths fall into
+  // kBuckets buckets, s_cum[b] counts the tiles of buckets 0 .. b, longest first, and the tile of a given rank
+  // is looked up as (bucket, sequence, place) -- in the producer's tile_of_rank, a few hundred cycles.
+  // Launches of more than kMaxRankedSeqs sequences keep the natural order, whose tail matters less the more
+  // items there are.
+  __shared__ int s_top[kMaxRankedSeqs];      // keys the sequence's last tile sees, rounded up to whole tiles; tile_tokens less per tile before
+  __shared__ int s_tiles[kMaxRankedSeqs];
+  __shared__ int s_cum[kBuckets];
+  const int tt = a.tile_tokens;
   const int n_seqs = a.dims ? __ldcg(a.dims) : a.n_seqs;
-  const int n_qtiles_max = a.dims ? __ldcg(a.dims + 1) : a.n_qtiles_max;
-  const int n_items = a.dims ? __ldcg(a.dims + 2) : a.n_items;
-  const int n_groups = n_seqs * n_qtiles_max;
-  const bool ranked = n_groups <= kMaxRanked;
+  auto reach = [&](int s, int x) {           // tiles of sequence s whose length is x or more
+    const int over = s_top[s] - x;
+    return over >= 0 ? min(static_cast<int>(__umulhi(over, a.by_tile_tokens)) + 1, s_tiles[s]) : 0;
+  };
+  bool ranked = n_seqs <= kMaxRankedSeqs;
+  int width = 1;                             // keys per bucket
   if (ranked) {
-    for (int j = threadIdx.x; j < n_groups; j += kThreads) {
-      const int z = j / n_qtiles_max, y = j - z * n_qtiles_max;
-      const int ql = __ldg(a.q_len + z);
-      const int nt = (ql + kQTile - 1) / kQTile;
-      s_key[j] = y < nt ? __ldg(a.ctx_len + z) + min((nt - y) * kQTile, ql) : -1;   // keys that tile sees; -1: no such tile
+    for (int s = threadIdx.x; s < n_seqs; s += kThreads) {
+      const int nt = (__ldg(a.q_len + s) + tt - 1) / tt;
+      s_tiles[s] = nt;
+      s_top[s] = nt > 0 ? __ldg(a.ctx_len + s) + nt * tt : 0;
     }
     __syncthreads();
-    for (int j = threadIdx.x; j < n_groups; j += kThreads) {
-      const int kj = s_key[j];
-      int rank = 0;
-      for (int k = 0; k < n_groups; ++k) {
-        const int kk = s_key[k];
-        rank += (kk > kj || (kk == kj && k < j)) ? 1 : 0;
-      }
-      s_order[rank] = static_cast<short>(j);
+    int longest = 0;
+    for (int s = 0; s < n_seqs; ++s) longest = max(longest, s_top[s]);
+    ranked = longest < (1 << 25);            // see by_tile_tokens
+    width = longest / kBuckets + 1;
+    if (threadIdx.x < kBuckets && ranked) {
+      const int x = (kBuckets - 1 - threadIdx.x) * width + 1;
+      int c = 0;
+      for (int s = 0; s < n_seqs; ++s) c += reach(s, x);
+      s_cum[threadIdx.x] = c;
     }
     __syncthreads();
   }
 
-  // The block is persistent: it takes (sequence, query tile, head) items until none are left.  Every
+  // The block is persistent: it takes (sequence, query tile, head tile) items until none are left.  Every
   // role runs its own loop over the items and keeps its own running counts of items (n) and key tiles
   // (g), from which ring stages, buffers and barrier parities follow; the roles are coupled only
   // through the barriers, so the producer prefetches the next item's Q and first K/V tiles, and the
@@ -333,11 +352,43 @@ __global__ void __launch_bounds__(kThreads, 2)
     // ================================ TMA producer ================================
     int n = 0, g = 0;
     unsigned round = 0;                                        // fixed deal: items taken so far
+    const int n_slots = ((a.dims ? __ldcg(a.dims + 1) : a.max_q_len) + tt - 1) / tt;   // tiles of the longest chunk
+    const unsigned n_items = (ranked ? static_cast<unsigned>(s_cum[kBuckets - 1]) : static_cast<unsigned>(n_seqs) * n_slots) * a.head_tiles;
+    // tile number `k` of the ranked list
+    auto tile_of_rank = [&](int k, int& seq, int& tile) {
+      int b = 0;
+      for (; b < kBuckets; b += 32) {
+        const unsigned past = __ballot_sync(0xffffffffu, s_cum[b + lane] > k);
+        if (past) { b += __ffs(past) - 1; break; }
+      }
+      if (b > 0) k -= s_cum[b - 1];                            // place in its bucket
+      const int lo = (kBuckets - 1 - b) * width + 1;
+      for (int s0 = 0; s0 < n_seqs; s0 += 32) {
+        int before = 0, mine = 0;                              // longer tiles of this lane's sequence, and those of the bucket
+        if (s0 + lane < n_seqs) {
+          before = reach(s0 + lane, lo + width);
+          mine = reach(s0 + lane, lo) - before;
+        }
+        int upto = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int x = __shfl_up_sync(0xffffffffu, upto, o);
+          if (lane >= o) upto += x;
+        }
+        const unsigned past = __ballot_sync(0xffffffffu, upto > k);
+        if (past) {
+          const int src = __ffs(past) - 1;
+          seq = s0 + src;
+          tile = s_tiles[seq] - 1 - (__shfl_sync(0xffffffffu, before + mine - upto, src) + k);
+          return;
+        }
+        k -= __shfl_sync(0xffffffffu, upto, 31);
+      }
+      seq = tile = -1;
+    };
     for (;;) {
       dead = __shfl_sync(0xffffffffu, dead ? 1 : 0, 0) != 0;   // only lane 0 waits: keep the warp in step
-      // next item that has work: heads fastest (the heads of a group share their K/V tiles through
-      // L2), groups in the order ranked above (or: a sequence's query tiles from the longest key
-      // range down, then sequences)
+      // next item that has work: head tiles fastest (those of a group share their K/V tiles through L2)
       ItemDesc d;
       int seq = 0;
       d.n_kt = -1;
@@ -352,21 +403,23 @@ __global__ void __launch_bounds__(kThreads, 2)
           t = round * gridDim.x + ((round & 1u) ? gridDim.x - 1u - blockIdx.x : blockIdx.x);
           ++round;
         }
-        if (t >= static_cast<unsigned>(n_items)) break;
-        const int head = static_cast<int>(t % a.q_heads);
-        int rest = static_cast<int>(t / a.q_heads);
-        if (ranked) rest = s_order[rest];
-        const int slot_y = rest % n_qtiles_max;
-        seq = rest / n_qtiles_max;
-        const int q_len = __ldg(a.q_len + seq);
-        const int tile = (q_len + kQTile - 1) / kQTile - 1 - slot_y;
+        if (t >= n_items) break;
+        const int rest = static_cast<int>(t / a.head_tiles);
+        int tile;
+        if (ranked) {
+          tile_of_rank(rest, seq, tile);
+        } else {
+          seq = rest / n_slots;
+          tile = (__ldg(a.q_len + seq) + tt - 1) / tt - 1 - (rest - seq * n_slots);
+        }
         if (tile < 0) continue;
-        const int ctx = __ldg(a.ctx_len + seq);
-        d.head = head;
-        d.row0 = __ldg(a.q_start + seq) + tile * kQTile;
-        d.rows_here = min(kQTile, q_len - tile * kQTile);
-        d.kv_total = ctx + tile * kQTile + d.rows_here;
-        d.limit0 = ctx + tile * kQTile;
+        const int q_len = __ldg(a.q_len + seq), ctx = __ldg(a.ctx_len + seq);
+        const int tokens = min(tt, q_len - tile * tt);
+        d.head = static_cast<int>(t % a.head_tiles) * a.pack;
+        d.row0 = __ldg(a.q_start + seq) + tile * tt;
+        d.rows_here = tokens * a.pack;
+        d.kv_total = ctx + tile * tt + tokens;
+        d.limit0 = ctx + tile * tt;
         d.n_kt = (d.kv_total + kKTile - 1) / kKTile;
         break;
       }
@@ -375,8 +428,8 @@ __global__ void __launch_bounds__(kThreads, 2)
         WAIT(BAR(Q_EMPTY + qb), ((n >> 1) & 1) ^ 1);
         s_item[qb] = d;
         if (d.n_kt > 0 && !dead) {
-          mbar_arrive_expect_tx(BAR(Q_FULL + qb), kQBytes);
-          tma_load_2d(sQ + qb * kQBytes, &qmap, d.head * kHd, d.row0, BAR(Q_FULL + qb));
+          mbar_arrive_expect_tx(BAR(Q_FULL + qb), static_cast<uint32_t>(a.pack * a.tile_tokens) * 128u);
+          tma_load_3d(sQ + qb * kQBytes, &qmap, 0, d.head, d.row0, BAR(Q_FULL + qb));
         } else {
           s_item[qb].n_kt = -1;
           mbar_arrive(BAR(Q_FULL + qb));        // "no more items"
@@ -483,7 +536,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       const ItemDesc d = s_item[qb];
       if (d.n_kt <= 0 || dead) break;
       const int n_kt = d.n_kt, kv_total = d.kv_total, rows_here = d.rows_here;
-      const int limit = d.limit0 + min(r, rows_here - 1);   // last visible key position of this row
+      const int limit = min(d.limit0 + static_cast<int>((r * a.by_pack) >> 16), kv_total - 1);   // last visible key position of this row
       // Reference maximum of the row.  It follows the true running maximum lazily: O and the row
       // sum stay in tensor memory and are only rescaled when the maximum has grown by more than
       // 2^8, so most tiles cost no read-modify-write of the accumulator at all.
@@ -529,7 +582,9 @@ __global__ void __launch_bounds__(kThreads, 2)
           // cannot start before this thread has arrived on P_FULL below.
           WAIT(BAR(PV_DONE + ((g - 1) & 1)), ((g - 1) >> 1) & 1);
           tc_fence_after();
-          const float m_new = fmaxf(m_used, mx);
+          // a row that did not grow that much itself keeps its maximum (f = 1): what a row computes depends
+          // on its own keys alone, not on the rows it shares a warp with
+          const float m_new = (mx - m_used) * sl2 > kRescaleThreshold ? mx : m_used;
           const float f = ex2_approx((m_used - m_new) * sl2);
           m_used = m_new;
 #pragma unroll
@@ -595,6 +650,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         unsigned char* my_row = stage + r * 128;
 #pragma unroll
         for (int dd = 0; dd < 32; dd += 8) {
+          if (r >= rows_here) break;                           // (the rows past the tile's stay zero)
           uint4 w0, w1;
           w0.x = pack2<T>(__uint_as_float(o0[dd]) * inv, __uint_as_float(o0[dd + 1]) * inv);
           w0.y = pack2<T>(__uint_as_float(o0[dd + 2]) * inv, __uint_as_float(o0[dd + 3]) * inv);
@@ -613,8 +669,9 @@ __global__ void __launch_bounds__(kThreads, 2)
         for (int i = 0; i < 8; ++i) {
           const int row = warp * 32 + i * 4 + (lane >> 3), ch = lane & 7;
           const uint4 w = *reinterpret_cast<const uint4*>(stage + row * 128 + ((ch ^ (row & 7)) << 4));
+          const int tok = static_cast<int>((row * a.by_pack) >> 16), h = row - tok * a.pack;
           if (row < rows_here)
-            *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(obase + static_cast<size_t>(row) * a.q_heads * kHd) + ch * 16) = w;
+            *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(obase + (static_cast<size_t>(tok) * a.q_heads + h) * kHd) + ch * 16) = w;
         }
       }
       // The Q buffer may be refilled (by TMA) once every thread is done with it: the item's
@@ -732,8 +789,15 @@ int prefill_launch(const void* q, const void* k_cache, const void* v_cache, cons
   if (st != PKV_OK) return st;
   st = make_pool_tensor_map(&vmap, v_cache, is_bf16, kv_dim, 16, pool_rows);
   if (st != PKV_OK) return st;
-  // q as [n_tokens][q_heads*head_dim]; rows past n_tokens read as zeros
-  st = make_pool_tensor_map(&qmap, q, is_bf16, q_heads * head_dim, kQTile, static_cast<uint64_t>(n_tokens));
+  // Heads per tile: the largest divisor of the group, up to 16, that leaves at most 8 of the 128 rows unused
+  // (a group of 13 would waste 11: its heads take tiles of their own).
+  const int group = q_heads / kv_heads;
+  int pack = 1;
+  for (int p = 2; p <= 16; ++p)
+    if (group % p == 0 && kQTile / p * p >= kQTile - 8) pack = p;
+  const int tile_tokens = kQTile / pack;
+  // q as [n_tokens][q_heads][head_dim]; rows past n_tokens read as zeros
+  st = make_rows_tensor_map(&qmap, q, is_bf16, q_heads, static_cast<uint64_t>(n_tokens), pack, tile_tokens);
   if (st != PKV_OK) return st;
 
   auto kern = prefill_tc_kernel<T>;
@@ -749,14 +813,18 @@ int prefill_launch(const void* q, const void* k_cache, const void* v_cache, cons
   a.block_tables = block_tables; a.table_offset = table_offset;
   a.q_start = q_start; a.q_len = q_len; a.ctx_len = ctx_len;
   a.out = out;
-  a.q_heads = q_heads; a.kv_heads = kv_heads; a.group = q_heads / kv_heads;
+  a.q_heads = q_heads; a.kv_heads = kv_heads; a.group = group;
+  a.pack = pack; a.tile_tokens = tile_tokens; a.head_tiles = q_heads / pack;
+  a.by_pack = 65536u / pack + 1u;
+  a.by_tile_tokens = 0xffffffffu / tile_tokens + 1u;
   a.block_size = block_size; a.bs_log2 = bsl;
   a.scale = scale;
-  a.n_qtiles_max = (max_q_len + kQTile - 1) / kQTile;
   a.n_seqs = n_seqs;
-  const long long n_items = static_cast<long long>(n_seqs) * a.n_qtiles_max * q_heads;
-  if (n_items > 0x7fffffffll) return fail(PKV_E_UNSUPPORTED, "%s: %lld work items; at most 2^31 - 1 per call", fn, n_items);
-  a.n_items = static_cast<int>(n_items);
+  a.max_q_len = max_q_len;
+  const long long slots = static_cast<long long>(n_seqs) * ((max_q_len + tile_tokens - 1) / tile_tokens) * a.head_tiles;
+  if (slots > 0x7fffffffll) return fail(PKV_E_UNSUPPORTED, "%s: %lld work items; at most 2^31 - 1 per call", fn, slots);
+  // every sequence has at most one tile that is not full
+  const long long n_items = std::min<long long>(slots, (n_tokens / tile_tokens + static_cast<long long>(n_seqs)) * a.head_tiles);
   a.dims = d_dims;
   a.host_err = error_mirror(may_allocate);
   const TicketPair tp = ticket_pair_for(static_cast<cudaStream_t>(stream), dev);

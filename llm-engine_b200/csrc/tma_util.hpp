@@ -48,6 +48,24 @@ inline int make_pool_tensor_map(CUtensorMap* map, const void* pool, bool is_bf16
   return PKV_OK;
 }
 
+// Rows of a packed step as a 3-D tensor [tokens][heads][64] of 16-bit elements, fetched in boxes of
+// box_tokens x box_heads x 64 (at most 256 each): row token * box_heads + head of the box, 128-byte swizzle.
+inline int make_rows_tensor_map(CUtensorMap* map, const void* rows, bool is_bf16, int heads, uint64_t tokens, int box_heads,
+                                int box_tokens) {
+  PFN_cuTensorMapEncodeTiled enc = tensor_map_encoder();
+  if (!enc) return fail(PKV_E_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  const cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(heads), tokens};
+  const cuuint64_t strides[2] = {128, static_cast<cuuint64_t>(heads) * 128};
+  const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_heads), static_cast<cuuint32_t>(box_tokens)};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = enc(map, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
+                         const_cast<void*>(rows), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(PKV_E_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", static_cast<int>(r));
+  return PKV_OK;
+}
+
 #if defined(__CUDACC__)
 // ---- mbarrier ---------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -109,6 +127,12 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n" ::"r"(dst),
       "l"(map), "r"(bar), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n" ::"r"(dst),
+      "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
 __device__ __forceinline__ void movmatrix_trans(uint32_t& dst, uint32_t src) {

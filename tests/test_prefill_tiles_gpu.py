@@ -1,0 +1,40 @@
+"""Query tiles that hold several heads of a group: every packing the launcher chooses, chunk lengths around its
+tile, and the order the tiles are handed out in (one, a few dozen, and more sequences than are ranked)."""
+import numpy as np
+import pytest
+
+from tests.gpu_util import TOL, from_device, rel_errors
+from tests.test_prefill_gpu import make_case, run_prefill
+
+pytestmark = pytest.mark.gpu
+
+
+def check(pkv, orc, torch, qh, kvh, ctx, new, seed, dtype="bf16"):
+    case = make_case(orc, pkv, dtype, qh, kvh, 16, ctx, new, seed)
+    _, _, want = case.expected(orc, threads=8)
+    d = run_prefill(pkv, torch, case)
+    _, got = from_device(torch, orc, d["out"], dtype)
+    assert np.isfinite(got).all()
+    e_ref, e_row = rel_errors(got.reshape(-1, 64), want.reshape(-1, 64))
+    assert e_ref <= TOL[dtype] and e_row <= TOL[dtype], (e_ref, e_row)
+
+
+@pytest.mark.parametrize("group", [1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 13, 16, 20, 28])
+def test_every_packing(pkv, orc, torch_cuda, group):
+    """Tiles of 128 / heads tokens: 8 (16 heads) to 128 (one head; also a group of 13, which would waste rows)."""
+    pack = max(p for p in range(1, 17) if group % p == 0 and (p == 1 or 128 // p * p >= 120))
+    tt = 128 // pack
+    check(pkv, orc, torch_cuda, 2 * group, 2, [0, 5, 64, 190, 0], [tt - 1, tt, tt + 1, 2 * tt + 3, 1], seed=group)
+
+
+@pytest.mark.parametrize("n_seqs", [1, 31, 33, 70, 257])
+def test_many_sequences(pkv, orc, torch_cuda, n_seqs):
+    rng = np.random.default_rng(n_seqs)
+    ctx = [int(x) for x in rng.integers(0, 300, size=n_seqs)]
+    new = [int(x) for x in rng.integers(1, 60, size=n_seqs)]
+    check(pkv, orc, torch_cuda, 14, 2, ctx, new, seed=5, dtype="f16")
+
+
+def test_equal_lengths(pkv, orc, torch_cuda):
+    """Every tile of a rank has the same length as its neighbours: one bucket, many ties."""
+    check(pkv, orc, torch_cuda, 8, 1, [64] * 24, [48] * 24, seed=6)
