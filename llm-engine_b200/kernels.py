@@ -22,6 +22,18 @@ def _suffix(t) -> str:
         raise TypeError(f"unsupported KV element type {t.dtype}") from None
 
 
+_BY_DTYPE = {}      # (entry point, torch.dtype) -> (name, function): the names are put together once
+
+
+def _fn(op: str, t):
+    """(name, C function) of the entry point `op` for the element type of pool tensor t."""
+    found = _BY_DTYPE.get((op, t.dtype))
+    if found is None:
+        name = op + _suffix(t)
+        found = _BY_DTYPE[op, t.dtype] = (name, getattr(_lib.lib(), name))
+    return found
+
+
 def _ptr(t):
     if t is None:
         return None
@@ -32,17 +44,31 @@ def _ptr(t):
     return t.data_ptr()
 
 
+def _no_raw_stream(_):
+    import torch
+    return torch.cuda.current_stream().cuda_stream
+
+
+_raw_stream = None   # (device index) -> the current stream's handle
+
+
 def _stream(stream):
-    if stream is None:
-        import torch
-        return torch.cuda.current_stream().cuda_stream
-    return getattr(stream, "cuda_stream", stream)
+    """The stream's handle; None: the current stream of the current device.  A torch.cuda.Stream object is not
+    built for it: that alone takes 3.4 us, as long as a launch."""
+    global _raw_stream
+    if stream is not None:
+        return getattr(stream, "cuda_stream", stream)
+    import torch
+    if _raw_stream is None:
+        torch.cuda.init()
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", _no_raw_stream)
+    return _raw_stream(torch.cuda.current_device())
 
 
 def launch_store_kv(k, v, slots, k_cache, v_cache, n_tokens: int, kv_dim: int, stream=None) -> None:
     """k_cache[slots[t]] = k[t], v_cache[slots[t]] = v[t] (engine::launch_store_kv)."""
-    fn = f"pkv_append_{_suffix(k_cache)}"
-    st = getattr(_lib.lib(), fn)(_ptr(k), _ptr(v), _ptr(slots), _ptr(k_cache), _ptr(v_cache), n_tokens, kv_dim,
+    fn, call = _fn("pkv_append_", k_cache)
+    st = call(_ptr(k), _ptr(v), _ptr(slots), _ptr(k_cache), _ptr(v_cache), n_tokens, kv_dim,
                                  _stream(stream))
     _lib.check(fn, st)
 
@@ -51,8 +77,8 @@ def launch_rope_store_kv(q, k, v, positions, cos_table, sin_table, slots, k_cach
                          q_heads: int, kv_heads: int, head_dim: int, stream=None) -> None:
     """launch_rope(q) + launch_rope(k) + launch_store_kv in one pass: q rotated in place, rotated k and v
     written to their slots (cos/sin: fp32 tables [max_positions][head_dim/2])."""
-    fn = f"pkv_rope_append_{_suffix(k_cache)}"
-    st = getattr(_lib.lib(), fn)(_ptr(q), _ptr(k), _ptr(v), _ptr(positions), _ptr(cos_table), _ptr(sin_table),
+    fn, call = _fn("pkv_rope_append_", k_cache)
+    st = call(_ptr(q), _ptr(k), _ptr(v), _ptr(positions), _ptr(cos_table), _ptr(sin_table),
                                  _ptr(slots), _ptr(k_cache), _ptr(v_cache), n_tokens, q_heads, kv_heads, head_dim,
                                  _stream(stream))
     _lib.check(fn, st)
@@ -73,10 +99,10 @@ def launch_attention_decode(q, k_cache, v_cache, block_tables, table_offset, tok
                             n_tokens: int, q_heads: int, kv_heads: int, head_dim: int, block_size: int,
                             scale: float, stream=None, workspace=None) -> None:
     """engine::launch_attention_decode; `workspace` (uint8 CUDA tensor) enables split-K."""
-    fn = f"pkv_decode_attn_{_suffix(k_cache)}"
+    fn, call = _fn("pkv_decode_attn_", k_cache)
     ws_ptr = _ptr(workspace)
     ws_bytes = workspace.numel() * workspace.element_size() if workspace is not None else 0
-    st = getattr(_lib.lib(), fn)(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables), _ptr(table_offset),
+    st = call(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables), _ptr(table_offset),
                                  _ptr(token_seq), _ptr(token_pos), _ptr(out), n_tokens, q_heads, kv_heads,
                                  head_dim, block_size, C.c_float(scale), ws_ptr, ws_bytes, _stream(stream))
     _lib.check(fn, st)
@@ -93,8 +119,8 @@ def launch_attention_mixed(q, k_cache, v_cache, block_tables, table_offset, toke
     llm-engine's forward pass calls launch_attention_decode (src/model/cuda/cuda_model.cu:362-377):
     runs of at least min_run consecutive tokens of one sequence go to the tensor-core prefill kernel,
     the rest to the decode kernels; the split is made on the device."""
-    fn = f"pkv_mixed_attn_{_suffix(k_cache)}"
-    st = getattr(_lib.lib(), fn)(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables), _ptr(table_offset),
+    fn, call = _fn("pkv_mixed_attn_", k_cache)
+    st = call(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables), _ptr(table_offset),
                                  _ptr(token_seq), _ptr(token_pos), _ptr(out), n_tokens, q_heads, kv_heads, head_dim,
                                  block_size, num_blocks, C.c_float(scale), min_run, _ptr(workspace),
                                  workspace.numel() * workspace.element_size(), _stream(stream))
@@ -184,9 +210,9 @@ class DecodePlan:
 
     def attention(self, q, k_cache, v_cache, block_tables, table_offset, token_seq, token_pos, out,
                   block_size: int, scale: float, stream=None) -> None:
-        fn = f"pkv_decode_attn_planned_{_suffix(k_cache)}"
+        fn, call = _fn("pkv_decode_attn_planned_", k_cache)
         p, n = self._ws()
-        st = getattr(_lib.lib(), fn)(C.byref(self.plan), _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables),
+        st = call(C.byref(self.plan), _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables),
                                      _ptr(table_offset), _ptr(token_seq), _ptr(token_pos), _ptr(out), block_size,
                                      C.c_float(scale), p, n, _stream(stream))
         _lib.check(fn, st)
@@ -194,9 +220,9 @@ class DecodePlan:
     def append_attention(self, q, k, v, slots, k_cache, v_cache, block_tables, table_offset, token_seq, token_pos, out,
                          block_size: int, scale: float, stream=None) -> None:
         """launch_store_kv + attention in one chain (decode steps only: one token per sequence)."""
-        fn = f"pkv_append_decode_attn_planned_{_suffix(k_cache)}"
+        fn, call = _fn("pkv_append_decode_attn_planned_", k_cache)
         p, n = self._ws()
-        st = getattr(_lib.lib(), fn)(C.byref(self.plan), _ptr(q), _ptr(k), _ptr(v), _ptr(slots), _ptr(k_cache), _ptr(v_cache),
+        st = call(C.byref(self.plan), _ptr(q), _ptr(k), _ptr(v), _ptr(slots), _ptr(k_cache), _ptr(v_cache),
                                      _ptr(block_tables), _ptr(table_offset), _ptr(token_seq), _ptr(token_pos), _ptr(out),
                                      block_size, C.c_float(scale), p, n, _stream(stream))
         _lib.check(fn, st)
@@ -206,8 +232,8 @@ def launch_attention_prefill(q, k_cache, v_cache, block_tables, table_offset, q_
                              n_tokens: int, n_seqs: int, max_q_len: int, q_heads: int, kv_heads: int, head_dim: int,
                              block_size: int, num_blocks: int, scale: float, stream=None) -> None:
     """Causal attention of each sequence's new chunk over its cached plus new tokens."""
-    fn = f"pkv_prefill_attn_{_suffix(k_cache)}"
-    st = getattr(_lib.lib(), fn)(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables), _ptr(table_offset),
+    fn, call = _fn("pkv_prefill_attn_", k_cache)
+    st = call(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables), _ptr(table_offset),
                                  _ptr(q_start), _ptr(q_len), _ptr(ctx_len), _ptr(out), n_tokens, n_seqs, max_q_len, q_heads,
                                  kv_heads, head_dim, block_size, num_blocks, C.c_float(scale), _stream(stream))
     _lib.check(fn, st)
@@ -216,8 +242,8 @@ def launch_attention_prefill(q, k_cache, v_cache, block_tables, table_offset, q_
 def launch_copy_blocks(k_cache, v_cache, src_dst_pairs, n_pairs: int, block_size: int, kv_dim: int,
                        stream=None) -> None:
     """Copy-on-write: block pairs[2i] -> block pairs[2i+1] in both pools."""
-    fn = f"pkv_copy_blocks_{_suffix(k_cache)}"
-    st = getattr(_lib.lib(), fn)(_ptr(k_cache), _ptr(v_cache), _ptr(src_dst_pairs), n_pairs, block_size, kv_dim,
+    fn, call = _fn("pkv_copy_blocks_", k_cache)
+    st = call(_ptr(k_cache), _ptr(v_cache), _ptr(src_dst_pairs), n_pairs, block_size, kv_dim,
                                  _stream(stream))
     _lib.check(fn, st)
 
