@@ -365,10 +365,10 @@ int persistent_sms() {
 
 template <typename T, int D, int NT, int MT, int NSTAGES, int WARPS, int MINB, int TOK = 1, bool FUSED = false>
 int launch_tma(const DecodeArgs& a, int grid, cudaStream_t stream) {
-  if constexpr (TOK == 1 && !FUSED) {
+  if constexpr (TOK == 1 && !FUSED && !IsF32<T>::value) {
     if (a.new_k != nullptr) return launch_tma<T, D, NT, MT, NSTAGES, WARPS, MINB, 1, true>(a, grid, stream);
   }
-  using S = TmaSmem<D, MT, NSTAGES, WARPS>;
+  using S = TmaSmem<D, MT, NSTAGES, WARPS, sizeof(T)>;
   auto kern = decode_tma_kernel<T, D, NT, MT, NSTAGES, WARPS, MINB, TOK, FUSED>;
   static thread_local int configured_device = -1;
   int dev = 0;
@@ -379,11 +379,11 @@ int launch_tma(const DecodeArgs& a, int grid, cudaStream_t stream) {
     configured_device = dev;
   }
   alignas(64) CUtensorMap kmap, vmap;
-  constexpr bool is_bf16 = !std::is_same<T, __half>::value;
+  constexpr PoolElem elem = IsF32<T>::value ? PoolElem::kF32 : std::is_same<T, __half>::value ? PoolElem::kF16 : PoolElem::kBF16;
   const int kv_dim = a.kv_heads * a.head_dim;
-  int st = make_pool_tensor_map(&kmap, a.k_cache, is_bf16, kv_dim, 16, a.pool_rows);
+  int st = make_pool_tensor_map(&kmap, a.k_cache, elem, kv_dim, 16, a.pool_rows);
   if (st != PKV_OK) return st;
-  st = make_pool_tensor_map(&vmap, a.v_cache, is_bf16, kv_dim, 16, a.pool_rows);
+  st = make_pool_tensor_map(&vmap, a.v_cache, elem, kv_dim, 16, a.pool_rows);
   if (st != PKV_OK) return st;
   // `grid` counts work units; every warp is a worker and blocks are persistent:
   // as many as can be resident, each warp striding through the unit list.
@@ -403,8 +403,10 @@ std::atomic<unsigned long long> g_cluster_launches{0};   // pkv_debug_cluster_la
 template <typename T, bool FUSED>
 int launch_tma_cluster_impl(const DecodeArgs& a, int cs, cudaStream_t stream, bool* launched) {
   constexpr int WARPS = 4;
-  using S = TmaSmem<64, 2, 2, WARPS>;
-  auto kern = decode_tma_kernel<T, 64, 1, 2, 2, WARPS, 3, 1, FUSED, true>;
+  // (fp32: slabs of 16 keys are as many bytes as 32 16-bit ones; its query rows and the landing area leave room for two blocks per SM)
+  constexpr int MT = IsF32<T>::value ? 1 : 2;
+  using S = TmaSmem<64, MT, 2, WARPS, sizeof(T)>;
+  auto kern = decode_tma_kernel<T, 64, 1, MT, 2, WARPS, IsF32<T>::value ? 2 : 3, 1, FUSED, true>;
   *launched = false;
   const long long pairs = static_cast<long long>(a.n_tokens) * a.kv_heads;
   if (!cluster_size_ok(cs) || pairs * cs > 0x7fffffffll) return PKV_OK;
@@ -440,11 +442,11 @@ int launch_tma_cluster_impl(const DecodeArgs& a, int cs, cudaStream_t stream, bo
   }
   if (pairs > max_clusters[cs]) return PKV_OK;
   alignas(64) CUtensorMap kmap, vmap;
-  constexpr bool is_bf16 = !std::is_same<T, __half>::value;
+  constexpr PoolElem elem = IsF32<T>::value ? PoolElem::kF32 : std::is_same<T, __half>::value ? PoolElem::kF16 : PoolElem::kBF16;
   const int kv_dim = a.kv_heads * a.head_dim;
-  int st = make_pool_tensor_map(&kmap, a.k_cache, is_bf16, kv_dim, 16, a.pool_rows);
+  int st = make_pool_tensor_map(&kmap, a.k_cache, elem, kv_dim, 16, a.pool_rows);
   if (st != PKV_OK) return st;
-  st = make_pool_tensor_map(&vmap, a.v_cache, is_bf16, kv_dim, 16, a.pool_rows);
+  st = make_pool_tensor_map(&vmap, a.v_cache, elem, kv_dim, 16, a.pool_rows);
   if (st != PKV_OK) return st;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
   cudaLaunchKernelEx(&cfg, kern, a, kmap, vmap);
@@ -456,12 +458,18 @@ int launch_tma_cluster_impl(const DecodeArgs& a, int cs, cudaStream_t stream, bo
 template <typename T>
 int launch_tma_cluster(const DecodeArgs& a, int cs, cudaStream_t stream, bool* launched) {
   *launched = false;
-  if constexpr (IsF32<T>::value) {
-    return PKV_OK;
-  } else {
+  if constexpr (!IsF32<T>::value) {
     if (a.new_k != nullptr) return launch_tma_cluster_impl<T, true>(a, cs, stream, launched);
-    return launch_tma_cluster_impl<T, false>(a, cs, stream, launched);
   }
+  if constexpr (IsF32<T>::value) {
+    // the planner counts on three resident blocks per SM: take the largest size that two hold
+    for (; cs >= 2; --cs) {
+      const int st = cluster_size_ok(cs) ? launch_tma_cluster_impl<T, false>(a, cs, stream, launched) : PKV_OK;
+      if (st != PKV_OK || *launched) return st;
+    }
+    return PKV_OK;
+  }
+  return launch_tma_cluster_impl<T, false>(a, cs, stream, launched);
 }
 
 template <typename T, int DJ>
@@ -495,8 +503,7 @@ int launch_combine(const DecodeArgs& a, cudaStream_t stream) {
 // Whether this geometry runs on decode_tma_kernel.
 template <typename T>
 bool tma_path(const DecodeArgs& a) {
-  if constexpr (IsF32<T>::value) return false;
-  return (a.head_dim == 64 || a.head_dim == 128) && a.group <= 16 && a.bs_log2 >= 4 && a.scale > 0.f && tuning().use_tma &&
+  return (a.head_dim == 64 || a.head_dim == 128) && a.group <= (IsF32<T>::value ? 8 : 16) && a.bs_log2 >= 4 && a.scale > 0.f && tuning().use_tma &&
          tensor_map_encoder() != nullptr;
 }
 
@@ -534,6 +541,10 @@ int launch_decode_main(const DecodeArgs& a, int grid, cudaStream_t stream, bool*
     }
   }
   *log2_domain = false;
+  if constexpr (IsF32<T>::value) {
+    if (tma_path<T>(a))
+      return a.head_dim == 64 ? launch_tma<T, 64, 1, 1, 2, 4, 3>(a, grid, stream) : launch_tma<T, 128, 1, 1, 2, 3, 2>(a, grid, stream);
+  }
   const int dj = (a.head_dim + 31) / 32;
   if (dj <= 2) return launch_simt<T, 2>(a, grid, stream);
   if (dj <= 4) return launch_simt<T, 4>(a, grid, stream);

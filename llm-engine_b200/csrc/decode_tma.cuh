@@ -1,5 +1,5 @@
-// Paged decode attention, TMA variant (sm_100a): 16-bit K/V, head_dim 64 or 128,
-// GQA group <= 16, block_size a multiple of 16.
+// Paged decode attention, TMA variant (sm_100a): head_dim 64 or 128, block_size a multiple
+// of 16, 16-bit K/V with a GQA group of up to 16 or fp32 K/V with one of up to 8.
 //
 // Work unit = (token, key range) x kv head.  Every WARP is an independent worker:
 // it owns a private ring of shared-memory stages, fetches its own units, and
@@ -20,6 +20,7 @@
 //           in the thread that owns its accumulator column -- no cross-lane traffic
 //           for the rescale, three shuffles per slab for the running maximum, one
 //           movmatrix per 8x8 block of P.
+//           fp32 K/V: fp32 arithmetic throughout (packed fused multiply-adds), see there.
 //   finish  a unit that covers its token's whole history writes the output rows; any
 //           other writes its split-K partial, fire and forget; decode_combine_kernel
 //           (decode_attn.cuh) merges the partials afterwards.
@@ -45,12 +46,13 @@ struct WarpGroup {
   static __device__ __forceinline__ int tid() { return threadIdx.x & 31; }
 };
 
-template <int D, int MT, int NSTAGES, int WARPS> struct TmaSmem {
-  static constexpr int kHalves = D / 64;
+template <int D, int MT, int NSTAGES, int WARPS, int ELEM = 2> struct TmaSmem {
+  static constexpr int kHalves = D * ELEM / 128;             // 128-byte boxes side by side in a row
   static constexpr int kKBytes = MT * kHalves * kBoxBytes;  // K part of a stage; V follows
   static constexpr int kStageBytes = 2 * kKBytes;
   static constexpr int kWarpBytes = NSTAGES * kStageBytes;
-  static constexpr int kBytes = WARPS * kWarpBytes + 1024;
+  static constexpr int kQBytes = ELEM == 4 ? 8 * (D + 4) * 4 : 0;   // fp32: a warp's query rows, behind the rings
+  static constexpr int kBytes = WARPS * (kWarpBytes + kQBytes) + 1024;
 };
 
 // TOK = 1: a unit serves one token.  TOK = 4: a unit serves up to four tokens whose sequences
@@ -89,12 +91,24 @@ __device__ __forceinline__ void cluster_push4(uint32_t dst_cluster_addr, float4 
                : "memory");
 }
 
+// (a.x, a.y) * (b.x, b.y) + (c.x, c.y), each rounded once, in one instruction.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n .reg .b64 ra, rb, rc, rd;\n mov.b64 ra, {%2, %3};\n mov.b64 rb, {%4, %5};\n mov.b64 rc, {%6, %7};\n"
+      " fma.rn.f32x2 rd, ra, rb, rc;\n mov.b64 {%0, %1}, rd;\n}\n"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+
 template <typename T, int D, int NT, int MT, int NSTAGES, int WARPS, int MIN_BLOCKS, int TOK = 1, bool FUSED_APPEND = false,
           bool CLUSTER = false>
 __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
     decode_tma_kernel(const DecodeArgs a, const __grid_constant__ CUtensorMap kmap,
                       const __grid_constant__ CUtensorMap vmap) {
-  using S = TmaSmem<D, MT, NSTAGES, WARPS>;
+  using S = TmaSmem<D, MT, NSTAGES, WARPS, sizeof(T)>;
+  constexpr bool F32 = sizeof(T) == 4;
+  static_assert(!F32 || (NT == 1 && MT == 1 && TOK == 1 && !FUSED_APPEND), "fp32: up to 8 heads, slabs of 16 keys");
   static_assert(TOK == 1 || TOK == 4, "a shared unit holds four tokens");
   static_assert(NT % TOK == 0, "whole head tiles per token");
   static_assert(!CLUSTER || TOK == 1, "cluster launches take ordinary tokens");
@@ -104,6 +118,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
   constexpr int KS = D / 16;
   constexpr int HALVES = S::kHalves;
   constexpr int SLAB = 16 * MT;
+  constexpr int kBoxCols = 128 / static_cast<int>(sizeof(T));
   constexpr float kLog2e = 1.4426950408889634f;
 
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -237,7 +252,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
       if constexpr (TOK == 1) {
         const char* qrow = reinterpret_cast<const char*>(static_cast<const T*>(a.q) +
                                                          (static_cast<size_t>(token) * a.q_heads + kvh * a.group) * D);
-        if (lane * 128 < a.group * D * 2) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(qrow + lane * 128));
+        if (lane * 128 < a.group * D * static_cast<int>(sizeof(T))) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(qrow + lane * 128));
       }
     }
     const int box0 = i_slab * MT;
@@ -276,8 +291,8 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
 #pragma unroll
           for (int h = 0; h < HALVES; ++h) {
             const uint32_t dst = st + (m * HALVES + h) * kBoxBytes;
-            tma_load_2d(dst, &kmap, i_x0 + 64 * h, y, fb);
-            tma_load_2d(dst + S::kKBytes, &vmap, i_x0 + 64 * h, y, fb);
+            tma_load_2d(dst, &kmap, i_x0 + kBoxCols * h, y, fb);
+            tma_load_2d(dst + S::kKBytes, &vmap, i_x0 + kBoxCols * h, y, fb);
           }
         }
       }
@@ -327,7 +342,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
     }
     // Q^T fragments (B operand): rows = dims, columns = heads of the group.
     uint32_t qb[KS][NT][2];
-    {
+    if constexpr (!F32) {
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
         const int ti = nt / NTG;                    // which token of the unit this head tile belongs to
@@ -344,6 +359,30 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
     }
     float o[KS][NT][4];
     float m_run[NT][2], l_run[NT][2];
+    // fp32: lane = (half of the dims, key of the slab) for the scores, whose running maximum and (this
+    // key's share of the) sum it keeps for four heads, and = 2 or 4 dims of all eight heads for the sums.
+    const int f_key = lane & 15, f_part = lane >> 4;
+    float f_m[4], f_l[4];
+    float2 f_o[8][D / 64];
+    float* f_q = reinterpret_cast<float*>(ring_ptr + (WARPS - warp) * S::kWarpBytes + warp * S::kQBytes);
+    if constexpr (F32) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { f_m[i] = -INFINITY; f_l[i] = 0.f; }
+#pragma unroll
+      for (int h = 0; h < 8; ++h)
+#pragma unroll
+        for (int x = 0; x < D / 64; ++x) f_o[h][x] = make_float2(0.f, 0.f);
+      // query rows, zeros past the group; the upper half of a row sits 16 bytes further on, so that the two
+      // halves of the warp read different banks
+      __syncwarp();
+      for (int i = lane; i < 8 * (D / 4); i += 32) {
+        const int h = i / (D / 4), d = 4 * (i - h * (D / 4));
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (h < a.group) x = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(a.q) + (static_cast<size_t>(token) * a.q_heads + kvh * a.group + h) * D + d));
+        *reinterpret_cast<float4*>(f_q + h * (D + 4) + d + (d >= D / 2 ? 4 : 0)) = x;
+      }
+      __syncwarp();
+    }
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
       m_run[nt][0] = m_run[nt][1] = -INFINITY;
@@ -403,6 +442,76 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
         __syncwarp();
       }
 
+      if constexpr (F32) {
+        // Scores: each lane half a row of K against the eight query rows, all from shared memory (16-byte reads:
+        // the K rows swizzled, the query rows broadcast), two partial sums per head.  One slab of 8 KB costs a
+        // warp about 600 issue slots, so twelve warps on an SM keep up with twice its share of HBM.
+        const unsigned char* kp = ring_ptr + slot * S::kStageBytes;
+        const unsigned char* vp = kp + S::kKBytes;
+        float2 s2[8];
+#pragma unroll
+        for (int h = 0; h < 8; ++h) s2[h] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int b = 0; b < HALVES / 2; ++b)
+#pragma unroll
+          for (int ch = 0; ch < 8; ++ch) {
+            const float4 kv = *reinterpret_cast<const float4*>(kp + (f_part * (HALVES / 2) + b) * kBoxBytes + f_key * 128 + ((ch ^ (f_key & 7)) << 4));
+            const float* qd = f_q + f_part * (D / 2 + 4) + b * 32 + ch * 4;
+#pragma unroll
+            for (int h = 0; h < 8; ++h) {
+              const float4 qv = *reinterpret_cast<const float4*>(qd + h * (D + 4));
+              s2[h] = fma2(make_float2(kv.x, kv.y), make_float2(qv.x, qv.y), s2[h]);
+              s2[h] = fma2(make_float2(kv.z, kv.w), make_float2(qv.z, qv.w), s2[h]);
+            }
+          }
+        // the halves of the warp trade halves of the dims for halves of the heads
+        float p[4], al[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float lo = s2[i].x + s2[i].y, hi = s2[4 + i].x + s2[4 + i].y;
+          const float got = __shfl_xor_sync(0xffffffffu, f_part ? lo : hi, 16);
+          const float sc = f_key < rows_valid ? ((f_part ? hi : lo) + got) * a.scale : -INFINITY;
+          float mx = sc;
+#pragma unroll
+          for (int off = 1; off < 16; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+          const float mn = fmaxf(f_m[i], mx);            // finite: key 0 of a slab is valid
+          al[i] = expf(f_m[i] - mn);
+          p[i] = expf(sc - mn);
+          f_l[i] = f_l[i] * al[i] + p[i];
+          f_m[i] = mn;
+        }
+        // weights [key][head] and rescale factors over the K rows, which nothing reads any more
+        float* sp = reinterpret_cast<float*>(ring_ptr + slot * S::kStageBytes);
+        __syncwarp();
+        *reinterpret_cast<float4*>(sp + f_key * 8 + f_part * 4) = make_float4(p[0], p[1], p[2], p[3]);
+        if (f_key == 0) *reinterpret_cast<float4*>(sp + 128 + f_part * 4) = make_float4(al[0], al[1], al[2], al[3]);
+        __syncwarp();
+        {
+          const float4 a0 = *reinterpret_cast<const float4*>(sp + 128), a1 = *reinterpret_cast<const float4*>(sp + 132);
+          const float alpha[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+          for (int h = 0; h < 8; ++h)
+#pragma unroll
+            for (int x = 0; x < D / 64; ++x) { f_o[h][x].x *= alpha[h]; f_o[h][x].y *= alpha[h]; }
+        }
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          float2 v[D / 64];
+          if constexpr (D == 64) {
+            v[0] = *reinterpret_cast<const float2*>(vp + f_part * kBoxBytes + k * 128 + ((((lane & 15) >> 1) ^ (k & 7)) << 4) + (lane & 1) * 8);
+          } else {
+            const float4 w = *reinterpret_cast<const float4*>(vp + (lane >> 3) * kBoxBytes + k * 128 + (((lane & 7) ^ (k & 7)) << 4));
+            v[0] = make_float2(w.x, w.y);
+            v[D / 64 - 1] = make_float2(w.z, w.w);
+          }
+          const float4 p0 = *reinterpret_cast<const float4*>(sp + k * 8), p1 = *reinterpret_cast<const float4*>(sp + k * 8 + 4);
+          const float pk[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+#pragma unroll
+          for (int h = 0; h < 8; ++h)
+#pragma unroll
+            for (int x = 0; x < D / 64; ++x) f_o[h][x] = fma2(make_float2(pk[h], pk[h]), v[x], f_o[h][x]);
+        }
+      } else {
       // S^T = K Q^T : MT m-tiles of 16 keys.
       float s[MT][NT][4];
 #pragma unroll
@@ -485,6 +594,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
           for (int nt = 0; nt < NT; ++nt) mma16816<T>(o[dm][nt], va, pb[mt][nt][0], pb[mt][nt][1]);
         }
       }
+      }
       ++n_consumed;
     }
     if constexpr (!CLUSTER) {
@@ -494,6 +604,38 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
     while (more && n_issued - n_consumed < NSTAGES) more = issue_next();  // keep loads flowing through the finish
 
     // ------------------------------ finish the unit ------------------------------
+    if constexpr (F32) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int off = 1; off < 16; off <<= 1) f_l[i] += __shfl_xor_sync(0xffffffffu, f_l[i], off);
+      const int head0 = kvh * a.group, d0 = lane * (D / 32);
+      if (part < 0) {
+        float* out = reinterpret_cast<float*>(out_row<T>(a, a.out, token)) + static_cast<size_t>(head0) * D + d0;
+#pragma unroll
+        for (int h = 0; h < 8; ++h) {
+          const float inv = 1.f / __shfl_sync(0xffffffffu, f_l[h & 3], (h >> 2) * 16);
+          if (h < a.group)
+#pragma unroll
+            for (int x = 0; x < D / 64; ++x)
+              *reinterpret_cast<float2*>(out + static_cast<size_t>(h) * D + 2 * x) = make_float2(f_o[h][x].x * inv, f_o[h][x].y * inv);
+        }
+      } else {
+        __syncwarp();     // (cluster launches: the partial goes over the ring, which other lanes may still be reading)
+        float* pacc = CLUSTER ? reinterpret_cast<float*>(ring_ptr) : a.part_acc + (static_cast<size_t>(part) * a.q_heads + head0) * D;
+        float* pml = CLUSTER ? reinterpret_cast<float*>(ring_ptr) + 8 * D : a.part_ml + (static_cast<size_t>(part) * a.q_heads + head0) * 2;
+#pragma unroll
+        for (int h = 0; h < 8; ++h)
+          if (h < a.group)
+#pragma unroll
+            for (int x = 0; x < D / 64; ++x) *reinterpret_cast<float2*>(pacc + static_cast<size_t>(h) * D + d0 + 2 * x) = f_o[h][x];
+        if (f_key == 0)
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (4 * f_part + i < a.group) { pml[2 * (4 * f_part + i)] = f_m[i]; pml[2 * (4 * f_part + i) + 1] = f_l[i]; }
+      }
+    }
+    if constexpr (!F32) {
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
 #pragma unroll
@@ -552,6 +694,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
         }
       }
     }
+    }
   }
   if constexpr (!CLUSTER && !FUSED_APPEND) {
     if (a.wait_last) pdl_wait();       // this launch's completion has to imply the previous one's
@@ -560,7 +703,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
     if (c_nsplits > 1) {               // the same for every thread of the cluster
       if (!waited) pdl_wait();         // warps without a range write output rows too
       asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");   // every block's landing barrier is armed
-      const uint32_t land0 = ring0 + WARPS * S::kWarpBytes;                   // landing area: behind the rings
+      const uint32_t land0 = ring0 + WARPS * (S::kWarpBytes + S::kQBytes);    // landing area: behind the rings
       const int ranges_max = WARPS * static_cast<int>(c_size);
       if (c_len > 0) {
         // send this warp's partial, head by head, to the heads' owners: 16 quads of sums and one with
@@ -600,7 +743,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
         for (int sp = 0; sp < c_nsplits; ++sp) {
           const unsigned char* rec = rec0 + sp * kClusterRecord;
           const float2 ml = *reinterpret_cast<const float2*>(rec + 256);
-          const float f = (ml.x == -INFINITY) ? 0.f : exp2f(ml.x - m_run);
+          const float f = (ml.x == -INFINITY) ? 0.f : softmax_exp<!F32>(ml.x - m_run);
           const float2 v = *reinterpret_cast<const float2*>(rec + 4 * d);
           l_run += f * ml.y;
           acc0 += f * v.x;
@@ -608,7 +751,8 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
         }
         const float inv = 1.f / l_run;
         T* o = out_row<T>(a, a.out, c_token) + static_cast<size_t>(c_kvh * a.group + h) * D + d;
-        *reinterpret_cast<uint32_t*>(o) = pack2<T>(acc0 * inv, acc1 * inv);
+        if constexpr (F32) *reinterpret_cast<float2*>(o) = make_float2(acc0 * inv, acc1 * inv);
+        else *reinterpret_cast<uint32_t*>(o) = pack2<T>(acc0 * inv, acc1 * inv);
       }
     }
   }

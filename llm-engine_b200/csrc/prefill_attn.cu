@@ -785,9 +785,9 @@ int prefill_launch(const void* q, const void* k_cache, const void* v_cache, cons
   alignas(64) CUtensorMap qmap, kmap, vmap;
   const int kv_dim = kv_heads * head_dim;
   const uint64_t pool_rows = num_blocks > 0 ? static_cast<uint64_t>(num_blocks) * block_size : (1ull << 30);
-  int st = make_pool_tensor_map(&kmap, k_cache, is_bf16, kv_dim, 16, pool_rows);
+  int st = make_pool_tensor_map(&kmap, k_cache, is_bf16 ? PoolElem::kBF16 : PoolElem::kF16, kv_dim, 16, pool_rows);
   if (st != PKV_OK) return st;
-  st = make_pool_tensor_map(&vmap, v_cache, is_bf16, kv_dim, 16, pool_rows);
+  st = make_pool_tensor_map(&vmap, v_cache, is_bf16 ? PoolElem::kBF16 : PoolElem::kF16, kv_dim, 16, pool_rows);
   if (st != PKV_OK) return st;
   // Heads per tile: the largest divisor of the group, up to 16, that leaves at most 8 of the 128 rows unused
   // (a group of 13 would waste 11: its heads take tiles of their own).

@@ -26,21 +26,22 @@ inline PFN_cuTensorMapEncodeTiled tensor_map_encoder() {
   return fn;
 }
 
-// A K or V pool viewed as a 2-D tensor [rows = slots][cols = kv_dim] of 16-bit
-// elements, fetched in boxes of box_rows x 64 columns (128 bytes) with the
-// 128-byte swizzle, so that consecutive rows of a box land in different
+// A K or V pool viewed as a 2-D tensor [rows = slots][cols = kv_dim], fetched in
+// boxes of box_rows x 128 bytes (64 16-bit or 32 fp32 columns) with the 128-byte swizzle, so that consecutive rows of a box land in different
 // shared-memory banks for ldmatrix.  The pool's slot count is not part of the
 // launcher signature; rows is therefore an upper bound used only for the
 // hardware's out-of-bounds check and block tables must name real blocks.
-inline int make_pool_tensor_map(CUtensorMap* map, const void* pool, bool is_bf16, int kv_dim, uint32_t box_rows,
+enum class PoolElem { kF16, kBF16, kF32 };
+inline int make_pool_tensor_map(CUtensorMap* map, const void* pool, PoolElem elem, int kv_dim, uint32_t box_rows,
                                 uint64_t rows_bound) {
+  const cuuint32_t bytes = elem == PoolElem::kF32 ? 4 : 2;
   PFN_cuTensorMapEncodeTiled enc = tensor_map_encoder();
   if (!enc) return fail(PKV_E_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(kv_dim), rows_bound};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(kv_dim) * 2};
-  const cuuint32_t box[2] = {64, box_rows};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(kv_dim) * bytes};
+  const cuuint32_t box[2] = {128 / bytes, box_rows};
   const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = enc(map, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
+  const CUresult r = enc(map, elem == PoolElem::kF32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : elem == PoolElem::kBF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
                          const_cast<void*>(pool), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);

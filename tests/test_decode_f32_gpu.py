@@ -1,0 +1,40 @@
+"""fp32 K/V on the TMA decode kernel against the CPU checker, 1e-5: group sizes below its eight head columns, both
+head dims, slab edges (16 keys), whole-history units, chunks, shares and the cluster form."""
+import numpy as np
+import pytest
+
+from tests.gpu_util import Case, check_case
+
+pytestmark = pytest.mark.gpu
+
+
+def make(orc, pkv, qh, kvh, hd, bs, ctx, seed):
+    nb = sum((c + bs) // bs for c in ctx) + 9
+    return Case(orc, "f32", qh, kvh, hd, bs, nb, ctx, [1] * len(ctx), seed=seed, pkv=pkv)
+
+
+@pytest.mark.parametrize("qh,kvh", [(2, 2), (6, 2), (4, 1), (10, 2), (14, 2), (16, 2)])
+@pytest.mark.parametrize("hd,bs", [(64, 16), (64, 64), (128, 16), (128, 32)])
+def test_groups_and_slab_edges(pkv, orc, torch_cuda, qh, kvh, hd, bs):
+    ctx = [0, 1, 14, 15, 16, 17, 31, 32, 47, 127, 128, 129, 300]
+    case = make(orc, pkv, qh, kvh, hd, bs, ctx, seed=qh + hd)
+    for mode in ("direct", "split", "device_plan"):
+        check_case(case, pkv, torch_cuda, orc, mode)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_shares(pkv, orc, torch_cuda, hd):
+    """Enough keys that the plan is cut into one share per warp; more shares than resident warps at 128 dims."""
+    ctx = [int(x) for x in np.random.default_rng(2).integers(200, 9000, size=40)]
+    case = make(orc, pkv, 8, 4, hd, 16, ctx, seed=3)
+    for mode in ("host_plan", "device_plan"):
+        check_case(case, pkv, torch_cuda, orc, mode)
+
+
+@pytest.mark.parametrize("ctx", [[511] * 8, [333], [0, 2000, 15, 16, 17, 700], list(range(120, 160))])
+def test_cluster_form(pkv, orc, torch_cuda, ctx):
+    case = make(orc, pkv, 14, 2, 64, 16, ctx, seed=4)
+    d = case.run_gpu(pkv, torch_cuda, "host_plan")
+    before = pkv.lib().pkv_debug_cluster_launches()
+    check_case(case, pkv, torch_cuda, orc, "host_plan")
+    assert d["plan"].plan.cluster >= 2 and pkv.lib().pkv_debug_cluster_launches() == before + 1
