@@ -21,6 +21,7 @@ static __device__ __align__(256) unsigned char g_builtin_scratch[kBuiltinScratch
 
 namespace pkv {
 int prefill_read_flags(unsigned int* flags);  // prefill_attn.cu
+int copy_read_flags(unsigned int* flags);     // copy_blocks.cu
 template <typename T>
 int prefill_launch(const void* q, const void* k_cache, const void* v_cache, const int* block_tables,
                    const int* table_offset, const int* q_start, const int* q_len, const int* ctx_len, void* out,
@@ -902,10 +903,11 @@ int pkv_debug_device_flags(unsigned int* flags) {
   cudaError_t e = cudaMemcpyFromSymbol(&v, g_pkv_device_error, sizeof(v));
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_pkv_device_error, &zero, sizeof(zero));
   if (e != cudaSuccess) return fail(PKV_E_CUDA, "pkv_debug_device_flags: %s", cudaGetErrorString(e));
-  unsigned int pf = 0;
-  const int st = pkv::prefill_read_flags(&pf);
+  unsigned int pf = 0, cf = 0;
+  int st = pkv::prefill_read_flags(&pf);
+  if (st == PKV_OK) st = pkv::copy_read_flags(&cf);
   if (st != PKV_OK) return st;
-  *flags = v | pf | pkv::take_error_mirror();
+  *flags = v | pf | cf | pkv::take_error_mirror();
   return PKV_OK;
 }
 
