@@ -38,3 +38,36 @@ def test_many_sequences(pkv, orc, torch_cuda, n_seqs):
 def test_equal_lengths(pkv, orc, torch_cuda):
     """Every tile of a rank has the same length as its neighbours: one bucket, many ties."""
     check(pkv, orc, torch_cuda, 8, 1, [64] * 24, [48] * 24, seed=6)
+
+
+@pytest.mark.parametrize("qh,kvh", [(14, 2), (8, 1), (26, 2), (32, 4)])
+@pytest.mark.parametrize("ctx,new", [
+    ([3000], [1]),                       # one tile, all eight blocks of a cluster on it
+    ([0], [250]),                        # parts of the keys that early rows do not see
+    ([5000, 64, 127], [33, 17, 60]),     # long and short items in one launch
+    ([700, 900, 1100], [70, 71, 140]),   # two and four blocks per item
+    ([63], [1]), ([64], [2]),            # around one key tile: nothing to share
+])
+def test_few_items_share_their_keys(pkv, orc, torch_cuda, qh, kvh, ctx, new):
+    check(pkv, orc, torch_cuda, qh, kvh, ctx, new, seed=7)
+
+
+def test_split_launch_replays_from_a_graph(pkv, orc, torch_cuda):
+    torch = torch_cuda
+    case = make_case(orc, pkv, "bf16", 14, 2, 16, [2000, 900], [40, 25], seed=8)
+    d = run_prefill(pkv, torch, case)
+    want = d["out"].clone()
+    i32 = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.int32)).cuda()
+    args = (i32([0, 40]), i32([40, 25]), i32([2000, 900]))
+    out = torch.zeros_like(want)
+    call = lambda: pkv.launch_attention_prefill(d["q"], d["kc"], d["vc"], d["block_tables"], d["table_offset"], *args, out,
+                                                case.N, 2, 40, 14, 2, 64, 16, case.nb, case.scale)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        for _ in range(5):
+            call()
+    for _ in range(3):
+        out.zero_()
+        g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want) and pkv.debug_device_flags() == 0
