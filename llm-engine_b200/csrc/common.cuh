@@ -83,6 +83,86 @@ __device__ __forceinline__ uint4 ld_nc_u4(const void* p) {
   return v;
 }
 
+// ---- integer scans -----------------------------------------------------------------
+struct ScanSum { static __device__ __forceinline__ int op(int a, int b) { return a + b; } };
+struct ScanMax { static __device__ __forceinline__ int op(int a, int b) { return max(a, b); } };
+template <typename Op>
+__device__ __forceinline__ int warp_scan(int v, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v = Op::op(v, x);
+  }
+  return v;
+}
+// Inclusive scan over a block of WARPS full warps, one value per thread.  `sm` holds one word per warp and is
+// free for the next scan only after another barrier; *total receives the block's result.
+template <typename Op, int WARPS>
+__device__ __forceinline__ int block_scan(int v, int* sm, int* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  v = warp_scan<Op>(v, lane);
+  if (lane == 31) sm[warp] = v;
+  __syncthreads();
+  const int w = warp_scan<Op>(sm[min(lane, WARPS - 1)], lane);   // every warp scans the totals for itself: one barrier
+  const int before = __shfl_sync(0xffffffffu, w, max(warp - 1, 0));
+  *total = __shfl_sync(0xffffffffu, w, WARPS - 1);
+  return warp ? Op::op(before, v) : v;
+}
+
+// ---- runs of a packed step ---------------------------------------------------------
+// A run is a maximal stretch of packed tokens of one sequence at consecutive positions.  Called by every thread
+// of a block of WARPS warps for n <= PER * 32 WARPS tokens; each thread gets PER consecutive tokens from
+// tid * ceil(n / threads), fewer at the end (first, count), with their positions, sequences and run lengths;
+// start_of holds the first token of each one's run.  pos, seq and scratch are shared-memory arrays of n words, `sm`
+// one of WARPS; ends without a barrier (the arrays may be reused after one).
+template <int WARPS, int PER> struct TokenRuns {
+  int first, count;
+  int pos[PER], seq[PER], start_of[PER], len[PER];
+  __device__ __forceinline__ void find(const int* __restrict__ token_pos, const int* __restrict__ token_seq, int n, int* s_pos,
+                                       int* s_seq, int* scratch, int* sm) {
+    constexpr int kThreads = 32 * WARPS;
+    for (int t = threadIdx.x; t < n; t += kThreads) {
+      s_pos[t] = token_pos[t];
+      s_seq[t] = token_seq[t];
+    }
+    __syncthreads();
+    const int per = (n + kThreads - 1) / kThreads;
+    first = threadIdx.x * per;
+    count = max(0, min(per, n - first));
+    auto starts = [&](int t) { return t == 0 || s_seq[t - 1] != s_seq[t] || s_pos[t - 1] + 1 != s_pos[t]; };
+    int last = -1;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      pos[i] = 0; seq[i] = 0; start_of[i] = -1; len[i] = 0;
+      if (i < count) {
+        pos[i] = s_pos[first + i];
+        seq[i] = s_seq[first + i];
+        if (starts(first + i)) last = first + i;
+        start_of[i] = last;
+      }
+    }
+    int total;
+    const int upto = block_scan<ScanMax, WARPS>(last, sm, &total);
+    int before = __shfl_up_sync(0xffffffffu, upto, 1);
+    if ((threadIdx.x & 31) == 0) {                       // the inclusive result of the warp before
+      before = -1;
+      for (int w = 0; w < static_cast<int>(threadIdx.x >> 5); ++w) before = max(before, sm[w]);
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      if (i < count) {
+        if (start_of[i] < 0) start_of[i] = before;
+        const int t = first + i;
+        if (t == n - 1 || starts(t + 1)) scratch[start_of[i]] = t - start_of[i] + 1;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+      if (i < count) len[i] = scratch[start_of[i]];
+  }
+};
+
 __device__ __forceinline__ float warp_sum(float x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);

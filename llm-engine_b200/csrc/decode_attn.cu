@@ -26,7 +26,7 @@ template <typename T>
 int prefill_launch(const void* q, const void* k_cache, const void* v_cache, const int* block_tables,
                    const int* table_offset, const int* q_start, const int* q_len, const int* ctx_len, void* out,
                    int n_tokens, int n_seqs, int max_q_len, int q_heads, int kv_heads, int head_dim, int block_size,
-                   int num_blocks, float scale, pkv_stream stream, const int* d_dims, bool may_allocate);
+                   int num_blocks, float scale, pkv_stream stream, const int* d_dims, bool may_allocate, const InlineRuns* runs);
 unsigned int* error_mirror(bool create);      // error_mirror.cu
 unsigned int take_error_mirror();
 int check_error_mirror(const char* fn);
@@ -100,31 +100,6 @@ struct RouteArgs {
   int* dims;        // [4] out: runs, tokens of the longest, tokens of none
 };
 
-// Inclusive scans over the block's threads, one value each (sum, or maximum).  `sm` holds one word per
-// warp and is free for the next scan only after another barrier; *total receives the block's result.
-struct ScanSum { static __device__ __forceinline__ int op(int a, int b) { return a + b; } };
-struct ScanMax { static __device__ __forceinline__ int op(int a, int b) { return max(a, b); } };
-template <typename Op>
-__device__ __forceinline__ int warp_scan(int v, int lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int x = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v = Op::op(v, x);
-  }
-  return v;
-}
-template <typename Op>
-__device__ __forceinline__ int block_scan(int v, int* sm, int* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  v = warp_scan<Op>(v, lane);
-  if (lane == 31) sm[warp] = v;
-  __syncthreads();
-  const int w = warp_scan<Op>(sm[lane], lane);        // every warp scans the 32 warp totals for itself: one barrier
-  const int before = __shfl_sync(0xffffffffu, w, max(warp - 1, 0));
-  *total = __shfl_sync(0xffffffffu, w, 31);
-  return warp ? Op::op(before, v) : v;
-}
-
 // One block: all of it is latency (a step of 600 tokens reads 5 KB), so a step of up to kPlanThreads
 // tokens keeps everything a token needs in its thread's registers and run lengths in shared memory, and
 // every scan costs one barrier.
@@ -167,7 +142,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
         sm_start[t] = start;
       }
       int tot;
-      const int rs = block_scan<ScanMax>(start ? t : -1, sm_scan[0], &tot);
+      const int rs = block_scan<ScanMax, kPlanThreads / 32>(start ? t : -1, sm_scan[0], &tot);
       if (t < n_tokens && sm_start[t + 1]) sm_len[rs] = t - rs + 1;   // the run's last token
       __syncthreads();
       int flag = 0, len = 0;
@@ -177,7 +152,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
         my_len = long_run ? 0 : max(pos, 0) + 1;
         flag = long_run && start;
       }
-      const int i = block_scan<ScanSum>(flag, sm_scan[1], &tot) - 1;
+      const int i = block_scan<ScanSum, kPlanThreads / 32>(flag, sm_scan[1], &tot) - 1;
       if (flag) {
         r.q_start[i] = t;
         r.q_len[i] = len;
@@ -193,7 +168,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
       for (int base = 0; base < n_tokens; base += kPlanThreads) {
         const int t = base + tid;
         int tot;
-        const int v = max(block_scan<ScanMax>((t < n_tokens && is_start(t)) ? t : -1, sm_scan[0], &tot), carry);
+        const int v = max(block_scan<ScanMax, kPlanThreads / 32>((t < n_tokens && is_start(t)) ? t : -1, sm_scan[0], &tot), carry);
         if (t < n_tokens) r.run_start[t] = v;
         carry = max(carry, tot);
         __syncthreads();
@@ -220,7 +195,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
           flag = long_run && rs == t;
         }
         int tot;
-        const int i = runs + block_scan<ScanSum>(flag, sm_scan[1], &tot) - 1;
+        const int i = runs + block_scan<ScanSum, kPlanThreads / 32>(flag, sm_scan[1], &tot) - 1;
         if (flag) {
           r.q_start[i] = t;
           r.q_len[i] = len;
@@ -248,7 +223,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
   if (small) {
     int tot;
     const int p = share_padded(my_len) / kShareSlab;       // scanned in slabs: 32 bits hold 2^36 keys
-    my_begin = static_cast<long long>(block_scan<ScanSum>(p, sm_scan[2], &tot) - p) * kShareSlab;
+    my_begin = static_cast<long long>(block_scan<ScanSum, kPlanThreads / 32>(p, sm_scan[2], &tot) - p) * kShareSlab;
     total = static_cast<long long>(tot) * kShareSlab;
   } else {
     long long loc = 0;
@@ -271,7 +246,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
     long long begin = my_begin;
     if (!small) {
       const int p = padded / kShareSlab;
-      begin = carry_begin + static_cast<long long>(block_scan<ScanSum>(p, sm_scan[2], &tot) - p) * kShareSlab;
+      begin = carry_begin + static_cast<long long>(block_scan<ScanSum, kPlanThreads / 32>(p, sm_scan[2], &tot) - p) * kShareSlab;
       carry_begin += static_cast<long long>(tot) * kShareSlab;
     }
     int ns = 0;
@@ -286,8 +261,8 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
     }
     const int np = ns > 1 ? ns : 0;
     int tot_items, tot_parts;
-    const int item0 = n_items + block_scan<ScanSum>(ns, sm_scan[3], &tot_items) - ns;
-    const int part0 = n_parts + block_scan<ScanSum>(np, sm_scan[4], &tot_parts) - np;
+    const int item0 = n_items + block_scan<ScanSum, kPlanThreads / 32>(ns, sm_scan[3], &tot_items) - ns;
+    const int part0 = n_parts + block_scan<ScanSum, kPlanThreads / 32>(np, sm_scan[4], &tot_parts) - np;
     if (t < n_tokens) {
       tok_split[t] = TokSplit{part0, ns};
       for (int s = 0; s < ns; ++s) {
@@ -364,19 +339,23 @@ int persistent_sms() {
   return sms;
 }
 
-template <typename T, int D, int NT, int MT, int NSTAGES, int WARPS, int MINB, int TOK = 1, bool FUSED = false>
+template <typename T, int D, int NT, int MT, int NSTAGES, int WARPS, int MINB, int TOK = 1, bool FUSED = false, bool INLINE = false>
 int launch_tma(const DecodeArgs& a, int grid, cudaStream_t stream) {
-  if constexpr (TOK == 1 && !FUSED && !IsF32<T>::value) {
+  if constexpr (TOK == 1 && !FUSED && !INLINE && !IsF32<T>::value) {
     if (a.new_k != nullptr) return launch_tma<T, D, NT, MT, NSTAGES, WARPS, MINB, 1, true>(a, grid, stream);
+    if constexpr (D == 64 && WARPS == 4) {
+      if (a.inline_min_run > 0) return launch_tma<T, D, NT, MT, NSTAGES, WARPS, MINB, 1, false, true>(a, grid, stream);
+    }
   }
   using S = TmaSmem<D, MT, NSTAGES, WARPS, sizeof(T)>;
-  auto kern = decode_tma_kernel<T, D, NT, MT, NSTAGES, WARPS, MINB, TOK, FUSED>;
+  auto kern = decode_tma_kernel<T, D, NT, MT, NSTAGES, WARPS, MINB, TOK, FUSED, false, INLINE>;
+  constexpr int kSmem = S::kBytes + (INLINE ? InlinePlan::kBytes : 0);
   static thread_local int configured_device = -1;
   int dev = 0;
   cudaGetDevice(&dev);
   if (configured_device != dev) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
-    if (e != cudaSuccess) return fail(PKV_E_CUDA, "decode: cannot reserve %d bytes of shared memory: %s", S::kBytes, cudaGetErrorString(e));
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    if (e != cudaSuccess) return fail(PKV_E_CUDA, "decode: cannot reserve %d bytes of shared memory: %s", kSmem, cudaGetErrorString(e));
     configured_device = dev;
   }
   alignas(64) CUtensorMap kmap, vmap;
@@ -391,7 +370,7 @@ int launch_tma(const DecodeArgs& a, int grid, cudaStream_t stream) {
   int blocks = (grid + WARPS - 1) / WARPS;
   const int resident = persistent_sms() * MINB;
   if (blocks > resident) blocks = resident;
-  launch_pdl(kern, dim3(blocks), dim3(WARPS * 32), S::kBytes, stream, a, kmap, vmap);
+  launch_pdl(kern, dim3(blocks), dim3(WARPS * 32), kSmem, stream, a, kmap, vmap);
   return check_launch("decode_tma_kernel");
 }
 
@@ -628,6 +607,7 @@ void fill_args(DecodeArgs& a, const void* q, const void* kc, const void* vc, con
   a.new_k = nullptr; a.new_v = nullptr; a.slots = nullptr;
   a.host_err = nullptr;
   a.wait_last = 0;
+  a.inline_min_run = 0; a.inline_max_shares = 0; a.inline_forced_chunk = 0;
   a.pool_rows = 1ull << 30;
 }
 
@@ -711,7 +691,7 @@ template <typename T>
 int decode_planned(const pkv_decode_plan* plan, const void* q, const void* kc, const void* vc, const int* bt,
                    const int* to, const int* ts, const int* tp, void* out, int block_size, float scale,
                    void* workspace, size_t workspace_bytes, pkv_stream stream, const PeerSetup* peers = nullptr,
-                   const FusedAppend* app = nullptr, bool may_allocate = true, bool wait_last = false) {
+                   const FusedAppend* app = nullptr, bool may_allocate = true, bool wait_last = false, int inline_min_run = 0) {
   const char* fn = peers ? "pkv_decode_attn_planned_peer" : (app ? "pkv_append_decode_attn_planned" : "pkv_decode_attn_planned");
   if (!plan) return fail(PKV_E_ARG, "%s: null plan", fn);
   if (plan->n_tokens <= 0) return PKV_OK;
@@ -723,13 +703,19 @@ int decode_planned(const pkv_decode_plan* plan, const void* q, const void* kc, c
   if (st != PKV_OK) return st;
   if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255)) return fail(PKV_E_ARG, "%s: workspace null or not 256-byte aligned", fn);
   WsLayout w;
-  if (plan_budget(plan->n_tokens, plan->q_heads, plan->kv_heads, plan->head_dim, workspace_bytes, &w) < 0)
+  const int budget = plan_budget(plan->n_tokens, plan->q_heads, plan->kv_heads, plan->head_dim, workspace_bytes, &w);
+  if (budget < 0)
     return fail(PKV_E_WORKSPACE, "%s: workspace of %zu bytes is smaller than the plan it should hold", fn, workspace_bytes);
   DecodeArgs a;
   fill_args(a, q, kc, vc, bt, to, ts, tp, out, plan->n_tokens, plan->q_heads, plan->kv_heads, plan->head_dim, block_size, scale);
   attach_workspace(a, workspace, w);
   a.host_err = error_mirror(may_allocate);
   a.wait_last = wait_last ? 1 : 0;
+  if (inline_min_run > 0) {
+    a.inline_min_run = inline_min_run;
+    a.inline_max_shares = max_shares_for(budget, decode_workers(a.q_heads, a.kv_heads, a.head_dim) / a.kv_heads);
+    a.inline_forced_chunk = tuning().forced_chunk;
+  }
   if (plan->num_blocks > 0) a.pool_rows = static_cast<unsigned long long>(plan->num_blocks) * block_size;
   if (peers) {
     if constexpr (sizeof(T) != 2) return fail(PKV_E_UNSUPPORTED, "%s: the head-sharded exchange is for 16-bit outputs", fn);
@@ -852,6 +838,14 @@ int mixed_attn(const void* q, const void* kc, const void* vc, const int* bt, con
   st = validate_pointers(fn, q, kc, vc, bt, to, ts, tp, out, sizeof(T) * static_cast<size_t>(head_dim));
   if (st != PKV_OK) return st;
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return fail(PKV_E_ARG, "%s: workspace must be 256-byte aligned", fn);
+  // Short enough for every block of both kernels to find the runs and the plan for itself: two launches and the
+  // merge.  (Longer steps, and geometries whose decode tokens do not run on the TMA kernel, get the planner.)
+  bool inline_plan = false;
+  {
+    DecodeArgs probe;
+    fill_args(probe, q, kc, vc, bt, to, ts, tp, out, n_tokens, q_heads, kv_heads, head_dim, block_size, scale);
+    inline_plan = n_tokens <= kInlineTokens && n_tokens / min_run <= kInlineRuns && tma_path<T>(probe) && tuning().variant < 4;
+  }
   const RouteLayout rl = route_layout(n_tokens);
   if (workspace_bytes < rl.total + ws_layout(n_tokens, q_heads, kv_heads, head_dim, 0).total)
     return fail(PKV_E_WORKSPACE, "%s: workspace of %zu bytes is too small for a step of %d tokens (pkv_mixed_attn_workspace_bytes)",
@@ -871,8 +865,17 @@ int mixed_attn(const void* q, const void* kc, const void* vc, const int* bt, con
   r.dims = reinterpret_cast<int*>(rbase + rl.off_dims);
   pkv_decode_plan plan;
   std::memset(&plan, 0, sizeof(plan));
-  st = plan_device(tp, n_tokens, q_heads, kv_heads, head_dim, workspace, dec_bytes, static_cast<cudaStream_t>(stream), &plan, &r);
-  if (st != PKV_OK) return st;
+  if (inline_plan) {
+    WsLayout w;
+    const int budget = plan_budget(n_tokens, q_heads, kv_heads, head_dim, dec_bytes, &w);
+    if (budget < 0) return fail(PKV_E_WORKSPACE, "%s: workspace of %zu bytes cannot hold the split of %d tokens", fn, dec_bytes, n_tokens);
+    plan.n_tokens = n_tokens; plan.q_heads = q_heads; plan.kv_heads = kv_heads; plan.head_dim = head_dim;
+    plan.n_items = n_tokens + budget;    // upper bound
+    plan.reserved = 1;
+  } else {
+    st = plan_device(tp, n_tokens, q_heads, kv_heads, head_dim, workspace, dec_bytes, static_cast<cudaStream_t>(stream), &plan, &r);
+    if (st != PKV_OK) return st;
+  }
   plan.num_blocks = num_blocks > 0 ? num_blocks : 0;
   // The long runs through the tensor-core kernel, whose item counts come from the router; then decode tokens
   // and short runs through the decode kernels (tokens of long runs are in no work item).  The prefill kernel
@@ -881,12 +884,13 @@ int mixed_attn(const void* q, const void* kc, const void* vc, const int* bt, con
   // two 300-token chunks and 20 decode tokens took 42 us a layer.
   const int max_runs = n_tokens / min_run;
   if constexpr (!IsF32<T>::value) {
+    const InlineRuns runs{tp, ts, to, min_run};
     st = prefill_launch<T>(q, kc, vc, bt, r.tbl_off, r.q_start, r.q_len, r.ctx_len, out, n_tokens, max_runs, n_tokens,
-                           q_heads, kv_heads, head_dim, block_size, num_blocks, scale, stream, r.dims, true);
+                           q_heads, kv_heads, head_dim, block_size, num_blocks, scale, stream, r.dims, true, inline_plan ? &runs : nullptr);
     if (st != PKV_OK) return st;
   }
   st = decode_planned<T>(&plan, q, kc, vc, bt, to, ts, tp, out, block_size, scale, workspace, dec_bytes, stream, nullptr, nullptr,
-                         true, true);
+                         true, true, inline_plan ? min_run : 0);
   return st;
 }
 

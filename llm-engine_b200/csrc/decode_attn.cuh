@@ -77,6 +77,11 @@ struct DecodeArgs {
   // complete, and writes nothing that it reads or writes (the prefill kernel of a mixed step): wait for it
   // before leaving instead of before loading.
   int wait_last;
+  // > 0: there is no plan in the workspace; the blocks of the attention kernel work it out for themselves
+  // (decode_tma_kernel with INLINE_PLAN, mixed steps of up to kInlineTokens tokens), leaving runs of at least
+  // this many tokens to the prefill kernel, and write tok_split for the merge.
+  int inline_min_run;
+  int inline_max_shares, inline_forced_chunk;
   unsigned long long pool_rows;   // slots the K/V tensor maps cover (the pool size when the caller gave it, else a bound)
 };
 
@@ -235,8 +240,9 @@ __global__ void __launch_bounds__(kCombineThreads) decode_combine_kernel(const D
   // The split record of this block's first (token, kv head) is part of the plan, which was complete
   // before the attention kernel started: fetch it while that kernel is still finishing.
   TokSplit ts_first{0, 0};
-  if (static_cast<int>(blockIdx.x) < pairs) ts_first = a.tok_split[blockIdx.x / a.kv_heads];
+  if (static_cast<int>(blockIdx.x) < pairs && a.inline_min_run == 0) ts_first = a.tok_split[blockIdx.x / a.kv_heads];
   pdl_wait();  // the attention kernel's partials
+  if (static_cast<int>(blockIdx.x) < pairs && a.inline_min_run > 0) ts_first = a.tok_split[blockIdx.x / a.kv_heads];
   for (int pr = blockIdx.x; pr < pairs; pr += gridDim.x) {
     const int token = pr / a.kv_heads, kvh = pr - token * a.kv_heads;
     const TokSplit ts = pr == static_cast<int>(blockIdx.x) ? ts_first : a.tok_split[token];

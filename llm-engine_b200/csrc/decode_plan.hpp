@@ -172,6 +172,19 @@ PKV_HD inline int max_shares_for(int extra, int workers_per_kv_head) {
   return fit < workers_per_kv_head ? (fit > 0 ? fit : 0) : workers_per_kv_head;
 }
 
+// ---- steps planned inside the kernels ------------------------------------------------
+// Mixed steps of up to this many tokens need no planner launch: every block of the prefill kernel finds the
+// long runs for itself, every block of the decode kernel the cuts (14 bytes of shared memory a token, which is
+// what three blocks on an SM leave).
+constexpr int kInlineTokens = 704;
+constexpr int kInlineRuns = 256;
+struct InlineRuns {
+  const int* token_pos;
+  const int* token_seq;
+  const int* table_offset;
+  int min_run;
+};
+
 // Chunk rule of the shared-prefix planner, and of the cluster form's offer.  items_at[j] = sum over tokens of ceil(L_t / (64 << j)).
 //   1. take the smallest chunk >= 256 keys whose item count stays within the
 //      budget (one item per token plus `extra_budget`): the most parallelism the

@@ -91,6 +91,144 @@ __device__ __forceinline__ void cluster_push4(uint32_t dst_cluster_addr, float4 
                : "memory");
 }
 
+// Place in a warp's list of units: (item, kv head), with `end` the end of the items of the current share.
+struct UnitCursor { int u, item, end, kvh; };
+
+// A mixed step's plan in shared memory, built by every block for itself (DecodeArgs::inline_min_run): the same cuts
+// as decode_plan_kernel makes, found through the tokens instead of a list.  A planner launch in front of the
+// attention kernel cost 4.6 us a layer, and the four dependent look-ups from its list to a unit's first load
+// 2 to 3 more; this costs every block about 1.5.
+struct InlinePlan {
+  static constexpr int kPer = (kInlineTokens + 127) / 128;
+  static constexpr int kBytes = kInlineTokens * (3 * 4 + 2);
+  struct Unit { int token, begin, len, part; };
+  int* s_len;              // keys of a token the decode path handles: position + 1, or 0
+  int* s_tbl;              // where its block table starts
+  int* s_key;              // shares: where it begins in the laid-out step, in slabs; chunks: its first item
+  unsigned short* s_part;  // its first partial slot
+  ShareRule rule;
+  int n_items;
+
+  __device__ __forceinline__ int table_of(int token) const { return s_tbl[token]; }
+
+  __device__ __forceinline__ void build(const DecodeArgs& a, unsigned char* smem) {
+    __shared__ int sm_scan[3][4];
+    s_len = reinterpret_cast<int*>(smem);
+    s_tbl = s_len + kInlineTokens;
+    s_key = s_tbl + kInlineTokens;
+    s_part = reinterpret_cast<unsigned short*>(s_key + kInlineTokens);
+    const int n = a.n_tokens;
+    TokenRuns<4, kPer> runs;
+    runs.find(a.token_pos, a.token_seq, n, s_len, s_tbl, s_key, sm_scan[0]);
+    int len[kPer], tbl[kPer], slabs = 0;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      len[i] = tbl[i] = 0;
+      if (i < runs.count && runs.len[i] < a.inline_min_run) {
+        len[i] = max(runs.pos[i], 0) + 1;
+        tbl[i] = __ldg(a.table_offset + runs.seq[i]);
+        slabs += share_padded(len[i]) / kShareSlab;
+      }
+    }
+    int total;
+    int at = block_scan<ScanSum, 4>(slabs, sm_scan[1], &total) - slabs;    // (and the barrier after which the arrays are free)
+    rule = share_rule(static_cast<long long>(total) * kShareSlab, a.inline_max_shares, a.inline_forced_chunk);
+    int begin[kPer], ns[kPer], sum = 0;                                    // items in the upper half, partials in the lower: < 2^16 each
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      begin[i] = at;
+      ns[i] = 0;
+      if (len[i] > 0) {
+        const int padded = share_padded(len[i]);
+        ns[i] = rule.per > 0 ? share_cuts(static_cast<long long>(at) * kShareSlab, padded, rule.per).n + 1
+                             : rule.chunk > 0 ? (len[i] + rule.chunk - 1) / rule.chunk : 1;
+        at += padded / kShareSlab;
+      }
+      sum += (ns[i] << 16) | (ns[i] > 1 ? ns[i] : 0);
+    }
+    int all;
+    int before = block_scan<ScanSum, 4>(sum, sm_scan[2], &all) - sum;
+    n_items = all >> 16;
+    TokSplit* split = const_cast<TokSplit*>(a.tok_split);
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      if (i < runs.count) {
+        const int t = runs.first + i;
+        s_len[t] = len[i];
+        s_tbl[t] = tbl[i];
+        s_key[t] = rule.per > 0 ? begin[i] : before >> 16;
+        s_part[t] = static_cast<unsigned short>(before & 0xffff);
+        if (blockIdx.x == 0) split[t] = TokSplit{before & 0xffff, ns[i]};
+        before += (ns[i] << 16) | (ns[i] > 1 ? ns[i] : 0);
+      }
+    }
+    __syncthreads();
+  }
+
+  // How many tokens have s_key < v (they come first: s_key does not decrease); by the whole warp.
+  __device__ __forceinline__ int below(int v, int n) const {
+    const int lane = threadIdx.x & 31, step = (n + 31) / 32;               // <= 22
+    const int last = (lane + 1) * step - 1;
+    const int seg = __popc(__ballot_sync(0xffffffffu, last < n && s_key[min(last, n - 1)] < v));
+    const int i = seg * step + lane;
+    return seg * step + __popc(__ballot_sync(0xffffffffu, lane < step && i < n && s_key[min(i, n - 1)] < v));
+  }
+
+  // The next unit of the warp's list; x.end: 1 while inside a share, whose next token is x.item.
+  __device__ __forceinline__ bool next(UnitCursor& x, Unit& w, int total, int stride, int kv_heads, int n) const {
+    if (rule.per == 0) {
+      x.u += stride;
+      if (x.u >= total) { x.u = total; return false; }
+      const int item = x.u / kv_heads;
+      x.kvh = x.u - item * kv_heads;
+      const int t = below(item + 1, n) - 1;                                // the last token whose first item is not past this one
+      const int len = s_len[t], s = item - s_key[t];
+      w.token = t;
+      w.begin = s * rule.chunk;
+      w.len = rule.chunk > 0 ? min(rule.chunk, len - w.begin) : len;
+      w.part = w.len < len ? s_part[t] + s : -1;
+      return true;
+    }
+    const int per = rule.per / kShareSlab;                                 // all in slabs from here
+    for (;;) {
+      if (x.end == 0) {
+        x.u += stride;
+        if (x.u >= total) { x.u = total; return false; }
+        const int j = x.u / kv_heads, c = j * per;
+        x.kvh = x.u - j * kv_heads;
+        x.item = below(c - 1, n);                                          // the first token that begins in this share
+        x.end = 1;
+        const int t = x.item - 1;
+        if (t >= 0) {
+          const int b = s_key[t], e = b + share_padded(s_len[t]) / kShareSlab;
+          if (e - c > 1) {                                                 // the token before it is cut here
+            const bool again = e - (c + per) > 1;
+            w.token = t;
+            w.begin = (c - b) * kShareSlab;
+            w.len = again ? rule.per : s_len[t] - w.begin;
+            w.part = s_part[t] + (c - ((b + 1) / per + 1) * per) / per + 1;
+            if (again) x.end = 0;
+            return true;
+          }
+        }
+      }
+      const int j = x.u / kv_heads;
+      int t = x.item;
+      if (t < n && s_len[t] == 0) t = below(s_key[t] + 1, n) - 1;          // tokens of long runs begin where the next token does
+      if (t >= n || s_len[t] == 0 || min((s_key[t] + 1) / per, rule.n_shares - 1) > j) { x.end = 0; continue; }
+      const int b = s_key[t], e = b + share_padded(s_len[t]) / kShareSlab, cut = ((b + 1) / per + 1) * per;
+      const bool cuts = e - cut > 1;
+      w.token = t;
+      w.begin = 0;
+      w.len = cuts ? (cut - b) * kShareSlab : s_len[t];
+      w.part = cuts ? s_part[t] : -1;
+      x.item = t + 1;
+      if (cuts) x.end = 0;
+      return true;
+    }
+  }
+};
+
 // (a.x, a.y) * (b.x, b.y) + (c.x, c.y), each rounded once, in one instruction.
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   float2 d;
@@ -102,7 +240,7 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 }
 
 template <typename T, int D, int NT, int MT, int NSTAGES, int WARPS, int MIN_BLOCKS, int TOK = 1, bool FUSED_APPEND = false,
-          bool CLUSTER = false>
+          bool CLUSTER = false, bool INLINE_PLAN = false>
 __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
     decode_tma_kernel(const DecodeArgs a, const __grid_constant__ CUtensorMap kmap,
                       const __grid_constant__ CUtensorMap vmap) {
@@ -190,12 +328,15 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
   // Units of this warp: one item each (item, kv head) dealt round-robin, or, when the plan has shares, all the
   // items of a (share, kv head) one after the other.  The issue side and the math side walk the same list,
   // each with a cursor of its own.
-  const int n_shares = (CLUSTER || TOK > 1 || a.direct) ? 0 : a.header->n_shares;
-  const int n_items = CLUSTER ? 0 : (TOK > 1 ? a.n_shared : (a.direct ? a.n_tokens : a.header->n_items));
+  static_assert(!INLINE_PLAN || (TOK == 1 && !FUSED_APPEND && !CLUSTER && !F32 && WARPS == 4), "mixed steps only");
+  InlinePlan ip;
+  if constexpr (INLINE_PLAN) ip.build(a, smem_raw + (ring0 - smem_u32(smem_raw)) + WARPS * S::kWarpBytes);
+  const int n_shares = INLINE_PLAN ? ip.rule.n_shares : (CLUSTER || TOK > 1 || a.direct) ? 0 : a.header->n_shares;
+  const int n_items = INLINE_PLAN ? ip.n_items : CLUSTER ? 0 : (TOK > 1 ? a.n_shared : (a.direct ? a.n_tokens : a.header->n_items));
   const int total = CLUSTER ? (c_len > 0 ? 1 : 0) : (n_shares > 0 ? n_shares : n_items) * a.kv_heads;
   const int gw = CLUSTER ? 0 : blockIdx.x * WARPS + warp, GW = CLUSTER ? 1 : gridDim.x * WARPS;
-  const int* share_first = CLUSTER || TOK > 1 || a.direct ? nullptr : reinterpret_cast<const int*>(a.items + n_items);
-  struct Cursor { int u, item, end, kvh; };
+  const int* share_first = CLUSTER || TOK > 1 || INLINE_PLAN || a.direct ? nullptr : reinterpret_cast<const int*>(a.items + n_items);
+  using Cursor = UnitCursor;
   auto next_unit = [&](Cursor& x) -> bool {
     if constexpr (CLUSTER) {             // at most one unit
       x.kvh = c_kvh;
@@ -223,13 +364,19 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
   int i_ent = 0, i_ent_base = -64;   // this lane's block-table entry for box i_ent_base + lane
   uint32_t n_issued = 0, n_consumed = 0;
 
+  InlinePlan::Unit i_unit, m_unit;
   // Issues the next slab of this warp's unit sequence, if there is one.
   auto issue_next = [&]() -> bool {
     while (i_slab >= i_nslabs) {
-      if (!next_unit(ic)) return false;
+      if (!(INLINE_PLAN ? ip.next(ic, i_unit, total, GW, a.kv_heads, a.n_tokens) : next_unit(ic))) return false;
       const int item = ic.item, kvh = ic.kvh;
       int token, part;
-      if constexpr (CLUSTER) {
+      if constexpr (INLINE_PLAN) {
+        token = i_unit.token;
+        i_kvbeg = i_unit.begin;
+        i_len = i_unit.len;
+        part = 0;
+      } else if constexpr (CLUSTER) {
         token = c_token;
         i_kvbeg = c_begin;
         i_len = c_len;
@@ -243,7 +390,8 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
       } else {
         load_item(a, item, token, i_kvbeg, i_len, part);
       }
-      i_tbl = a.block_tables + __ldg(a.table_offset + __ldg(a.token_seq + token));
+      if constexpr (INLINE_PLAN) i_tbl = a.block_tables + ip.table_of(token);
+      else i_tbl = a.block_tables + __ldg(a.table_offset + __ldg(a.token_seq + token));
       i_nslabs = (i_len + SLAB - 1) / SLAB;
       i_slab = 0;
       i_x0 = kvh * D;
@@ -306,11 +454,14 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
   const int mi = lane >> 3, r8 = lane & 7;
   bool more = true;
   Cursor mc{gw - GW, 0, 0, 0};
-  while (next_unit(mc)) {
+  while (INLINE_PLAN ? ip.next(mc, m_unit, total, GW, a.kv_heads, a.n_tokens) : next_unit(mc)) {
     const int item = mc.item, kvh = mc.kvh;
     int token, kv_begin, kv_len, part;
     int toks[TOK], parts[TOK], n_tok = 1;
-    if constexpr (CLUSTER) {
+    if constexpr (INLINE_PLAN) {
+      token = m_unit.token; kv_begin = m_unit.begin; kv_len = m_unit.len; part = m_unit.part;
+      toks[0] = token; parts[0] = part;
+    } else if constexpr (CLUSTER) {
       token = c_token; kv_begin = c_begin; kv_len = c_len;
       part = c_nsplits > 1 ? c_split : -1;
       toks[0] = token; parts[0] = part;
@@ -697,7 +848,9 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
     }
   }
   if constexpr (!CLUSTER && !FUSED_APPEND) {
-    if (a.wait_last) pdl_wait();       // this launch's completion has to imply the previous one's
+    // This launch's completion has to imply the previous one's: one block stays for it.  (All of them waiting
+    // here kept the blocks that had found no room yet from starting before the previous launch's end.)
+    if (a.wait_last && blockIdx.x == 0) pdl_wait();
   }
   if constexpr (CLUSTER) {
     if (c_nsplits > 1) {               // the same for every thread of the cluster

@@ -60,6 +60,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "decode_plan.hpp"
 #include "launch_util.hpp"
 #include "status.hpp"
 #include "tma_util.hpp"
@@ -123,6 +124,10 @@ struct PrefillArgs {
   // kernel on the stream: the mixed-step router decides on the device which runs of tokens are prefill
   // chunks); the two fields above are then upper bounds that sized the grid.
   const int* dims;
+  // runs.token_pos != nullptr: a mixed step of n_tokens packed tokens whose long runs every block finds for itself
+  // (n_seqs and max_q_len are upper bounds again, and the four per-sequence arrays are not read)
+  InlineRuns runs;
+  int n_tokens;
   unsigned int* host_err;   // pinned host word that also receives a give-up (null: none)
 };
 
@@ -312,9 +317,45 @@ __global__ void __launch_bounds__(kThreads, 2)
 
   // In a mixed step (a.dims) the launch behind this one is the decode kernel, which does not wait for this
   // one before it reads the router's plan: it may start only once the plan is complete.
-  if (a.dims == nullptr) pdl_launch_dependents();
+  const bool mixed = a.dims != nullptr || a.runs.token_pos != nullptr;
+  if (!mixed) pdl_launch_dependents();
   pdl_wait();
-  if (a.dims != nullptr) pdl_launch_dependents();
+  if (mixed) pdl_launch_dependents();
+
+  const int* q_start = a.q_start;
+  const int* q_lens = a.q_len;
+  const int* ctx_lens = a.ctx_len;
+  const int* table_offset = a.table_offset;
+  int n_seqs = a.dims ? __ldcg(a.dims) : a.n_seqs;
+  if (!SPLIT && a.runs.token_pos != nullptr) {
+    // the runs of at least min_run tokens, in packed order; the ring serves as scratch
+    __shared__ int sm_scan[2][kThreads / 32];
+    constexpr int kPer = (kInlineTokens + kThreads - 1) / kThreads;
+    int* scratch = reinterpret_cast<int*>(base_ptr + kSmemKV);
+    TokenRuns<kThreads / 32, kPer> runs;
+    runs.find(a.runs.token_pos, a.runs.token_seq, a.n_tokens, scratch, scratch + kInlineTokens, scratch + 2 * kInlineTokens, sm_scan[0]);
+    int mine = 0;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) mine += (i < runs.count && runs.start_of[i] == runs.first + i && runs.len[i] >= a.runs.min_run) ? 1 : 0;
+    int at = block_scan<ScanSum, kThreads / 32>(mine, sm_scan[1], &n_seqs) - mine;
+    int* s_runs = reinterpret_cast<int*>(base_ptr + kSmemTotal - 1024);   // [4][kInlineRuns] behind everything else
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      if (i < runs.count && runs.start_of[i] == runs.first + i && runs.len[i] >= a.runs.min_run) {
+        s_runs[at] = runs.first + i;
+        s_runs[kInlineRuns + at] = runs.len[i];
+        s_runs[2 * kInlineRuns + at] = max(runs.pos[i], 0);
+        s_runs[3 * kInlineRuns + at] = __ldg(a.runs.table_offset + runs.seq[i]);
+        ++at;
+      }
+    }
+    q_start = s_runs;
+    q_lens = s_runs + kInlineRuns;
+    ctx_lens = s_runs + 2 * kInlineRuns;
+    table_offset = s_runs + 3 * kInlineRuns;
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");       // the ring goes to the copies next
+    __syncthreads();
+  }
 
   // Query tiles are handed out longest key range first, so that the launch ends on its shortest items and the
   // blocks finish together (configuration 4: 515 us for four layers sequence by sequence, 486 us this way).
@@ -327,7 +368,6 @@ __global__ void __launch_bounds__(kThreads, 2)
   __shared__ int s_tiles[kMaxRankedSeqs];
   __shared__ int s_cum[kBuckets];
   const int tt = a.tile_tokens;
-  const int n_seqs = a.dims ? __ldcg(a.dims) : a.n_seqs;
   auto reach = [&](int s, int x) {           // tiles of sequence s whose length is x or more
     const int over = s_top[s] - x;
     return over >= 0 ? min(static_cast<int>(__umulhi(over, a.by_tile_tokens)) + 1, s_tiles[s]) : 0;
@@ -336,9 +376,9 @@ __global__ void __launch_bounds__(kThreads, 2)
   int width = 1;                             // keys per bucket
   if (ranked) {
     for (int s = threadIdx.x; s < n_seqs; s += kThreads) {
-      const int nt = (__ldg(a.q_len + s) + tt - 1) / tt;
+      const int nt = (q_lens[s] + tt - 1) / tt;
       s_tiles[s] = nt;
-      s_top[s] = nt > 0 ? __ldg(a.ctx_len + s) + nt * tt : 0;
+      s_top[s] = nt > 0 ? ctx_lens[s] + nt * tt : 0;
     }
     __syncthreads();
     int longest = 0;
@@ -449,13 +489,13 @@ __global__ void __launch_bounds__(kThreads, 2)
           tile_of_rank(rest, seq, tile);
         } else {
           seq = rest / n_slots;
-          tile = (__ldg(a.q_len + seq) + tt - 1) / tt - 1 - (rest - seq * n_slots);
+          tile = (q_lens[seq] + tt - 1) / tt - 1 - (rest - seq * n_slots);
         }
         if (tile < 0) continue;
-        const int q_len = __ldg(a.q_len + seq), ctx = __ldg(a.ctx_len + seq);
+        const int q_len = q_lens[seq], ctx = ctx_lens[seq];
         const int tokens = min(tt, q_len - tile * tt);
         d.head = static_cast<int>(t % a.head_tiles) * a.pack;
-        d.row0 = __ldg(a.q_start + seq) + tile * tt;
+        d.row0 = q_start[seq] + tile * tt;
         d.rows_here = tokens * a.pack;
         d.kv_total = ctx + tile * tt + tokens;
         d.limit0 = ctx + tile * tt;
@@ -488,7 +528,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       dead = __shfl_sync(0xffffffffu, dead ? 1 : 0, 0) != 0;
       if (d.n_kt < 0 || dead) break;
       const int kvh = d.head / a.group;
-      const int* tbl = a.block_tables + __ldg(a.table_offset + seq);
+      const int* tbl = a.block_tables + table_offset[seq];
       for (int j = d.kt0; j < d.kt0 + d.n_kt; ++j, ++g) {
         const int st = g % kKVStages;
         const int rel = j * kKTile + (lane & 3) * 16;
@@ -895,7 +935,7 @@ template <typename T>
 int prefill_launch(const void* q, const void* k_cache, const void* v_cache, const int* block_tables,
                    const int* table_offset, const int* q_start, const int* q_len, const int* ctx_len, void* out,
                    int n_tokens, int n_seqs, int max_q_len, int q_heads, int kv_heads, int head_dim, int block_size,
-                   int num_blocks, float scale, pkv_stream stream, const int* d_dims, bool may_allocate) {
+                   int num_blocks, float scale, pkv_stream stream, const int* d_dims, bool may_allocate, const InlineRuns* runs) {
   const char* fn = "pkv_prefill_attn";
   if (n_seqs <= 0 || n_tokens <= 0 || max_q_len <= 0) return PKV_OK;
   if (!q || !k_cache || !v_cache || !block_tables || !table_offset || !q_start || !q_len || !ctx_len || !out)
@@ -926,6 +966,7 @@ int prefill_launch(const void* q, const void* k_cache, const void* v_cache, cons
   if (st != PKV_OK) return st;
   // Heads per tile: the largest divisor of the group, up to 16, that leaves at most 8 of the 128 rows unused
   // (a group of 13 would waste 11: its heads take tiles of their own).
+  constexpr int kInlineSmem = kSmemTotal + 4 * kInlineRuns * static_cast<int>(sizeof(int));   // still two blocks per SM
   const int group = q_heads / kv_heads;
   int pack = 1;
   for (int p = 2; p <= 16; ++p)
@@ -949,7 +990,7 @@ int prefill_launch(const void* q, const void* k_cache, const void* v_cache, cons
   split.dynamicSmemBytes = kSmemTotal;
   split.attrs = split_attr;
   if (configured_device != dev) {
-    cudaError_t e = cudaFuncSetAttribute(prefill_tc_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTotal);
+    cudaError_t e = cudaFuncSetAttribute(prefill_tc_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kInlineSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_tc_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTotal);
     if (e != cudaSuccess) return fail(PKV_E_CUDA, "%s: cannot reserve %d bytes of shared memory: %s", fn, kSmemTotal, cudaGetErrorString(e));
     split.numAttrs = 1;
@@ -976,11 +1017,10 @@ int prefill_launch(const void* q, const void* k_cache, const void* v_cache, cons
   if (slots > 0x7fffffffll) return fail(PKV_E_UNSUPPORTED, "%s: %lld work items; at most 2^31 - 1 per call", fn, slots);
   // every sequence has at most one tile that is not full
   const long long n_items = std::min<long long>(slots, (n_tokens / tile_tokens + static_cast<long long>(n_seqs)) * a.head_tiles);
-  a.dims = d_dims;
+  a.dims = runs ? nullptr : d_dims;
+  a.runs = runs ? *runs : InlineRuns{nullptr, nullptr, nullptr, 0};
+  a.n_tokens = n_tokens;
   a.host_err = error_mirror(may_allocate);
-  const TicketPair tp = ticket_pair_for(static_cast<cudaStream_t>(stream), dev);
-  a.ticket = tp.ticket;
-  a.done = tp.done;
   // Persistent blocks: two per SM, or one per item if there are fewer.
   static thread_local int sms = 0;
   if (!sms) {
@@ -990,6 +1030,10 @@ int prefill_launch(const void* q, const void* k_cache, const void* v_cache, cons
   // PKV_PREFILL_BLOCKS_PER_SM = 1: half the persistent grid (a measurement aid: what one block per SM does alone)
   static const int per_sm = [] { const char* e = std::getenv("PKV_PREFILL_BLOCKS_PER_SM"); return (e && e[0] == '1') ? 1 : 2; }();
   const int blocks = static_cast<int>(std::min<long long>(n_items, static_cast<long long>(per_sm) * sms));
+  // A block that gets one item at most needs no ticket for it (nor the look-up of the stream's counter).
+  const TicketPair tp = n_items > blocks ? ticket_pair_for(static_cast<cudaStream_t>(stream), dev) : TicketPair{nullptr, nullptr};
+  a.ticket = tp.ticket;
+  a.done = tp.done;
   // Few items: the largest cluster per item that leaves all of them resident (up to 15 items eight blocks, 33
   // four, 73 two).  Measured per layer with its rope + append: 50 tokens behind 4,000 (6 items) 53.2 -> 16.7 us,
   // 128 behind 2,000 (32 items) 33.6 -> 20.5; short fresh chunks, which no block shares, lose 1 to 2 us of 9
@@ -1005,17 +1049,17 @@ int prefill_launch(const void* q, const void* k_cache, const void* v_cache, cons
     split.numAttrs = pdl_enabled() ? 2 : 1;
     cudaLaunchKernelEx(&split, prefill_tc_kernel<T, true>, a, qmap, kmap, vmap);
   } else {
-    launch_pdl(prefill_tc_kernel<T, false>, dim3(blocks), dim3(kThreads), kSmemTotal, static_cast<cudaStream_t>(stream), a, qmap, kmap, vmap);
+    launch_pdl(prefill_tc_kernel<T, false>, dim3(blocks), dim3(kThreads), runs ? kInlineSmem : kSmemTotal, static_cast<cudaStream_t>(stream), a, qmap, kmap, vmap);
   }
   return check_launch("prefill_tc_kernel");
 }
 
 template int prefill_launch<__nv_bfloat16>(const void*, const void*, const void*, const int*, const int*, const int*,
                                            const int*, const int*, void*, int, int, int, int, int, int, int, int, float,
-                                           pkv_stream, const int*, bool);
+                                           pkv_stream, const int*, bool, const InlineRuns*);
 template int prefill_launch<__half>(const void*, const void*, const void*, const int*, const int*, const int*, const int*,
                                     const int*, void*, int, int, int, int, int, int, int, int, float, pkv_stream,
-                                    const int*, bool);
+                                    const int*, bool, const InlineRuns*);
 
 namespace {
 
@@ -1030,7 +1074,7 @@ int prefill_impl(const void* q, const void* k_cache, const void* v_cache, const 
   if (num_blocks <= 0) return fail(PKV_E_ARG, "pkv_prefill_attn: num_blocks %d must be > 0", num_blocks);
   return prefill_launch<T>(q, k_cache, v_cache, block_tables, table_offset, q_start, q_len, ctx_len, out, n_tokens,
                            n_seqs, max_q_len, q_heads, kv_heads, head_dim, block_size, num_blocks, scale, stream,
-                           nullptr, true);
+                           nullptr, true, nullptr);
 }
 
 }  // namespace
