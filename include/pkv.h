@@ -209,11 +209,13 @@ typedef struct pkv_decode_plan {
                      at most 8 query heads per kv head, every cluster resident at once, at most 256 keys per
                      warp -- unless the environment has PKV_DECODE_CLUSTER=0 (read at every call); the other
                      planners leave 0.  A caller may clear it; a launch the kernel or the device cannot take
-                     (fp32 K/V, block_size < 16, clusters that would not all be resident) runs the ordinary form.
+                     (block_size < 16, clusters that would not all be resident) runs the ordinary form.
                      A captured launch of this form stays correct when replayed over later steps of the same
                      token count: it reads no plan, only token_pos.
                      No counterpart in llm-engine. */
-  int pad[2];
+  int cluster_wide; /* the same at head_dim 128 (at most 128 keys per warp, two blocks per SM resident); `cluster` is
+                       0 there */
+  int pad;
 } pkv_decode_plan;
 
 size_t pkv_decode_plan_staging_bytes(int n_tokens, int kv_heads);

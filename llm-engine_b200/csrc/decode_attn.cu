@@ -380,17 +380,19 @@ std::atomic<unsigned long long> g_cluster_launches{0};   // pkv_debug_cluster_la
 // per (token, kv head), merge inside the launch.  *launched stays false, with nothing enqueued, when
 // this device cannot hold all the clusters at once (they would queue behind one another): the
 // caller then takes the ordinary path.
-template <typename T, bool FUSED>
+template <typename T, int D, bool FUSED>
 int launch_tma_cluster_impl(const DecodeArgs& a, int cs, cudaStream_t stream, bool* launched) {
   constexpr int WARPS = 4;
-  // (fp32: slabs of 16 keys are as many bytes as 32 16-bit ones; its query rows and the landing area leave room for two blocks per SM)
-  constexpr int MT = IsF32<T>::value ? 1 : 2;
-  using S = TmaSmem<64, MT, 2, WARPS, sizeof(T)>;
-  auto kern = decode_tma_kernel<T, 64, 1, MT, 2, WARPS, IsF32<T>::value ? 2 : 3, 1, FUSED, true>;
+  // Slabs of 8 KB (16 KB for fp32 at 128 dims), two per warp in flight.  With the landing area, and fp32's query
+  // rows, three blocks fit an SM at 64 dims of 16 bits, two at 128 or of fp32, one at 128 of fp32.
+  constexpr int MT = IsF32<T>::value || D == 128 ? 1 : 2;
+  constexpr int kResident = 3 - (IsF32<T>::value ? 1 : 0) - (D == 128 ? 1 : 0);
+  using S = TmaSmem<D, MT, 2, WARPS, sizeof(T)>;
+  auto kern = decode_tma_kernel<T, D, 1, MT, 2, WARPS, kResident, 1, FUSED, true>;
   *launched = false;
   const long long pairs = static_cast<long long>(a.n_tokens) * a.kv_heads;
   if (!cluster_size_ok(cs) || pairs * cs > 0x7fffffffll) return PKV_OK;
-  constexpr int kSmem = S::kBytes + kClusterLandBytes;
+  constexpr int kSmem = S::kBytes + cluster_land_bytes(D);
   static thread_local int configured_device = -1;
   static thread_local int max_clusters[9];
   int dev = 0;
@@ -435,21 +437,23 @@ int launch_tma_cluster_impl(const DecodeArgs& a, int cs, cudaStream_t stream, bo
   return check_launch("decode_tma_kernel (clusters)");
 }
 
+template <typename T, int D>
+int launch_tma_cluster_dim(const DecodeArgs& a, int cs, cudaStream_t stream, bool* launched) {
+  // the planner does not know the element type: fp32 takes the largest size its fewer resident blocks hold
+  for (; cs >= 2; --cs) {
+    if (!cluster_size_ok(cs)) continue;
+    int st;
+    if constexpr (IsF32<T>::value) st = launch_tma_cluster_impl<T, D, false>(a, cs, stream, launched);
+    else st = a.new_k != nullptr ? launch_tma_cluster_impl<T, D, true>(a, cs, stream, launched) : launch_tma_cluster_impl<T, D, false>(a, cs, stream, launched);
+    if (st != PKV_OK || *launched || !IsF32<T>::value) return st;
+  }
+  return PKV_OK;
+}
+
 template <typename T>
 int launch_tma_cluster(const DecodeArgs& a, int cs, cudaStream_t stream, bool* launched) {
   *launched = false;
-  if constexpr (!IsF32<T>::value) {
-    if (a.new_k != nullptr) return launch_tma_cluster_impl<T, true>(a, cs, stream, launched);
-  }
-  if constexpr (IsF32<T>::value) {
-    // the planner counts on three resident blocks per SM: take the largest size that two hold
-    for (; cs >= 2; --cs) {
-      const int st = cluster_size_ok(cs) ? launch_tma_cluster_impl<T, false>(a, cs, stream, launched) : PKV_OK;
-      if (st != PKV_OK || *launched) return st;
-    }
-    return PKV_OK;
-  }
-  return launch_tma_cluster_impl<T, false>(a, cs, stream, launched);
+  return a.head_dim == 128 ? launch_tma_cluster_dim<T, 128>(a, cs, stream, launched) : launch_tma_cluster_dim<T, 64>(a, cs, stream, launched);
 }
 
 template <typename T, int DJ>
@@ -752,9 +756,10 @@ int decode_planned(const pkv_decode_plan* plan, const void* q, const void* kc, c
     a.shared_items = reinterpret_cast<const int4*>(a.items + plan->n_items);
     a.n_shared = n_shared;
   }
-  if (plan->cluster >= 2 && !peers && n_shared == 0 && a.head_dim == 64 && a.group <= 8 && tma_path<T>(a)) {
+  const int cluster = a.head_dim == 128 ? plan->cluster_wide : plan->cluster;
+  if (cluster >= 2 && !peers && n_shared == 0 && a.group <= 8 && tma_path<T>(a)) {
     bool launched = false;
-    st = launch_tma_cluster<T>(a, plan->cluster, static_cast<cudaStream_t>(stream), &launched);
+    st = launch_tma_cluster<T>(a, cluster, static_cast<cudaStream_t>(stream), &launched);
     if (st != PKV_OK || launched) return st;
   }
   // Work units, or their upper bound when the plan was made on the device.  The TMA kernel turns them into
@@ -766,6 +771,29 @@ int decode_planned(const pkv_decode_plan* plan, const void* q, const void* kc, c
   if (!plan->exact && !tma_path<T>(a) && blocks > persistent_grid()) blocks = persistent_grid();
   if (blocks > 0x7fffffffll) blocks = 0x7fffffffll;
   return launch_decode<T>(a, static_cast<int>(blocks), static_cast<cudaStream_t>(stream), (plan->reserved & 1) != 0);
+}
+
+// Whether the attention kernel can plan a step of n_tokens for itself.
+template <typename T>
+bool inline_plan_ok(int n_tokens, int q_heads, int kv_heads, int head_dim, int block_size, float scale) {
+  if (IsF32<T>::value || head_dim != 64 || n_tokens > kInlineTokens || tuning().variant >= 4) return false;
+  DecodeArgs probe;
+  fill_args(probe, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, n_tokens, q_heads, kv_heads, head_dim, block_size, scale);
+  return tma_path<T>(probe);
+}
+// The plan record of such a step: upper bounds only.
+int inline_plan(const char* fn, int n_tokens, int q_heads, int kv_heads, int head_dim, void* workspace, size_t workspace_bytes,
+                pkv_decode_plan* plan) {
+  if (reinterpret_cast<uintptr_t>(workspace) & 255) return fail(PKV_E_ARG, "%s: workspace must be 256-byte aligned", fn);
+  WsLayout w;
+  const int budget = plan_budget(n_tokens, q_heads, kv_heads, head_dim, workspace_bytes, &w);
+  if (budget < 0)
+    return fail(PKV_E_WORKSPACE, "%s: workspace of %zu bytes cannot hold the split of %d tokens", fn, workspace_bytes, n_tokens);
+  std::memset(plan, 0, sizeof(*plan));
+  plan->n_tokens = n_tokens; plan->q_heads = q_heads; plan->kv_heads = kv_heads; plan->head_dim = head_dim;
+  plan->n_items = n_tokens + budget;
+  plan->reserved = 1;
+  return PKV_OK;
 }
 
 template <typename T>
@@ -790,6 +818,13 @@ int decode_all_in_one(const void* q, const void* kc, const void* vc, const int* 
     return launch_decode<T>(a, static_cast<int>(blocks), static_cast<cudaStream_t>(stream), false);
   }
   pkv_decode_plan plan;
+  if (inline_plan_ok<T>(n_tokens, q_heads, kv_heads, head_dim, block_size, scale)) {
+    // no run is long enough for anything but the decode kernel
+    st = inline_plan(fn, n_tokens, q_heads, kv_heads, head_dim, workspace, workspace_bytes, &plan);
+    if (st != PKV_OK) return st;
+    return decode_planned<T>(&plan, q, kc, vc, bt, to, ts, tp, out, block_size, scale, workspace, workspace_bytes, stream,
+                             nullptr, nullptr, may_allocate, false, 0x7fffffff);
+  }
   st = plan_device(tp, n_tokens, q_heads, kv_heads, head_dim, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), &plan);
   if (st != PKV_OK) return st;
   return decode_planned<T>(&plan, q, kc, vc, bt, to, ts, tp, out, block_size, scale, workspace, workspace_bytes, stream,
@@ -840,12 +875,7 @@ int mixed_attn(const void* q, const void* kc, const void* vc, const int* bt, con
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return fail(PKV_E_ARG, "%s: workspace must be 256-byte aligned", fn);
   // Short enough for every block of both kernels to find the runs and the plan for itself: two launches and the
   // merge.  (Longer steps, and geometries whose decode tokens do not run on the TMA kernel, get the planner.)
-  bool inline_plan = false;
-  {
-    DecodeArgs probe;
-    fill_args(probe, q, kc, vc, bt, to, ts, tp, out, n_tokens, q_heads, kv_heads, head_dim, block_size, scale);
-    inline_plan = n_tokens <= kInlineTokens && n_tokens / min_run <= kInlineRuns && tma_path<T>(probe) && tuning().variant < 4;
-  }
+  const bool inlined = n_tokens / min_run <= kInlineRuns && inline_plan_ok<T>(n_tokens, q_heads, kv_heads, head_dim, block_size, scale);
   const RouteLayout rl = route_layout(n_tokens);
   if (workspace_bytes < rl.total + ws_layout(n_tokens, q_heads, kv_heads, head_dim, 0).total)
     return fail(PKV_E_WORKSPACE, "%s: workspace of %zu bytes is too small for a step of %d tokens (pkv_mixed_attn_workspace_bytes)",
@@ -865,13 +895,9 @@ int mixed_attn(const void* q, const void* kc, const void* vc, const int* bt, con
   r.dims = reinterpret_cast<int*>(rbase + rl.off_dims);
   pkv_decode_plan plan;
   std::memset(&plan, 0, sizeof(plan));
-  if (inline_plan) {
-    WsLayout w;
-    const int budget = plan_budget(n_tokens, q_heads, kv_heads, head_dim, dec_bytes, &w);
-    if (budget < 0) return fail(PKV_E_WORKSPACE, "%s: workspace of %zu bytes cannot hold the split of %d tokens", fn, dec_bytes, n_tokens);
-    plan.n_tokens = n_tokens; plan.q_heads = q_heads; plan.kv_heads = kv_heads; plan.head_dim = head_dim;
-    plan.n_items = n_tokens + budget;    // upper bound
-    plan.reserved = 1;
+  if (inlined) {
+    st = inline_plan(fn, n_tokens, q_heads, kv_heads, head_dim, workspace, dec_bytes, &plan);
+    if (st != PKV_OK) return st;
   } else {
     st = plan_device(tp, n_tokens, q_heads, kv_heads, head_dim, workspace, dec_bytes, static_cast<cudaStream_t>(stream), &plan, &r);
     if (st != PKV_OK) return st;
@@ -886,11 +912,11 @@ int mixed_attn(const void* q, const void* kc, const void* vc, const int* bt, con
   if constexpr (!IsF32<T>::value) {
     const InlineRuns runs{tp, ts, to, min_run};
     st = prefill_launch<T>(q, kc, vc, bt, r.tbl_off, r.q_start, r.q_len, r.ctx_len, out, n_tokens, max_runs, n_tokens,
-                           q_heads, kv_heads, head_dim, block_size, num_blocks, scale, stream, r.dims, true, inline_plan ? &runs : nullptr);
+                           q_heads, kv_heads, head_dim, block_size, num_blocks, scale, stream, r.dims, true, inlined ? &runs : nullptr);
     if (st != PKV_OK) return st;
   }
   st = decode_planned<T>(&plan, q, kc, vc, bt, to, ts, tp, out, block_size, scale, workspace, dec_bytes, stream, nullptr, nullptr,
-                         true, true, inline_plan ? min_run : 0);
+                         true, true, inlined ? min_run : 0);
   return st;
 }
 
@@ -1035,14 +1061,15 @@ static int plan_host_image(const char* fn, const int* h_token_pos, int n_tokens,
   // once, and no warp of a cluster would get more than a few slabs, the attention call runs as clusters
   // and merges inside the launch (the image above stays valid: the call falls back to it if the device
   // turns the cluster launch down).
-  if (cluster_form_enabled() && np > 0 && head_dim == 64 && q_heads / kv_heads <= 8) {
+  if (cluster_form_enabled() && np > 0 && (head_dim == 64 || head_dim == 128) && q_heads / kv_heads <= 8) {
     const long long pairs = static_cast<long long>(n_tokens) * kv_heads;
-    const long long resident = static_cast<long long>(persistent_sms()) * 3;
+    const long long resident = static_cast<long long>(persistent_sms()) * (head_dim == 64 ? 3 : 2);
+    const int max_keys = tuning().cluster_max_keys * 64 / head_dim;    // as many bytes per warp
     if (pairs * 2 <= resident) {
       int cs = static_cast<int>(std::min<long long>(8, resident / pairs));
       if (tuning().cluster_size >= 2 && tuning().cluster_size < cs) cs = tuning().cluster_size;
       while (cs > 2 && !cluster_size_ok(cs)) --cs;       // 8, 4, 3 or 2 blocks: what the landing areas are sized for
-      if ((max_len + 4 * cs - 1) / (4 * cs) <= tuning().cluster_max_keys) plan->cluster = cs;
+      if ((max_len + 4 * cs - 1) / (4 * cs) <= max_keys) (head_dim == 64 ? plan->cluster : plan->cluster_wide) = cs;
     }
   }
   return PKV_OK;

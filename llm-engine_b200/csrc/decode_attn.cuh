@@ -78,8 +78,8 @@ struct DecodeArgs {
   // before leaving instead of before loading.
   int wait_last;
   // > 0: there is no plan in the workspace; the blocks of the attention kernel work it out for themselves
-  // (decode_tma_kernel with INLINE_PLAN, mixed steps of up to kInlineTokens tokens), leaving runs of at least
-  // this many tokens to the prefill kernel, and write tok_split for the merge.
+  // (decode_tma_kernel with INLINE_PLAN, steps of up to kInlineTokens tokens), leaving runs of at least this many
+  // tokens to the prefill kernel, and write tok_split for the merge.
   int inline_min_run;
   int inline_max_shares, inline_forced_chunk;
   unsigned long long pool_rows;   // slots the K/V tensor maps cover (the pool size when the caller gave it, else a bound)

@@ -173,9 +173,9 @@ PKV_HD inline int max_shares_for(int extra, int workers_per_kv_head) {
 }
 
 // ---- steps planned inside the kernels ------------------------------------------------
-// Mixed steps of up to this many tokens need no planner launch: every block of the prefill kernel finds the
-// long runs for itself, every block of the decode kernel the cuts (14 bytes of shared memory a token, which is
-// what three blocks on an SM leave).
+// Steps of up to this many tokens whose caller brings no plan need no planner launch: every block of the decode
+// kernel finds the cuts for itself (14 bytes of shared memory a token, which is what three blocks on an SM
+// leave), and in mixed steps every block of the prefill kernel the long runs.
 constexpr int kInlineTokens = 704;
 constexpr int kInlineRuns = 256;
 struct InlineRuns {

@@ -73,10 +73,10 @@ template <int D, int MT, int NSTAGES, int WARPS, int ELEM = 2> struct TmaSmem {
 // expect, folds them from its own shared memory into the output rows.  No plan, no workspace, no
 // merge kernel, no cluster-wide barrier after the first (which only publishes the mbarriers): the
 // ranges and the byte counts follow from token_pos alone.
-constexpr int kClusterRecord = 68 * 4;   // one (head, range) record in a landing area: 64 sums, maximum, sum, 8 bytes unused
+__host__ __device__ constexpr int cluster_record(int d) { return (d + 4) * 4; }   // one (head, range) record in a landing area: d sums, maximum, sum, 8 bytes unused
 // Landing area of a block: records for ceil(8 / blocks) heads x (4 warps x blocks) ranges; the
 // cluster sizes the launcher offers (2, 3, 4, 8) need at most 3 x 12 of them.
-constexpr int kClusterLandBytes = 36 * kClusterRecord + 96;
+__host__ __device__ constexpr int cluster_land_bytes(int d) { return 36 * cluster_record(d) + 96; }
 __host__ __device__ constexpr bool cluster_size_ok(int cs) { return cs == 2 || cs == 3 || cs == 4 || cs == 8; }
 
 __device__ __forceinline__ uint32_t cluster_map(uint32_t smem_addr, uint32_t rank) {
@@ -94,7 +94,7 @@ __device__ __forceinline__ void cluster_push4(uint32_t dst_cluster_addr, float4 
 // Place in a warp's list of units: (item, kv head), with `end` the end of the items of the current share.
 struct UnitCursor { int u, item, end, kvh; };
 
-// A mixed step's plan in shared memory, built by every block for itself (DecodeArgs::inline_min_run): the same cuts
+// A step's plan in shared memory, built by every block for itself (DecodeArgs::inline_min_run): the same cuts
 // as decode_plan_kernel makes, found through the tokens instead of a list.  A planner launch in front of the
 // attention kernel cost 4.6 us a layer, and the four dependent look-ups from its list to a unit's first load
 // 2 to 3 more; this costs every block about 1.5.
@@ -250,7 +250,8 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
   static_assert(TOK == 1 || TOK == 4, "a shared unit holds four tokens");
   static_assert(NT % TOK == 0, "whole head tiles per token");
   static_assert(!CLUSTER || TOK == 1, "cluster launches take ordinary tokens");
-  static_assert(!CLUSTER || (NT == 1 && D == 64), "the cluster form is written for up to 8 heads of 64 dims per kv head");
+  static_assert(!CLUSTER || NT == 1, "the cluster form is written for up to 8 heads per kv head");
+  constexpr int kClusterRecord = cluster_record(D);
   static_assert(!CLUSTER || (8 * NT * D + 32 * NT) * 4 <= S::kWarpBytes, "a warp's partial must fit its ring");
   constexpr int NTG = NT / TOK;   // head tiles (8 heads each) per token
   constexpr int KS = D / 16;
@@ -330,7 +331,13 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
   // each with a cursor of its own.
   static_assert(!INLINE_PLAN || (TOK == 1 && !FUSED_APPEND && !CLUSTER && !F32 && WARPS == 4), "mixed steps only");
   InlinePlan ip;
-  if constexpr (INLINE_PLAN) ip.build(a, smem_raw + (ring0 - smem_u32(smem_raw)) + WARPS * S::kWarpBytes);
+  if constexpr (INLINE_PLAN) {
+    if (!waited) {       // not behind a prefill launch that has waited for the index arrays' producers
+      pdl_wait();
+      waited = true;
+    }
+    ip.build(a, smem_raw + (ring0 - smem_u32(smem_raw)) + WARPS * S::kWarpBytes);
+  }
   const int n_shares = INLINE_PLAN ? ip.rule.n_shares : (CLUSTER || TOK > 1 || a.direct) ? 0 : a.header->n_shares;
   const int n_items = INLINE_PLAN ? ip.n_items : CLUSTER ? 0 : (TOK > 1 ? a.n_shared : (a.direct ? a.n_tokens : a.header->n_items));
   const int total = CLUSTER ? (c_len > 0 ? 1 : 0) : (n_shares > 0 ? n_shares : n_items) * a.kv_heads;
@@ -859,16 +866,16 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
       const uint32_t land0 = ring0 + WARPS * (S::kWarpBytes + S::kQBytes);    // landing area: behind the rings
       const int ranges_max = WARPS * static_cast<int>(c_size);
       if (c_len > 0) {
-        // send this warp's partial, head by head, to the heads' owners: 16 quads of sums and one with
+        // send this warp's partial, head by head, to the heads' owners: D / 4 quads of sums and one with
         // (maximum, sum) per head, read back from where the unit's finish left them
         __syncwarp();
         const float* pacc = reinterpret_cast<const float*>(ring_ptr);
         const float* pml = pacc + 8 * NT * D;
-        for (int i = lane; i < a.group * 17; i += 32) {
-          const int h = i / 17, k = i - h * 17;
+        for (int i = lane; i < a.group * (D / 4 + 1); i += 32) {
+          const int h = i / (D / 4 + 1), k = i - h * (D / 4 + 1);
           const uint32_t owner = static_cast<uint32_t>(h) % c_size, j = static_cast<uint32_t>(h) / c_size;
           float4 v;
-          if (k < 16) {
+          if (k < D / 4) {
             v = *reinterpret_cast<const float4*>(pacc + h * D + 4 * k);
           } else {
             const float2 ml = *reinterpret_cast<const float2*>(pml + 2 * h);
@@ -890,12 +897,12 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
         const unsigned char* rec0 = land_ptr + static_cast<size_t>(j) * ranges_max * kClusterRecord;
         float m_run = -INFINITY;
 #pragma unroll 4
-        for (int sp = 0; sp < c_nsplits; ++sp) m_run = fmaxf(m_run, *reinterpret_cast<const float*>(rec0 + sp * kClusterRecord + 256));
+        for (int sp = 0; sp < c_nsplits; ++sp) m_run = fmaxf(m_run, *reinterpret_cast<const float*>(rec0 + sp * kClusterRecord + 4 * D));
         float l_run = 0.f, acc0 = 0.f, acc1 = 0.f;
 #pragma unroll 4
         for (int sp = 0; sp < c_nsplits; ++sp) {
           const unsigned char* rec = rec0 + sp * kClusterRecord;
-          const float2 ml = *reinterpret_cast<const float2*>(rec + 256);
+          const float2 ml = *reinterpret_cast<const float2*>(rec + 4 * D);
           const float f = (ml.x == -INFINITY) ? 0.f : softmax_exp<!F32>(ml.x - m_run);
           const float2 v = *reinterpret_cast<const float2*>(rec + 4 * d);
           l_run += f * ml.y;

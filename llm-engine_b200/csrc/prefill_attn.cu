@@ -94,6 +94,7 @@ constexpr int kSmemOnes = kSmemKV + kKVStages * 2 * kKBytes; // a V-shaped tile 
 constexpr int kSmemTotal = kSmemOnes + kKBytes + 1024;       // 105 KB: two blocks per SM
 constexpr int kLandRecord = (kHd + 4) * 4;                   // split launches: one row's partial, 64 sums, maximum, sum, 8 bytes unused
 static_assert(kQTile * kLandRecord <= kKVStages * 2 * kKBytes, "s sources x 128 / s rows, whatever s, fit the ring");
+constexpr int kSplitSmem = 118 * 1024;  // more than half an SM's: the blocks of a cluster take an SM each (2 x 300 tokens behind 1,200: 21.5 -> 19.5 us a layer)
 constexpr int kMinSplitTiles = 4;     // key tiles a block has at least when its item is shared: a tile is 0.7 us, the sharing 2 to 3
 constexpr int kThreads = 192, kProducerWarp = 4, kMmaWarp = 5;   // warps 0-3: softmax, one thread per row of the tile
 constexpr uint32_t kTmemCols = 256;                          // two blocks per SM share the 512 columns
@@ -987,12 +988,12 @@ int prefill_launch(const void* q, const void* k_cache, const void* v_cache, cons
   split_attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   split_attr[1].val.programmaticStreamSerializationAllowed = 1;
   split.blockDim = dim3(kThreads);
-  split.dynamicSmemBytes = kSmemTotal;
+  split.dynamicSmemBytes = kSplitSmem;
   split.attrs = split_attr;
   if (configured_device != dev) {
     cudaError_t e = cudaFuncSetAttribute(prefill_tc_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kInlineSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_tc_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTotal);
-    if (e != cudaSuccess) return fail(PKV_E_CUDA, "%s: cannot reserve %d bytes of shared memory: %s", fn, kSmemTotal, cudaGetErrorString(e));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_tc_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem);
+    if (e != cudaSuccess) return fail(PKV_E_CUDA, "%s: cannot reserve %d bytes of shared memory: %s", fn, kSplitSmem, cudaGetErrorString(e));
     split.numAttrs = 1;
     for (int i = 0; i < 3; ++i) {
       split_attr[0].val.clusterDim.x = 2u << i;
