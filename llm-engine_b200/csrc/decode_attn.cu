@@ -234,7 +234,12 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
     __syncthreads();
     for (int w = 0; w < kPlanThreads / 32; ++w) total += sm_tot[w];
   }
-  const ShareRule rule = share_rule(total, max_shares, forced_chunk);
+  bool any_long = small && my_len > kMinShareKeys;
+  if (!small)
+    for (int t = tid; t < n_tokens; t += kPlanThreads) any_long |= length_of(t) > kMinShareKeys;
+  bool may_halve = __syncthreads_or(any_long) != 0;
+  if constexpr (ROUTE) may_halve = may_halve && sm_misc[0] == 0;
+  const ShareRule rule = share_rule(total, max_shares, forced_chunk, may_halve);
 
   int n_items = 0, n_parts = 0;
   long long carry_begin = 0;
@@ -975,7 +980,7 @@ static int plan_host_image(const char* fn, const int* h_token_pos, int n_tokens,
     max_len = std::max(max_len, h_token_pos[t] + 1);
   }
   const int max_shares = max_shares_for(budget, decode_workers(q_heads, kv_heads, head_dim) / kv_heads);
-  const ShareRule rule = share_rule(total, max_shares, tuning().forced_chunk);
+  const ShareRule rule = share_rule(total, max_shares, tuning().forced_chunk, false);
   const int chunk = rule.chunk;
   long long n_items = n_tokens;
   if (rule.per > 0) {

@@ -127,6 +127,14 @@ constexpr int kShareSlab = 32;
 // Below this many keys a share the tokens are cut one by one into chunks of this length instead:
 // equal shares would cut short tokens that need no merge at all when left whole.
 constexpr int kMinShareKeys = 128;
+// ... and of half that when there are so few keys a share that the longest units decide: four dependent slabs a
+// warp become two.  Only in steps planned on the device that have something to merge anyway (a token of more
+// than kMinShareKeys keys) and no prefill chunk, whose kernel the decode units hide behind (a mixed step of two
+// chunks and 20 decode tokens lost 3 %); small host-planned steps take the cluster form.
+// Engine decode steps, us a layer with 128- and 64-key chunks: 1 sequence of 333 keys 10.8, 9.4; 6 of 100-900 (4 kv
+// heads) 12.0, 10.7; 40 of 50-1,000 14.4, 12.9 (15 keys a share); 100 of 60-300 16.8, 16.3 (33); 48 of 32-1,500
+// 16.8, 17.5 (41); 100 of 60-2,000 17.7, 19.9 (63).
+constexpr int kFineShareKeys = 36;
 
 PKV_HD inline int share_padded(int len) { return (len + kShareSlab - 1) & ~(kShareSlab - 1); }
 
@@ -153,12 +161,16 @@ struct ShareRule {
   int n_shares;
   int chunk;      // per == 0: keys per chunk, 0 = tokens are not cut
 };
-// total: padded keys of the step; max_shares: warps per kv head (0: the workspace has no room for splits).
-PKV_HD inline ShareRule share_rule(long long total, int max_shares, int forced_chunk) {
+// total: padded keys of the step; max_shares: warps per kv head (0: the workspace has no room for splits); may_halve:
+// see kFineShareKeys.
+PKV_HD inline ShareRule share_rule(long long total, int max_shares, int forced_chunk, bool may_halve) {
   ShareRule r{0, 0, 0};
   if (max_shares <= 0) return r;
   if (forced_chunk > 0 && total / forced_chunk <= max_shares) { r.chunk = forced_chunk; return r; }
-  if (total < static_cast<long long>(max_shares) * kMinShareKeys) { r.chunk = kMinShareKeys; return r; }
+  if (total < static_cast<long long>(max_shares) * kMinShareKeys) {
+    r.chunk = may_halve && total < static_cast<long long>(max_shares) * kFineShareKeys ? kMinShareKeys / 2 : kMinShareKeys;
+    return r;
+  }
   const long long per = ((total + max_shares - 1) / max_shares + kShareSlab - 1) / kShareSlab * kShareSlab;
   if (per > 0x40000000) return r;
   r.per = static_cast<int>(per);

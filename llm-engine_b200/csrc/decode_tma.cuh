@@ -121,18 +121,22 @@ struct InlinePlan {
     TokenRuns<4, kPer> runs;
     runs.find(a.token_pos, a.token_seq, n, s_len, s_tbl, s_key, sm_scan[0]);
     int len[kPer], tbl[kPer], slabs = 0;
+    bool any_long = false, in_run = false;
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
       len[i] = tbl[i] = 0;
+      in_run |= i < runs.count && runs.len[i] >= a.inline_min_run;
       if (i < runs.count && runs.len[i] < a.inline_min_run) {
         len[i] = max(runs.pos[i], 0) + 1;
         tbl[i] = __ldg(a.table_offset + runs.seq[i]);
         slabs += share_padded(len[i]) / kShareSlab;
+        any_long |= len[i] > kMinShareKeys;
       }
     }
+    const bool may_halve = __syncthreads_or(any_long) != 0 && __syncthreads_or(in_run) == 0;
     int total;
     int at = block_scan<ScanSum, 4>(slabs, sm_scan[1], &total) - slabs;    // (and the barrier after which the arrays are free)
-    rule = share_rule(static_cast<long long>(total) * kShareSlab, a.inline_max_shares, a.inline_forced_chunk);
+    rule = share_rule(static_cast<long long>(total) * kShareSlab, a.inline_max_shares, a.inline_forced_chunk, may_halve);
     int begin[kPer], ns[kPer], sum = 0;                                    // items in the upper half, partials in the lower: < 2^16 each
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
@@ -330,7 +334,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
   // items of a (share, kv head) one after the other.  The issue side and the math side walk the same list,
   // each with a cursor of its own.
   static_assert(!INLINE_PLAN || (TOK == 1 && !FUSED_APPEND && !CLUSTER && !F32 && WARPS == 4), "mixed steps only");
-  InlinePlan ip;
+  InlinePlan ip = {};
   if constexpr (INLINE_PLAN) {
     if (!waited) {       // not behind a prefill launch that has waited for the index arrays' producers
       pdl_wait();

@@ -1037,7 +1037,7 @@ int prefill_launch(const void* q, const void* k_cache, const void* v_cache, cons
   a.done = tp.done;
   // Few items: the largest cluster per item that leaves all of them resident (up to 15 items eight blocks, 33
   // four, 73 two).  Measured per layer with its rope + append: 50 tokens behind 4,000 (6 items) 53.2 -> 16.7 us,
-  // 128 behind 2,000 (32 items) 33.6 -> 20.5; short fresh chunks, which no block shares, lose 1 to 2 us of 9
+  // 128 behind 2,000 (32 items) 33.6 -> 18.1; short fresh chunks, which no block shares, lose 1 to 2 us of 9
   // to 13 to the cluster launch.  A mixed step knows only a loose bound of its items, most often of none:
   // it keeps the ordinary launch.
   int cs = 0;

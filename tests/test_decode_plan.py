@@ -66,7 +66,7 @@ def check(image, pos, kvh):
 
 STEPS = {
     "one": [0], "one long": [70000], "slab edges": [30, 31, 32, 33, 63, 64, 65, 95, 96, 127, 128] * 40,
-    "small": [5, 300, 17, 129, 1500], "equal": [4095] * 256, "short": [99] * 1500, "single keys": [0] * 2500,
+    "small": [5, 300, 17, 129, 1500], "none long": [127, 3, 90, 64, 65, 127], "fine or not": [128] * 60, "equal": [4095] * 256, "short": [99] * 1500, "single keys": [0] * 2500,
     "ragged": np.random.default_rng(3).integers(0, 8192, size=256), "last token of one slab": [127] * 3551 + [31],
 }
 
@@ -96,7 +96,7 @@ def test_small_workspaces_take_fewer_shares(pkv, extra):
 @pytest.mark.parametrize("name", sorted(STEPS))
 def test_device_plan_is_the_host_plan(pkv, torch_cuda, name):
     """Same cuts, slots and shares, around the 1,024 tokens one pass of the planner block takes (chunked steps
-    list the same items in another order)."""
+    list the items in another order, and may have chunks half as long)."""
     torch = torch_cuda
     pos = np.asarray(STEPS[name], dtype=np.int32)
     for n in sorted({pos.size, min(pos.size, 1024), min(pos.size, 1025)}):
@@ -109,6 +109,9 @@ def test_device_plan_is_the_host_plan(pkv, torch_cuda, name):
         image, _ = host_image(pkv, p, 32, 4, 64)
         want = read(image, n, 4)
         check(plan.workspace.cpu().numpy(), p, 4)
+        if want[3] is None and got[0][2] == MIN_SHARE // 2:
+            assert want[0][2] == MIN_SHARE and p.max() >= MIN_SHARE and got[3] is None
+            continue
         assert got[0].tolist() == want[0].tolist() and (got[1][:, 1] == want[1][:, 1]).all()
         key = lambda items: sorted(map(tuple, items.tolist()))
         assert key(got[2]) == key(want[2])
