@@ -456,7 +456,7 @@ def run_ours(args, rank, local_rank, world):
     peak, peak_src = peaks()
     algo_bytes = w.decode_bytes_per_layer()
     achieved = algo_bytes / (attn_ms * 1e-3) / 1e9
-    roofline = {"bound": "hbm", "kernel": ("decode_tma_kernel + decode_combine_kernel" if w.dtype != "f32" else "decode_simt_kernel + decode_combine_kernel"),
+    roofline = {"bound": "hbm", "kernel": ("decode_tma_kernel + decode_combine_kernel" if w.dtype != "f32" else "decode_tma_kernel (fp32)"),
                 "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": NCU_TRAFFIC.get(args.workload, {}).get("bytes"),
                 "traffic_source": NCU_TRAFFIC.get(args.workload, {}).get("source"),
@@ -1086,7 +1086,7 @@ def measure_cow_rotated(pkv, torch, dev, pools, w, sets=8, pairs_per_set=127, wa
     torch.cuda.synchronize()
     us = a.elapsed_time(b) / waves * 1e3
     peak, _ = peaks()
-    return {"kernel": "copy_blocks_kernel", "pairs_per_wave": pairs_per_set, "pools": 2 * L, "disjoint_pair_sets_in_rotation": sets,
+    return {"kernel": "copy_blocks_bulk_kernel", "pairs_per_wave": pairs_per_set, "pools": 2 * L, "disjoint_pair_sets_in_rotation": sets,
             "bytes_read_plus_written_per_wave": wave_bytes, "bytes_between_reuse_of_a_block": wave_bytes * sets,
             "us_per_wave": us, "GBps": wave_bytes / us / 1e3, "frac_of_measured_hbm": wave_bytes / us / 1e3 / peak}
 
@@ -1160,7 +1160,7 @@ def run_cow(args, rank, local_rank, world):
                           "steps": max(args.steps, 8) * 4, "warmup": 8, "ms_per_step": res["us_per_wave"] / 1e3, "higher_is_better": True,
                           "scaling": "weak", "vs_baseline": None, "dtype": "u8", "data": "synthetic",
                           "config": {"workload": f"cow: {WORKLOAD_TEXT['cow']}", "l2": "a block is touched again only after 8 waves (733 MB) of other traffic"},
-                          "roofline": {"bound": "hbm", "kernel": "copy_blocks_kernel", "achieved": res["GBps"], "peak": peak, "unit": "GB/s",
+                          "roofline": {"bound": "hbm", "kernel": "copy_blocks_bulk_kernel", "achieved": res["GBps"], "peak": peak, "unit": "GB/s",
                                        "frac": res["GBps"] / peak, "traffic": None, "peak_source": src,
                                        "algorithmic_bytes_per_launch": res["bytes_read_plus_written_per_wave"], "us_per_launch": res["us_per_wave"]},
                           "cpu_baseline": None, "e2e": None, "gpu_launches": max(args.steps, 8) * 4, "clocks": clocks, "detail": res}), flush=True)
