@@ -531,7 +531,11 @@ int launch_decode_main(const DecodeArgs& a, int grid, cudaStream_t stream, bool*
   }
   *log2_domain = false;
   if constexpr (IsF32<T>::value) {
-    if (tma_path<T>(a))
+    // Without a plan a unit is a token's whole history, which the SIMT kernel gives to the four warps of a block and
+    // the TMA kernel to one: four times the chain, in time (us a layer with its append, TMA and SIMT: 4 kv heads, 1 x
+    // 4,000 keys 275, 227; 8 x 2,000 141, 117; 150 x 50-500 49, 38) and in rounding (1 x 4,000 keys against 64 bits
+    // 1.1e-6, 6.8e-7).
+    if (tma_path<T>(a) && !a.direct)
       return a.head_dim == 64 ? launch_tma<T, 64, 1, 1, 2, 4, 3>(a, grid, stream) : launch_tma<T, 128, 1, 1, 2, 3, 2>(a, grid, stream);
   }
   const int dj = (a.head_dim + 31) / 32;

@@ -3,7 +3,7 @@ head dims, slab edges (16 keys), whole-history units, chunks, shares and the clu
 import numpy as np
 import pytest
 
-from tests.gpu_util import Case, check_case
+from tests.gpu_util import Case, check_case, from_device
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +38,30 @@ def test_cluster_form(pkv, orc, torch_cuda, ctx):
     before = pkv.lib().pkv_debug_cluster_launches()
     check_case(case, pkv, torch_cuda, orc, "host_plan")
     assert d["plan"].plan.cluster >= 2 and pkv.lib().pkv_debug_cluster_launches() == before + 1
+
+
+def in_64_bits(case):
+    out = np.empty((case.N, case.qh, case.hd))
+    kc, vc = (x.copy().reshape(-1, case.kvh, case.hd).astype(np.float64) for x in (case.kc, case.vc))
+    kc[case.idx.slots], vc[case.idx.slots] = (x.reshape(-1, case.kvh, case.hd) for x in (case.k, case.v))
+    for t in range(case.N):
+        pos = np.arange(case.idx.token_pos[t] + 1)
+        table = case.idx.block_tables[case.idx.table_offset[case.idx.token_seq[t]]:]
+        rows = table[pos // case.bs] * case.bs + pos % case.bs
+        q = case.q[t].reshape(case.kvh, -1, case.hd).astype(np.float64)
+        s = np.einsum("gid,kgd->gik", q, kc[rows]) * case.scale
+        w = np.exp(s - s.max(-1, keepdims=True))
+        out[t] = np.einsum("gik,kgd->gid", w / w.sum(-1, keepdims=True), vc[rows]).reshape(case.qh, case.hd)
+    return out
+
+
+@pytest.mark.parametrize("qh,kvh,hd,keys", [(4, 4, 64, 4000), (14, 2, 64, 8000), (8, 2, 128, 8000), (16, 2, 128, 3001)])
+def test_long_histories_without_a_workspace(pkv, orc, torch_cuda, qh, kvh, hd, keys):
+    """A whole history is summed by the four warps of a block.  A chain of n terms of random sign, each step rounded
+    to 24 bits, ends up 2^-24 sqrt(n / 6) of the sum away; n = keys / 4, a fifth more allowed for the exponentials.
+    (One chain of all the keys is twice that.)"""
+    case = make(orc, pkv, qh, kvh, hd, 16, [keys - 1, keys - 20, keys - 333], seed=keys)
+    check_case(case, pkv, torch_cuda, orc, "direct")
+    got = from_device(torch_cuda, orc, case.run_gpu(pkv, torch_cuda, "direct")["out"], "f32")[1].reshape(case.N, qh, hd).astype(np.float64)
+    want = in_64_bits(case)
+    assert np.linalg.norm(got - want) <= 1.2 * 2.0 ** -24 * np.sqrt(keys / 24) * np.linalg.norm(want)
