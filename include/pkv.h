@@ -65,7 +65,8 @@ const char* pkv_last_error(void);
  * pipeline wait; 8: a peer GPU's flag in the head-sharded exchange; 16: a block copy -- kept in two
  * places: a device word, and one pinned host word the kernels store to.  The attention
  * entry points (pkv_decode_attn_*, the planned, fused, peer and mixed forms,
- * pkv_prefill_attn_*) look at the host word before they enqueue anything: the first
+ * pkv_prefill_attn_*) look at the host word before they enqueue anything, and so do
+ * pkv_copy_blocks_* for the bit of an earlier copy: the first
  * such call after an incomplete launch has reached the host returns PKV_E_CUDA once,
  * with the bits in pkv_last_error(), and enqueues nothing; the record is cleared by
  * that report and the next call runs normally (nothing is disabled).  The three
@@ -73,7 +74,7 @@ const char* pkv_last_error(void);
  *
  * pkv_debug_device_flags is the one entry point that SYNCHRONISES the device: it
  * reads and clears both records (0: no kernel gave up).
- * pkv_debug_set_reported_flags is a testing aid: it makes the next attention call
+ * pkv_debug_set_reported_flags is a testing aid: it makes the next call that looks
  * behave as if a kernel had recorded `flags` (works without a GPU).
  * No llm-engine counterparts. */
 int pkv_debug_device_flags(unsigned int* flags);

@@ -12,6 +12,7 @@
 
 namespace pkv {
 unsigned int* error_mirror(bool create);                 // error_mirror.cu
+int check_error_mirror(const char* fn, unsigned int bits);
 
 __device__ unsigned int g_pkv_copy_error = 0;
 
@@ -70,10 +71,11 @@ __global__ void __launch_bounds__(32) copy_blocks_bulk_kernel(TwoPools two, void
   unsigned long long slot_dst[kBulkStages];
   unsigned slot_bytes[kBulkStages];
   unsigned long long at = 0;                        // copies looked at
-  unsigned head = 0, tail = 0;                      // loads issued, stores issued
+  unsigned head = 0, tail = 0;                      // loads issued, loads done with
+  bool gave_up = false;
   for (;;) {
     // fill the ring: the slot of load `head` was last read by store head - kBulkStages, which is not the newest
-    while (at < mine && head - tail < (tail ? kBulkStages - 1 : kBulkStages)) {
+    while (!gave_up && at < mine && head - tail < (tail ? kBulkStages - 1 : kBulkStages)) {
       if (at % 32 == 0) {
         my_bytes = 0;
         if (at + lane < mine) {
@@ -103,11 +105,17 @@ __global__ void __launch_bounds__(32) copy_blocks_bulk_kernel(TwoPools two, void
     }
     if (tail == head) break;
     const unsigned slot = tail % kBulkStages;
-    if (!mbar_wait(smem_u32(&full[slot]), (tail / kBulkStages) & 1u)) {
+    // A wait that runs out ends the block's copies, but not before every load that is still on its way into the
+    // ring has been waited for (as long again, once each) and those that arrive have been stored: the ring's memory
+    // goes to another block when this one leaves.
+    bool landed = mbar_wait(smem_u32(&full[slot]), (tail / kBulkStages) & 1u);
+    landed = __all_sync(0xffffffffu, landed);
+    if (!landed && !gave_up) {
+      gave_up = true;
       if (lane == 0) copy_give_up(host_err);
-      break;
+      continue;
     }
-    if (lane == 0) {
+    if (lane == 0 && landed) {
 #pragma unroll
       for (int i = 0; i < kBulkStages; ++i)
         if (i == static_cast<int>(slot)) bulk_store(reinterpret_cast<void*>(slot_dst[i]), smem_u32(ring) + i * kBulkBytes, slot_bytes[i]);
@@ -138,13 +146,15 @@ int copy_impl(TwoPools two, void* const* pools, int n_pools, bool pools_aligned,
   if (!pairs) return fail(PKV_E_ARG, "pkv_copy_blocks: null pair list");
   if (n_pairs > 65535 || n_pools > 65535)
     return fail(PKV_E_UNSUPPORTED, "pkv_copy_blocks: at most 65535 pairs and 65535 pools per call (got %d, %d)", n_pairs, n_pools);
+  const int st = check_error_mirror("pkv_copy_blocks", kErrCopyWait);   // a copy that gave up; anything else is the attention calls' to report
+  if (st != PKV_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (block_bytes % 16 == 0 && pools_aligned) {
     const unsigned long long pieces = (block_bytes + kBulkBytes - 1) / kBulkBytes, tasks = pieces * n_pairs * n_pools;
     const unsigned blocks = static_cast<unsigned>(std::min<unsigned long long>(tasks, 148 * kBulkBlocksPerSm));
     auto kern = pools ? copy_blocks_bulk_kernel<true> : copy_blocks_bulk_kernel<false>;
     launch_pdl(kern, dim3(blocks), dim3(32), kBulkStages * kBulkBytes, s, two, pools, pairs, n_pairs, block_bytes, pieces, tasks,
-               error_mirror(false));
+               error_mirror(true));
     return check_launch("copy_blocks_bulk_kernel");
   }
   dim3 grid(static_cast<unsigned>((block_bytes + kCopyThreads * 8 - 1) / (kCopyThreads * 8)), n_pairs, n_pools);

@@ -28,8 +28,8 @@ int prefill_launch(const void* q, const void* k_cache, const void* v_cache, cons
                    int n_tokens, int n_seqs, int max_q_len, int q_heads, int kv_heads, int head_dim, int block_size,
                    int num_blocks, float scale, pkv_stream stream, const int* d_dims, bool may_allocate, const InlineRuns* runs);
 unsigned int* error_mirror(bool create);      // error_mirror.cu
-unsigned int take_error_mirror();
-int check_error_mirror(const char* fn);
+unsigned int take_error_mirror(unsigned int bits = ~0u);
+int check_error_mirror(const char* fn, unsigned int bits = ~0u);
 namespace {
 
 // ---- tuning knobs (read once) ---------------------------------------------------

@@ -759,9 +759,12 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
       }
       ++n_consumed;
     }
-    if constexpr (!CLUSTER) {
-      if (!ok) break;   // this warp has copies in flight only into its own ring; nothing else depends on it
-    }                   // (in a cluster the warp stays for the barriers; its give-up is on record)
+    if (!ok) {
+      // The copies still on their way into this warp's ring are waited for (as long again, once each): the ring's
+      // memory goes to another block when this one leaves.
+      for (uint32_t i = n_consumed; i != n_issued; ++i) mbar_wait(bars + 8 * (i % NSTAGES), (i / NSTAGES) & 1u);
+      if constexpr (!CLUSTER) break;   // (in a cluster the warp stays for the barriers; its give-up is on record)
+    }
 
     while (more && n_issued - n_consumed < NSTAGES) more = issue_next();  // keep loads flowing through the finish
 

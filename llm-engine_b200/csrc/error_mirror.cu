@@ -3,9 +3,9 @@
 // Every wait inside the kernels is bounded; a wait that runs out leaves a bit in a device word
 // (pkv_debug_device_flags reads it, synchronising) and, so that the caller learns of it without
 // synchronising, in one pinned host word that the kernels can store to.  The attention entry points
-// look at that word before they enqueue anything: the call that follows an incomplete launch
-// returns PKV_E_CUDA once (the word is cleared by the report), in the manner of CUDA's own
-// asynchronous errors.  The launch after that runs normally: nothing is disabled.
+// look at that word before they enqueue anything, and so do the block copies for a copy's bit: the call
+// that follows an incomplete launch returns PKV_E_CUDA once (the word is cleared by the report), in the
+// manner of CUDA's own asynchronous errors.  The launch after that runs normally: nothing is disabled.
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -29,7 +29,12 @@ unsigned int* error_mirror(bool create) {
   if (g_mirror || !create || g_tried) return g_mirror;
   g_tried = true;
   void* p = nullptr;
-  if (cudaHostAlloc(&p, 64, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess && p) {
+  // the first call may be one that is being captured into a graph, which an allocation must not end
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  const cudaError_t e = cudaHostAlloc(&p, 64, cudaHostAllocPortable | cudaHostAllocMapped);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e == cudaSuccess && p) {
     std::memset(p, 0, 64);
     __atomic_store_n(&g_mirror, static_cast<unsigned int*>(p), __ATOMIC_RELEASE);
   } else {
@@ -38,23 +43,24 @@ unsigned int* error_mirror(bool create) {
   return g_mirror;
 }
 
-unsigned int take_error_mirror() {
+// Takes those of `bits` that are recorded.
+unsigned int take_error_mirror(unsigned int bits) {
   // the common case -- nothing recorded -- is two plain loads, no lock and no write
   unsigned int* m = __atomic_load_n(&g_mirror, __ATOMIC_ACQUIRE);
-  if (__atomic_load_n(&g_plain, __ATOMIC_RELAXED) == 0 && (!m || __atomic_load_n(m, __ATOMIC_RELAXED) == 0)) return 0;
+  if ((__atomic_load_n(&g_plain, __ATOMIC_RELAXED) & bits) == 0 && (!m || (__atomic_load_n(m, __ATOMIC_RELAXED) & bits) == 0)) return 0;
   std::lock_guard<std::mutex> lock(g_mu);
-  unsigned int v = g_plain;
-  g_plain = 0;
-  if (g_mirror) v |= __atomic_exchange_n(g_mirror, 0u, __ATOMIC_ACQ_REL);
+  unsigned int v = g_plain & bits;
+  g_plain &= ~bits;
+  if (g_mirror) v |= __atomic_fetch_and(g_mirror, ~bits, __ATOMIC_ACQ_REL) & bits;
   return v;
 }
 
-int check_error_mirror(const char* fn) {
-  const unsigned int v = take_error_mirror();
+int check_error_mirror(const char* fn, unsigned int bits) {
+  const unsigned int v = take_error_mirror(bits);
   if (!v) return PKV_OK;
   return fail(PKV_E_CUDA,
               "%s: an earlier launch gave up on a bounded wait (flags 0x%x: 1 TMA producer, 2 tile consumer, 4 prefill "
-              "pipeline, 8 peer GPU) and left its output incomplete; this call enqueued nothing, the next one runs normally",
+              "pipeline, 8 peer GPU, 16 block copy) and left its output incomplete; this call enqueued nothing, the next one runs normally",
               fn, v);
 }
 

@@ -428,6 +428,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   if (warp == kProducerWarp) {
     // ================================ TMA producer ================================
     int n = 0, g = 0;
+    int q_sent = 0, kv_sent = 0;                               // lane 0: up to which loads have been issued
     unsigned round = 0;                                        // fixed deal: items taken so far
     const int n_slots = ((a.dims ? __ldcg(a.dims + 1) : a.max_q_len) + tt - 1) / tt;   // tiles of the longest chunk
     const unsigned n_items = (ranked ? static_cast<unsigned>(s_cum[kBuckets - 1]) : static_cast<unsigned>(n_seqs) * n_slots) * a.head_tiles;
@@ -519,11 +520,13 @@ __global__ void __launch_bounds__(kThreads, 2)
         if (d.n_kt == 0 && !dead) {
           mbar_arrive(BAR(Q_FULL + qb));        // the item is the team's, but this block has no part of its keys
         } else if (d.n_kt > 0 && !dead) {
+          q_sent = n + 1;
           mbar_arrive_expect_tx(BAR(Q_FULL + qb), static_cast<uint32_t>(a.pack * a.tile_tokens) * 128u);
           tma_load_3d(sQ + qb * kQBytes, &qmap, 0, d.head, d.row0, BAR(Q_FULL + qb));
         } else {
           s_item[qb].n_kt = -1;
-          mbar_arrive(BAR(Q_FULL + qb));        // "no more items"
+          // "no more items"; after a give-up the buffer's last tile may still be on its way: it has to arrive first
+          if (!dead || n < 2 || mbar_wait(BAR(Q_FULL + qb), ((n >> 1) & 1) ^ 1)) mbar_arrive(BAR(Q_FULL + qb));
         }
       }
       dead = __shfl_sync(0xffffffffu, dead ? 1 : 0, 0) != 0;
@@ -546,13 +549,16 @@ __global__ void __launch_bounds__(kThreads, 2)
           int nvalid = 0;
 #pragma unroll
           for (int b = 0; b < 4; ++b) nvalid += (j * kKTile + 16 * b < d.kv_total) ? 1 : 0;
-          mbar_arrive_expect_tx(BAR(KV_FULL + st), static_cast<uint32_t>(nvalid) * 2u * kBox);
-          const uint32_t kdst = sKV + st * 2 * kKBytes, vdst = kdst + kKBytes;
+          if (!dead) {
+            kv_sent = g + 1;
+            mbar_arrive_expect_tx(BAR(KV_FULL + st), static_cast<uint32_t>(nvalid) * 2u * kBox);
+            const uint32_t kdst = sKV + st * 2 * kKBytes, vdst = kdst + kKBytes;
 #pragma unroll
-          for (int b = 0; b < 4; ++b) {
-            if (j * kKTile + 16 * b < d.kv_total) {
-              tma_load_2d(kdst + b * kBox, &kmap, kvh * kHd, y[b], BAR(KV_FULL + st));
-              tma_load_2d(vdst + b * kBox, &vmap, kvh * kHd, y[b], BAR(KV_FULL + st));
+            for (int b = 0; b < 4; ++b) {
+              if (j * kKTile + 16 * b < d.kv_total) {
+                tma_load_2d(kdst + b * kBox, &kmap, kvh * kHd, y[b], BAR(KV_FULL + st));
+                tma_load_2d(vdst + b * kBox, &vmap, kvh * kHd, y[b], BAR(KV_FULL + st));
+              }
             }
           }
         }
@@ -560,6 +566,13 @@ __global__ void __launch_bounds__(kThreads, 2)
       }
       ++n;
     }
+    // Everything this warp has sent for has arrived before the block leaves, whoever gave up on it (the memory goes
+    // to another block): the last load of every stage and the last Q tile, once each, with the usual limit.
+    if (lane == 0) {
+      for (int i = max(kv_sent - kKVStages, 0); i < kv_sent; ++i) mbar_wait(BAR(KV_FULL + i % kKVStages), (i / kKVStages) & 1);
+      if (q_sent > 0) mbar_wait(BAR(Q_FULL + ((q_sent - 1) & 1)), ((q_sent - 1) >> 1) & 1);
+    }
+    __syncwarp();
   } else if (warp == kMmaWarp) {
     // ================================ MMA issuer ================================
     // One thread issues everything.  A tcgen05.mma returns to the issuing thread at the rate the
@@ -926,7 +939,7 @@ TicketPair ticket_pair_for(cudaStream_t stream, int dev) {
 }  // namespace
 
 unsigned int* error_mirror(bool create);                 // error_mirror.cu
-int check_error_mirror(const char* fn);
+int check_error_mirror(const char* fn, unsigned int bits = ~0u);
 
 // Shared by the C entry points below and by the mixed-step router (decode_attn.cu).  With d_dims the
 // per-sequence arrays and their counts come from an earlier kernel on the stream: n_seqs and

@@ -224,3 +224,22 @@ def test_launcher_symbols_throw_what_the_c_abi_returns(pkv, tmp_path):
     assert H.harness_layer(*args(4, 14, 2)) == 1 and b"gave up" in err.value and b"launch_attention_decode" in err.value
     assert H.harness_layer(*args(0, 14, 2)) == 0          # an empty step is a silent no-op
     assert pkv.lib().pkv_mixed_attn_workspace_bytes(300, 14, 2, 64) > pkv.lib().pkv_decode_workspace_bytes(300, 14, 2, 64)
+
+
+def test_a_copy_that_gave_up_is_reported_by_the_next_copy_or_attention_call(pkv):
+    """Block copies wait too (bit 16): the next copy says so, or the next attention call, whichever comes first.  What
+    an attention launch recorded is left to the attention calls: a copy behind one runs."""
+    L = pkv.lib()
+    one = 0x1000
+    f = C.c_float(0.125)
+    copies = (lambda: L.pkv_copy_blocks_layers(one, 4, None, 3, 8192, None), lambda: L.pkv_copy_blocks_bf16(one, one, one, 3, 16, 128, None))
+    assert L.pkv_debug_set_reported_flags(16) == 0
+    assert copies[1]() == pkv._lib.PKV_E_CUDA
+    assert "16 block copy" in L.pkv_last_error().decode() and "0x10:" in L.pkv_last_error().decode()
+    assert L.pkv_debug_set_reported_flags(16 | 2) == 0
+    assert L.pkv_copy_blocks_layers(one, 4, one, 3, 8192, None) == pkv._lib.PKV_E_CUDA and "0x10:" in L.pkv_last_error().decode()
+    assert copies[0]() == pkv._lib.PKV_E_ARG                 # cleared; bit 2 does not stop it from looking at its arguments
+    attention = lambda: L.pkv_decode_attn_bf16(one, one, one, one, one, one, one, one, 4, 14, 2, 64, 16, f, None, 0, None)
+    assert attention() == pkv._lib.PKV_E_CUDA and "0x2:" in L.pkv_last_error().decode()
+    assert L.pkv_debug_set_reported_flags(16) == 0
+    assert attention() == pkv._lib.PKV_E_CUDA and "0x10:" in L.pkv_last_error().decode()
