@@ -106,22 +106,23 @@ struct RouteArgs {
 // (The kernel it replaces made one histogram per chunk candidate and five passes with three to five barriers
 // each: 6.8 us for 48 tokens, 7.9 us for 620.)
 template <bool ROUTE>
-__global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __restrict__ token_pos, int n_tokens, int max_shares,
-                                                                    int forced_chunk, int kv_heads, PlanHeader* header,
+__global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __restrict__ token_pos, int n_tokens, const PlanLimits lim,
+                                                                    PlanHeader* header,
                                                                     TokSplit* tok_split, int* counters, WorkItem* items,
                                                                     const RouteArgs r) {
   extern __shared__ int sm_first[];                       // [max_shares + 1] first item of every share
   __shared__ int sm_scan[8][kPlanThreads / 32];
   __shared__ int sm_len[kPlanThreads];                    // run lengths of a step of up to kPlanThreads tokens
   __shared__ int sm_start[kPlanThreads + 1];              // ... and whether a run starts at a token
-  __shared__ int sm_misc[4];                              // long runs, longest of them, tokens of none
+  __shared__ int sm_misc[4];                              // long runs, longest of them, tokens of none, longest token
   const int tid = threadIdx.x;
   const bool small = n_tokens <= kPlanThreads;
   // the next launch on the stream is the prefill kernel, which waits for this one before it reads anything
   if constexpr (ROUTE) pdl_launch_dependents();
   if (tid < 4) sm_misc[tid] = 0;
-  for (int i = tid; i <= max_shares; i += kPlanThreads) sm_first[i] = 0x7fffffff;
+  for (int i = tid; i <= lim.max_shares; i += kPlanThreads) sm_first[i] = 0x7fffffff;
   if (tid == 0) sm_start[n_tokens < kPlanThreads ? n_tokens : kPlanThreads] = 1;
+  __syncthreads();
   pdl_wait();
   if (tid == 0) counters[0] = 0;
 
@@ -217,29 +218,36 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
     return max(token_pos[t], 0) + 1;
   };
 
-  // padded keys of the whole step -> how it is cut
+  // padded keys of the whole step and its longest token -> how it is cut
   long long total = 0;
   long long my_begin = 0;                                  // where token tid begins in the laid-out step, when it is small
+  int longest = my_len;
   if (small) {
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if ((tid & 31) == 0) atomicMax(&sm_misc[3], longest);
     int tot;
     const int p = share_padded(my_len) / kShareSlab;       // scanned in slabs: 32 bits hold 2^36 keys
     my_begin = static_cast<long long>(block_scan<ScanSum, kPlanThreads / 32>(p, sm_scan[2], &tot) - p) * kShareSlab;
     total = static_cast<long long>(tot) * kShareSlab;
   } else {
     long long loc = 0;
-    for (int t = tid; t < n_tokens; t += kPlanThreads) loc += share_padded(length_of(t));
+    longest = 0;
+    for (int t = tid; t < n_tokens; t += kPlanThreads) {
+      const int L = length_of(t);
+      loc += share_padded(L);
+      longest = max(longest, L);
+    }
     for (int o = 16; o > 0; o >>= 1) loc += __shfl_xor_sync(0xffffffffu, loc, o);
+    longest = __reduce_max_sync(0xffffffffu, longest);
     __shared__ long long sm_tot[kPlanThreads / 32];
-    if ((tid & 31) == 0) sm_tot[tid >> 5] = loc;
+    if ((tid & 31) == 0) {
+      sm_tot[tid >> 5] = loc;
+      atomicMax(&sm_misc[3], longest);
+    }
     __syncthreads();
     for (int w = 0; w < kPlanThreads / 32; ++w) total += sm_tot[w];
   }
-  bool any_long = small && my_len > kMinShareKeys;
-  if (!small)
-    for (int t = tid; t < n_tokens; t += kPlanThreads) any_long |= length_of(t) > kMinShareKeys;
-  bool may_halve = __syncthreads_or(any_long) != 0;
-  if constexpr (ROUTE) may_halve = may_halve && sm_misc[0] == 0;
-  const ShareRule rule = share_rule(total, max_shares, forced_chunk, may_halve);
+  const ShareRule rule = share_rule(total, sm_misc[3], n_tokens, lim, !ROUTE || sm_misc[0] == 0);
 
   int n_items = 0, n_parts = 0;
   long long carry_begin = 0;
@@ -299,7 +307,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
     header->chunk = rule.per > 0 ? rule.per : rule.chunk;
     header->n_tokens = n_tokens;
     header->n_parts = n_parts;
-    header->kv_heads = kv_heads;
+    header->kv_heads = lim.kv_heads;
     header->n_shares = rule.n_shares;
     header->pad = 0;
   }
@@ -620,7 +628,7 @@ void fill_args(DecodeArgs& a, const void* q, const void* kc, const void* vc, con
   a.new_k = nullptr; a.new_v = nullptr; a.slots = nullptr;
   a.host_err = nullptr;
   a.wait_last = 0;
-  a.inline_min_run = 0; a.inline_max_shares = 0; a.inline_forced_chunk = 0;
+  a.inline_min_run = 0; a.inline_max_shares = 0;
   a.pool_rows = 1ull << 30;
 }
 
@@ -646,10 +654,21 @@ int persistent_grid() {
   return sms * 4;
 }
 
-// Warps the attention kernel of this geometry keeps resident: what a step's keys are shared out over.
-int decode_workers(int q_heads, int kv_heads, int head_dim) {
-  (void)q_heads; (void)kv_heads;
-  return persistent_sms() * (head_dim == 128 ? 8 : 12);
+// Whether these heads run on the TMA or the tensor-core kernel, as far as a planner can tell: it knows neither the
+// element type nor the block size (calls that plan for themselves do: shares_ok).
+bool tensor_heads(int q_heads, int kv_heads, int head_dim) {
+  return (head_dim == 64 || head_dim == 128) && q_heads / kv_heads <= 16;
+}
+PlanLimits plan_limits(int budget, int q_heads, int kv_heads, int head_dim, bool shares) {
+  const int warps = head_dim == 128 ? 8 : 12;             // that the TMA kernel keeps resident on an SM (launch_decode_main)
+  PlanLimits lim;
+  lim.max_shares = max_shares_for(budget, persistent_sms() * warps / kv_heads);
+  lim.max_extra = budget;
+  lim.kv_heads = kv_heads;
+  lim.wave_units = tuning().wave_ctas;
+  lim.forced_chunk = tuning().forced_chunk;
+  lim.shares = shares && tensor_heads(q_heads, kv_heads, head_dim) ? 1 : 0;
+  return lim;
 }
 
 // Budget of extra items for this workspace: what fits, capped by the target grid.
@@ -662,7 +681,8 @@ int plan_budget(int n_tokens, int q_heads, int kv_heads, int head_dim, size_t wo
 }
 
 int plan_device(const int* token_pos, int n_tokens, int q_heads, int kv_heads, int head_dim, void* workspace,
-                size_t workspace_bytes, cudaStream_t stream, pkv_decode_plan* plan, const RouteArgs* route = nullptr) {
+                size_t workspace_bytes, cudaStream_t stream, pkv_decode_plan* plan, const RouteArgs* route = nullptr,
+                bool shares = true) {
   if (!token_pos || !workspace || !plan) return fail(PKV_E_ARG, "pkv_decode_plan_device: null pointer");
   std::memset(plan, 0, sizeof(*plan));
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return fail(PKV_E_ARG, "pkv_decode_plan_device: workspace must be 256-byte aligned");
@@ -671,10 +691,10 @@ int plan_device(const int* token_pos, int n_tokens, int q_heads, int kv_heads, i
   if (budget < 0)
     return fail(PKV_E_WORKSPACE, "pkv_decode_plan_device: workspace of %zu bytes cannot hold the plan for %d tokens", workspace_bytes, n_tokens);
   char* base = static_cast<char*>(workspace);
-  const int max_shares = max_shares_for(w.cap_extra < budget ? w.cap_extra : budget, decode_workers(q_heads, kv_heads, head_dim) / kv_heads);
-  const size_t smem = sizeof(int) * static_cast<size_t>(max_shares + 1);
+  const PlanLimits lim = plan_limits(budget, q_heads, kv_heads, head_dim, shares);
+  const size_t smem = sizeof(int) * static_cast<size_t>(lim.max_shares + 1);
   auto kern = route ? decode_plan_kernel<true> : decode_plan_kernel<false>;
-  launch_pdl(kern, dim3(1), dim3(kPlanThreads), smem, stream, token_pos, n_tokens, max_shares, tuning().forced_chunk, kv_heads,
+  launch_pdl(kern, dim3(1), dim3(kPlanThreads), smem, stream, token_pos, n_tokens, lim,
              reinterpret_cast<PlanHeader*>(base), reinterpret_cast<TokSplit*>(base + w.off_tok),
              reinterpret_cast<int*>(base + w.off_cnt), reinterpret_cast<WorkItem*>(base + w.off_items),
              route ? *route : RouteArgs{});
@@ -726,8 +746,7 @@ int decode_planned(const pkv_decode_plan* plan, const void* q, const void* kc, c
   a.wait_last = wait_last ? 1 : 0;
   if (inline_min_run > 0) {
     a.inline_min_run = inline_min_run;
-    a.inline_max_shares = max_shares_for(budget, decode_workers(a.q_heads, a.kv_heads, a.head_dim) / a.kv_heads);
-    a.inline_forced_chunk = tuning().forced_chunk;
+    a.inline_max_shares = plan_limits(budget, a.q_heads, a.kv_heads, a.head_dim, true).max_shares;
   }
   if (plan->num_blocks > 0) a.pool_rows = static_cast<unsigned long long>(plan->num_blocks) * block_size;
   if (peers) {
@@ -782,13 +801,22 @@ int decode_planned(const pkv_decode_plan* plan, const void* q, const void* kc, c
   return launch_decode<T>(a, static_cast<int>(blocks), static_cast<cudaStream_t>(stream), (plan->reserved & 1) != 0);
 }
 
-// Whether the attention kernel can plan a step of n_tokens for itself.
 template <typename T>
-bool inline_plan_ok(int n_tokens, int q_heads, int kv_heads, int head_dim, int block_size, float scale) {
-  if (IsF32<T>::value || head_dim != 64 || n_tokens > kInlineTokens || tuning().variant >= 4) return false;
+bool on_tma_kernel(int n_tokens, int q_heads, int kv_heads, int head_dim, int block_size, float scale) {
   DecodeArgs probe;
   fill_args(probe, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, n_tokens, q_heads, kv_heads, head_dim, block_size, scale);
   return tma_path<T>(probe);
+}
+// Whether shares are for the kernel of this geometry (PlanLimits::shares).
+template <typename T>
+bool shares_ok(int n_tokens, int q_heads, int kv_heads, int head_dim, int block_size, float scale) {
+  return on_tma_kernel<T>(n_tokens, q_heads, kv_heads, head_dim, block_size, scale) || (!IsF32<T>::value && log2_exact(block_size) >= 0);
+}
+// Whether the attention kernel can plan a step of n_tokens for itself.
+template <typename T>
+bool inline_plan_ok(int n_tokens, int q_heads, int kv_heads, int head_dim, int block_size, float scale) {
+  return !IsF32<T>::value && head_dim == 64 && n_tokens <= kInlineTokens && tuning().variant < 4 && tuning().forced_chunk == 0 &&
+         on_tma_kernel<T>(n_tokens, q_heads, kv_heads, head_dim, block_size, scale);
 }
 // The plan record of such a step: upper bounds only.
 int inline_plan(const char* fn, int n_tokens, int q_heads, int kv_heads, int head_dim, void* workspace, size_t workspace_bytes,
@@ -834,7 +862,8 @@ int decode_all_in_one(const void* q, const void* kc, const void* vc, const int* 
     return decode_planned<T>(&plan, q, kc, vc, bt, to, ts, tp, out, block_size, scale, workspace, workspace_bytes, stream,
                              nullptr, nullptr, may_allocate, false, 0x7fffffff);
   }
-  st = plan_device(tp, n_tokens, q_heads, kv_heads, head_dim, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), &plan);
+  st = plan_device(tp, n_tokens, q_heads, kv_heads, head_dim, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), &plan, nullptr,
+                   shares_ok<T>(n_tokens, q_heads, kv_heads, head_dim, block_size, scale));
   if (st != PKV_OK) return st;
   return decode_planned<T>(&plan, q, kc, vc, bt, to, ts, tp, out, block_size, scale, workspace, workspace_bytes, stream,
                            nullptr, nullptr, may_allocate);
@@ -908,7 +937,8 @@ int mixed_attn(const void* q, const void* kc, const void* vc, const int* bt, con
     st = inline_plan(fn, n_tokens, q_heads, kv_heads, head_dim, workspace, dec_bytes, &plan);
     if (st != PKV_OK) return st;
   } else {
-    st = plan_device(tp, n_tokens, q_heads, kv_heads, head_dim, workspace, dec_bytes, static_cast<cudaStream_t>(stream), &plan, &r);
+    st = plan_device(tp, n_tokens, q_heads, kv_heads, head_dim, workspace, dec_bytes, static_cast<cudaStream_t>(stream), &plan, &r,
+                     shares_ok<T>(n_tokens, q_heads, kv_heads, head_dim, block_size, scale));
     if (st != PKV_OK) return st;
   }
   plan.num_blocks = num_blocks > 0 ? num_blocks : 0;
@@ -983,8 +1013,7 @@ static int plan_host_image(const char* fn, const int* h_token_pos, int n_tokens,
     total += share_padded(h_token_pos[t] + 1);
     max_len = std::max(max_len, h_token_pos[t] + 1);
   }
-  const int max_shares = max_shares_for(budget, decode_workers(q_heads, kv_heads, head_dim) / kv_heads);
-  const ShareRule rule = share_rule(total, max_shares, tuning().forced_chunk, false);
+  const ShareRule rule = share_rule(total, max_len, n_tokens, plan_limits(budget, q_heads, kv_heads, head_dim, true), false);
   const int chunk = rule.chunk;
   long long n_items = n_tokens;
   if (rule.per > 0) {

@@ -81,7 +81,7 @@ struct DecodeArgs {
   // (decode_tma_kernel with INLINE_PLAN, steps of up to kInlineTokens tokens), leaving runs of at least this many
   // tokens to the prefill kernel, and write tok_split for the merge.
   int inline_min_run;
-  int inline_max_shares, inline_forced_chunk;
+  int inline_max_shares;
   unsigned long long pool_rows;   // slots the K/V tensor maps cover (the pool size when the caller gave it, else a bound)
 };
 

@@ -124,16 +124,15 @@ inline int ws_extra_for_bytes(int n_tokens, int q_heads, int kv_heads, int head_
 // or less work on some warps and 1,100 partials, where shares give each warp the same 1,145 keys
 // and 650 partials.
 constexpr int kShareSlab = 32;
-// Below this many keys a share the tokens are cut one by one into chunks of this length instead:
-// equal shares would cut short tokens that need no merge at all when left whole.
+// Below this many keys a share the tokens are cut one by one into chunks instead (chunk_rule): equal shares would cut
+// short tokens that need no merge at all when left whole.
 constexpr int kMinShareKeys = 128;
-// ... and of half that when there are so few keys a share that the longest units decide: four dependent slabs a
-// warp become two.  Only in steps planned on the device that have something to merge anyway (a token of more
-// than kMinShareKeys keys) and no prefill chunk, whose kernel the decode units hide behind (a mixed step of two
-// chunks and 20 decode tokens lost 3 %); small host-planned steps take the cluster form.
-// Engine decode steps, us a layer with 128- and 64-key chunks: 1 sequence of 333 keys 10.8, 9.4; 6 of 100-900 (4 kv
-// heads) 12.0, 10.7; 40 of 50-1,000 14.4, 12.9 (15 keys a share); 100 of 60-300 16.8, 16.3 (33); 48 of 32-1,500
-// 16.8, 17.5 (41); 100 of 60-2,000 17.7, 19.9 (63).
+// Chunks go down to this length when there are so few keys a share that the longest units decide: four dependent slabs
+// a warp become two.  Only in steps planned on the device that have no prefill chunk, whose kernel the decode units
+// hide behind; small host-planned steps take the cluster form.  Engine decode steps, us a layer with 128- and 64-key chunks: 1 sequence of 333 keys 11.7, 10.2; 6 of 100-900
+// (4 kv heads) 12.4, 11.0; 40 of 50-1,000 14.7, 13.3 (15 keys a share); 60 of 60-300 16.3, 15.1 (23); 80 of 60-300 16.7, 15.9
+// (31).
+constexpr int kFineChunk = 64;
 constexpr int kFineShareKeys = 36;
 
 PKV_HD inline int share_padded(int len) { return (len + kShareSlab - 1) & ~(kShareSlab - 1); }
@@ -161,20 +160,53 @@ struct ShareRule {
   int n_shares;
   int chunk;      // per == 0: keys per chunk, 0 = tokens are not cut
 };
-// total: padded keys of the step; max_shares: warps per kv head (0: the workspace has no room for splits); may_halve:
-// see kFineShareKeys.
-PKV_HD inline ShareRule share_rule(long long total, int max_shares, int forced_chunk, bool may_halve) {
+// What a plan is made for and may use.
+struct PlanLimits {
+  int max_shares;    // warps per kv head, as far as the workspace has room for their partials
+  int max_extra;     // items beyond one per token
+  int kv_heads;
+  int wave_units;    // units that keep the GPU busy
+  int forced_chunk;  // 0: the rules below
+  int shares;        // whether shares are for the kernel of this geometry: not for the SIMT kernel, which gives an item a
+                     // block and wants long ones first (200 tokens of 100-2,000 keys at head_dim 96: 114 us a layer in
+                     // shares, 101 in chunks)
+};
+// Keys per chunk when tokens are cut one by one: the smallest of 256, 512, ... that the workspace has room for, 128
+// where that leaves fewer units than the GPU has workers, 0 when nothing fits.  A token of L keys has at most L / chunk
+// items beyond its first, so the step's total bounds their sum.
+PKV_HD inline int chunk_rule(long long total, int n_tokens, const PlanLimits& lim) {
+  int log2 = 8;
+  while (log2 <= 14 && (total >> log2) > lim.max_extra) ++log2;
+  if (log2 > 14) return 0;
+  const long long items = (total >> 8) + n_tokens / 2;      // of 256 keys, about
+  if (log2 == 8 && (items > n_tokens ? items : n_tokens) * lim.kv_heads < lim.wave_units && (total >> 7) <= lim.max_extra) log2 = 7;
+  return 1 << log2;
+}
+// The rule for plans in token order.  slabs: of the whole step; longest: keys of its longest token; max_shares: as below;
+// fine: see kFineChunk.  A chunk of 128 or 64 keys makes fewer extra items than there may be shares.
+template <typename Int>
+PKV_HD inline ShareRule ordered_share_rule(Int slabs, int longest, int max_shares, bool fine) {
   ShareRule r{0, 0, 0};
   if (max_shares <= 0) return r;
-  if (forced_chunk > 0 && total / forced_chunk <= max_shares) { r.chunk = forced_chunk; return r; }
-  if (total < static_cast<long long>(max_shares) * kMinShareKeys) {
-    r.chunk = may_halve && total < static_cast<long long>(max_shares) * kFineShareKeys ? kMinShareKeys / 2 : kMinShareKeys;
+  const Int most = max_shares;
+  if (slabs < most * (kMinShareKeys / kShareSlab)) {
+    r.chunk = fine && longest > 128 && slabs * kShareSlab < most * kFineShareKeys ? kFineChunk : kMinShareKeys;
     return r;
   }
-  const long long per = ((total + max_shares - 1) / max_shares + kShareSlab - 1) / kShareSlab * kShareSlab;
-  if (per > 0x40000000) return r;
-  r.per = static_cast<int>(per);
-  r.n_shares = static_cast<int>((total + r.per - 1) / r.per);
+  const Int per = (slabs + most - 1) / most;
+  if (per > 0x40000000 / kShareSlab) return r;
+  r.per = static_cast<int>(per) * kShareSlab;
+  r.n_shares = static_cast<int>((slabs + per - 1) / per);
+  return r;
+}
+// total: padded keys of the step.
+PKV_HD inline ShareRule share_rule(long long total, int longest, int n_tokens, const PlanLimits& lim, bool fine) {
+  ShareRule r{0, 0, 0};
+  if (lim.max_shares <= 0) return r;
+  if (lim.forced_chunk > 0 && total / lim.forced_chunk <= lim.max_extra) { r.chunk = lim.forced_chunk; return r; }
+  const bool few = total < static_cast<long long>(lim.max_shares) * kMinShareKeys;
+  if (!few && !lim.shares) { r.chunk = chunk_rule(total, n_tokens, lim); return r; }
+  r = ordered_share_rule<long long>(total / kShareSlab, longest, lim.max_shares, fine);
   return r;
 }
 // Shares a workspace with room for `extra` items beyond one per token takes: the items, their
@@ -197,7 +229,7 @@ struct InlineRuns {
   int min_run;
 };
 
-// Chunk rule of the shared-prefix planner, and of the cluster form's offer.  items_at[j] = sum over tokens of ceil(L_t / (64 << j)).
+// Chunk rule of the shared-prefix planner.  items_at[j] = sum over tokens of ceil(L_t / (64 << j)).
 //   1. take the smallest chunk >= 256 keys whose item count stays within the
 //      budget (one item per token plus `extra_budget`): the most parallelism the
 //      workspace and the target grid allow, without paying a partial per 16 KB;

@@ -113,6 +113,8 @@ struct InlinePlan {
 
   __device__ __forceinline__ void build(const DecodeArgs& a, unsigned char* smem) {
     __shared__ int sm_scan[3][4];
+    __shared__ int sm_step[2];                                             // longest token, whether there is a run for the prefill kernel
+    if (threadIdx.x < 2) sm_step[threadIdx.x] = 0;                         // (the barriers of find() come before its first use)
     s_len = reinterpret_cast<int*>(smem);
     s_tbl = s_len + kInlineTokens;
     s_key = s_tbl + kInlineTokens;
@@ -120,8 +122,8 @@ struct InlinePlan {
     const int n = a.n_tokens;
     TokenRuns<4, kPer> runs;
     runs.find(a.token_pos, a.token_seq, n, s_len, s_tbl, s_key, sm_scan[0]);
-    int len[kPer], tbl[kPer], slabs = 0;
-    bool any_long = false, in_run = false;
+    int len[kPer], tbl[kPer], slabs = 0, longest = 0;
+    bool in_run = false;
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
       len[i] = tbl[i] = 0;
@@ -130,13 +132,15 @@ struct InlinePlan {
         len[i] = max(runs.pos[i], 0) + 1;
         tbl[i] = __ldg(a.table_offset + runs.seq[i]);
         slabs += share_padded(len[i]) / kShareSlab;
-        any_long |= len[i] > kMinShareKeys;
+        longest = max(longest, len[i]);
       }
     }
-    const bool may_halve = __syncthreads_or(any_long) != 0 && __syncthreads_or(in_run) == 0;
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if ((threadIdx.x & 31) == 0) atomicMax(&sm_step[0], longest);
+    if (in_run) sm_step[1] = 1;
     int total;
     int at = block_scan<ScanSum, 4>(slabs, sm_scan[1], &total) - slabs;    // (and the barrier after which the arrays are free)
-    rule = share_rule(static_cast<long long>(total) * kShareSlab, a.inline_max_shares, a.inline_forced_chunk, may_halve);
+    rule = ordered_share_rule(total, sm_step[0], a.inline_max_shares, sm_step[1] == 0);
     int begin[kPer], ns[kPer], sum = 0;                                    // items in the upper half, partials in the lower: < 2^16 each
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {

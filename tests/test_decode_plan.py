@@ -117,3 +117,17 @@ def test_device_plan_is_the_host_plan(pkv, torch_cuda, name):
         assert key(got[2]) == key(want[2])
         if want[3] is not None:
             assert (got[3] == want[3]).all() and (got[2] == want[2]).all()
+
+
+def ragged(n, lo, hi, seed=5):
+    return np.random.default_rng(seed).integers(lo, hi, size=n).astype(np.int32)
+
+
+@pytest.mark.parametrize("qh,kvh,hd", [(32, 1, 64), (16, 4, 96), (8, 2, 256), (40, 2, 128)])
+def test_kernels_that_give_an_item_a_block_get_chunks(pkv, qh, kvh, hd):
+    """Head dims other than 64 and 128 and groups above 16: chunks, full ones first, however many keys there are."""
+    pos = ragged(200, 100, 2000)
+    header, _, items, first = read(host_image(pkv, pos, qh, kvh, hd)[0], pos.size, kvh)
+    assert first is None and header[2] in (128, 256, 512) and (np.diff(items[:, 2]) <= 0).all()
+    check(host_image(pkv, pos, qh, kvh, hd)[0], pos, kvh)
+    assert read(host_image(pkv, pos, 32, 4, 64)[0], pos.size, 4)[3] is not None
