@@ -659,7 +659,7 @@ int persistent_grid() {
 bool tensor_heads(int q_heads, int kv_heads, int head_dim) {
   return (head_dim == 64 || head_dim == 128) && q_heads / kv_heads <= 16;
 }
-PlanLimits plan_limits(int budget, int q_heads, int kv_heads, int head_dim, bool shares) {
+PlanLimits plan_limits(int budget, int q_heads, int kv_heads, int head_dim, bool shares, bool sorted) {
   const int warps = head_dim == 128 ? 8 : 12;             // that the TMA kernel keeps resident on an SM (launch_decode_main)
   PlanLimits lim;
   lim.max_shares = max_shares_for(budget, persistent_sms() * warps / kv_heads);
@@ -668,6 +668,7 @@ PlanLimits plan_limits(int budget, int q_heads, int kv_heads, int head_dim, bool
   lim.wave_units = tuning().wave_ctas;
   lim.forced_chunk = tuning().forced_chunk;
   lim.shares = shares && tensor_heads(q_heads, kv_heads, head_dim) ? 1 : 0;
+  lim.sorted = sorted ? 1 : 0;
   return lim;
 }
 
@@ -691,7 +692,7 @@ int plan_device(const int* token_pos, int n_tokens, int q_heads, int kv_heads, i
   if (budget < 0)
     return fail(PKV_E_WORKSPACE, "pkv_decode_plan_device: workspace of %zu bytes cannot hold the plan for %d tokens", workspace_bytes, n_tokens);
   char* base = static_cast<char*>(workspace);
-  const PlanLimits lim = plan_limits(budget, q_heads, kv_heads, head_dim, shares);
+  const PlanLimits lim = plan_limits(budget, q_heads, kv_heads, head_dim, shares, false);
   const size_t smem = sizeof(int) * static_cast<size_t>(lim.max_shares + 1);
   auto kern = route ? decode_plan_kernel<true> : decode_plan_kernel<false>;
   launch_pdl(kern, dim3(1), dim3(kPlanThreads), smem, stream, token_pos, n_tokens, lim,
@@ -746,7 +747,7 @@ int decode_planned(const pkv_decode_plan* plan, const void* q, const void* kc, c
   a.wait_last = wait_last ? 1 : 0;
   if (inline_min_run > 0) {
     a.inline_min_run = inline_min_run;
-    a.inline_max_shares = plan_limits(budget, a.q_heads, a.kv_heads, a.head_dim, true).max_shares;
+    a.inline_max_shares = plan_limits(budget, a.q_heads, a.kv_heads, a.head_dim, true, false).max_shares;
   }
   if (plan->num_blocks > 0) a.pool_rows = static_cast<unsigned long long>(plan->num_blocks) * block_size;
   if (peers) {
@@ -1013,7 +1014,7 @@ static int plan_host_image(const char* fn, const int* h_token_pos, int n_tokens,
     total += share_padded(h_token_pos[t] + 1);
     max_len = std::max(max_len, h_token_pos[t] + 1);
   }
-  const ShareRule rule = share_rule(total, max_len, n_tokens, plan_limits(budget, q_heads, kv_heads, head_dim, true), false);
+  const ShareRule rule = share_rule(total, max_len, n_tokens, plan_limits(budget, q_heads, kv_heads, head_dim, true, true), false);
   const int chunk = rule.chunk;
   long long n_items = n_tokens;
   if (rule.per > 0) {

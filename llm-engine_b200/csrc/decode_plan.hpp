@@ -127,6 +127,10 @@ constexpr int kShareSlab = 32;
 // Below this many keys a share the tokens are cut one by one into chunks instead (chunk_rule): equal shares would cut
 // short tokens that need no merge at all when left whole.
 constexpr int kMinShareKeys = 128;
+// A plan listed longest first does better with chunks up to this many keys a share, too, if its tokens are mostly
+// shorter than two shares (600 tokens of 60-700 keys, us a layer: 2 kv heads, 180 keys a share, shares 26.5, chunks 25.8;
+// but 8 of 3,000 at 8 kv heads, 162 keys a share, 27.2 and 28.9).
+constexpr int kMinSortedShareKeys = 192;
 // Chunks go down to this length when there are so few keys a share that the longest units decide: four dependent slabs
 // a warp become two.  Only in steps planned on the device that have no prefill chunk, whose kernel the decode units
 // hide behind; small host-planned steps take the cluster form.  Engine decode steps, us a layer with 128- and 64-key chunks: 1 sequence of 333 keys 11.7, 10.2; 6 of 100-900
@@ -170,6 +174,7 @@ struct PlanLimits {
   int shares;        // whether shares are for the kernel of this geometry: not for the SIMT kernel, which gives an item a
                      // block and wants long ones first (200 tokens of 100-2,000 keys at head_dim 96: 114 us a layer in
                      // shares, 101 in chunks)
+  int sorted;        // whether chunks are listed longest first (the host's planner)
 };
 // Keys per chunk when tokens are cut one by one: the smallest of 256, 512, ... that the workspace has room for, 128
 // where that leaves fewer units than the GPU has workers, 0 when nothing fits.  A token of L keys has at most L / chunk
@@ -193,6 +198,8 @@ PKV_HD inline ShareRule ordered_share_rule(Int slabs, int longest, int max_share
     r.chunk = fine && longest > 128 && slabs * kShareSlab < most * kFineShareKeys ? kFineChunk : kMinShareKeys;
     return r;
   }
+  // many tokens, all short: whole (a plan that is sorted leaves more of them whole, see share_rule)
+  if (longest <= 128) { r.chunk = 256; return r; }
   const Int per = (slabs + most - 1) / most;
   if (per > 0x40000000 / kShareSlab) return r;
   r.per = static_cast<int>(per) * kShareSlab;
@@ -207,6 +214,14 @@ PKV_HD inline ShareRule share_rule(long long total, int longest, int n_tokens, c
   const bool few = total < static_cast<long long>(lim.max_shares) * kMinShareKeys;
   if (!few && !lim.shares) { r.chunk = chunk_rule(total, n_tokens, lim); return r; }
   r = ordered_share_rule<long long>(total / kShareSlab, longest, lim.max_shares, fine);
+  if (lim.sorted) {
+    const int chunk = chunk_rule(total, n_tokens, lim);
+    // Enough tokens to fill the GPU, none of them cut: shares would add the merge for nothing (1,000 tokens of 20 to 200
+    // keys, us a layer: 4 kv heads 31.0 in shares, 26.3 whole; 2 kv heads 19.0, 14.6.  In token order they are balanced
+    // better by shares: 34.3 against 36.2).
+    if ((few && longest > 128) || (!few && chunk == 256 && longest <= 256) ||
+        (r.per > 0 && r.per <= kMinSortedShareKeys && total < 2ll * r.per * n_tokens)) r = ShareRule{0, 0, chunk};
+  }
   return r;
 }
 // Shares a workspace with room for `extra` items beyond one per token takes: the items, their

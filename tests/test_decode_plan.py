@@ -131,3 +131,21 @@ def test_kernels_that_give_an_item_a_block_get_chunks(pkv, qh, kvh, hd):
     assert first is None and header[2] in (128, 256, 512) and (np.diff(items[:, 2]) <= 0).all()
     check(host_image(pkv, pos, qh, kvh, hd)[0], pos, kvh)
     assert read(host_image(pkv, pos, 32, 4, 64)[0], pos.size, 4)[3] is not None
+
+
+def test_steps_of_many_short_tokens_are_not_cut(pkv):
+    """Whole tokens fill the GPU: no partials, and so no merge launch; a few longer ones are cut as before."""
+    for kvh, most in ((2, 199), (2, 100), (4, 199), (8, 199)):
+        pos = ragged(1000, 20, most)
+        image, plan = host_image(pkv, pos, 4 * kvh, kvh, 64)
+        header = check(image, pos, kvh)
+        assert header[4] == 0 and plan.reserved == 0 and header[6] == 0
+    assert check(host_image(pkv, ragged(60, 20, 199), 16, 4, 64)[0], ragged(60, 20, 199), 4)[4] > 0
+
+
+def test_shares_are_for_tokens_longer_than_a_share(pkv):
+    """Up to 192 keys a share: chunks where the tokens are mostly shorter than two shares."""
+    short, long = ragged(600, 60, 440), np.full(8, 2999, np.int32)
+    assert check(host_image(pkv, short, 14, 2, 64)[0], short, 2)[6] == 0
+    assert check(host_image(pkv, short, 32, 4, 64)[0], short, 4)[6] > 0        # 370 keys a share
+    assert check(host_image(pkv, long, 32, 8, 128)[0], long, 8)[6] > 0         # 162
