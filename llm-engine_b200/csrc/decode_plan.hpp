@@ -133,11 +133,13 @@ constexpr int kMinShareKeys = 128;
 constexpr int kMinSortedShareKeys = 192;
 // Chunks go down to this length when there are so few keys a share that the longest units decide: four dependent slabs
 // a warp become two.  Only in steps planned on the device that have no prefill chunk, whose kernel the decode units
-// hide behind; small host-planned steps take the cluster form.  Engine decode steps, us a layer with 128- and 64-key chunks: 1 sequence of 333 keys 11.7, 10.2; 6 of 100-900
+// hide behind, and no token of so many chunks that their merge outweighs the shorter units; small host-planned steps take
+// the cluster form.  Engine decode steps, us a layer with 128- and 64-key chunks: 1 sequence of 333 keys 11.7, 10.2; 6 of 100-900
 // (4 kv heads) 12.4, 11.0; 40 of 50-1,000 14.7, 13.3 (15 keys a share); 60 of 60-300 16.3, 15.1 (23); 80 of 60-300 16.7, 15.9
-// (31).
+// (31); and without a caller's plan 1 of 8,000 16.8, 20.6, 8 of 3,000 13.4, 15.5.
 constexpr int kFineChunk = 64;
 constexpr int kFineShareKeys = 36;
+constexpr int kFineMaxKeys = 2048;
 
 PKV_HD inline int share_padded(int len) { return (len + kShareSlab - 1) & ~(kShareSlab - 1); }
 
@@ -195,7 +197,7 @@ PKV_HD inline ShareRule ordered_share_rule(Int slabs, int longest, int max_share
   if (max_shares <= 0) return r;
   const Int most = max_shares;
   if (slabs < most * (kMinShareKeys / kShareSlab)) {
-    r.chunk = fine && longest > 128 && slabs * kShareSlab < most * kFineShareKeys ? kFineChunk : kMinShareKeys;
+    r.chunk = fine && longest > 128 && longest <= kFineMaxKeys && slabs * kShareSlab < most * kFineShareKeys ? kFineChunk : kMinShareKeys;
     return r;
   }
   // many tokens, all short: whole (a plan that is sorted leaves more of them whole, see share_rule)

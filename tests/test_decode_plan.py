@@ -149,3 +149,15 @@ def test_shares_are_for_tokens_longer_than_a_share(pkv):
     assert check(host_image(pkv, short, 14, 2, 64)[0], short, 2)[6] == 0
     assert check(host_image(pkv, short, 32, 4, 64)[0], short, 4)[6] > 0        # 370 keys a share
     assert check(host_image(pkv, long, 32, 8, 128)[0], long, 8)[6] > 0         # 162
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pos,chunk", [([2047], 64), ([2048], 128), ([7999], 128), ([2999] * 8, 128), ([900, 100, 400, 300, 250, 128], 64),
+                                       ([127] * 30, 128)])
+def test_half_chunks_are_for_short_histories(pkv, torch_cuda, pos, chunk):
+    """Chunks of 64 keys: something to merge (a token above 128 keys) and no token of more than 32 of them."""
+    plan = pkv.DecodePlan(len(pos), 14, 2, 64).build_device(torch_cuda.tensor(pos, dtype=torch_cuda.int32, device="cuda"))
+    torch_cuda.cuda.synchronize()
+    image = plan.workspace.cpu().numpy()
+    check(image, pos, 2)
+    assert read(image, len(pos), 2)[0][2] == chunk
