@@ -273,9 +273,11 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
       }
     }
     const int np = ns > 1 ? ns : 0;
-    int tot_items, tot_parts;
-    const int item0 = n_items + block_scan<ScanSum, kPlanThreads / 32>(ns, sm_scan[3], &tot_items) - ns;
-    const int part0 = n_parts + block_scan<ScanSum, kPlanThreads / 32>(np, sm_scan[4], &tot_parts) - np;
+    // both in one scan: 1,024 tokens and the most shares or extra items a workspace holds stay below 2^15
+    int both;
+    const int upto = block_scan<ScanSum, kPlanThreads / 32>((ns << 16) | np, sm_scan[3], &both) - ((ns << 16) | np);
+    const int tot_items = both >> 16, tot_parts = both & 0xffff;
+    const int item0 = n_items + (upto >> 16), part0 = n_parts + (upto & 0xffff);
     if (t < n_tokens) {
       tok_split[t] = TokSplit{part0, ns};
       for (int s = 0; s < ns; ++s) {
