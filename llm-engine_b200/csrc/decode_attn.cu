@@ -545,8 +545,11 @@ int launch_decode_main(const DecodeArgs& a, int grid, cudaStream_t stream, bool*
     // the TMA kernel to one: four times the chain, in time (us a layer with its append, TMA and SIMT: 4 kv heads, 1 x
     // 4,000 keys 275, 227; 8 x 2,000 141, 117; 150 x 50-500 49, 38) and in rounding (1 x 4,000 keys against 64 bits
     // 1.1e-6, 6.8e-7).
+    // 128 dims: as many warps as shares (plan_limits), whatever the planner could tell of the element type; eight on
+    // an SM leave room for one 16 KB stage each.  Six with two stages walk 1,184 equal shares in two rounds (us a layer:
+    // 40 sequences of 200-9,000 keys 182, 124; 100 of 500-1,500 196, 140; 3 of 8,000, in chunks, 59, 65).
     if (tma_path<T>(a) && !a.direct)
-      return a.head_dim == 64 ? launch_tma<T, 64, 1, 1, 2, 4, 3>(a, grid, stream) : launch_tma<T, 128, 1, 1, 2, 3, 2>(a, grid, stream);
+      return a.head_dim == 64 ? launch_tma<T, 64, 1, 1, 2, 4, 3>(a, grid, stream) : launch_tma<T, 128, 1, 1, 1, 4, 2>(a, grid, stream);
   }
   const int dj = (a.head_dim + 31) / 32;
   if (dj <= 2) return launch_simt<T, 2>(a, grid, stream);
