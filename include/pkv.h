@@ -216,7 +216,8 @@ typedef struct pkv_decode_plan {
                      No counterpart in llm-engine. */
   int cluster_wide; /* the same at head_dim 128 (at most 128 keys per warp, two blocks per SM resident); `cluster` is
                        0 there */
-  int pad;
+  int cluster_least; /* fewest blocks per cluster at which no warp gets more keys than that.  fp32 K/V, which holds fewer
+                        clusters at once, may take fewer blocks than `cluster`, but not fewer than two thirds of these */
 } pkv_decode_plan;
 
 size_t pkv_decode_plan_staging_bytes(int n_tokens, int kv_heads);

@@ -453,9 +453,12 @@ int launch_tma_cluster_impl(const DecodeArgs& a, int cs, cudaStream_t stream, bo
 }
 
 template <typename T, int D>
-int launch_tma_cluster_dim(const DecodeArgs& a, int cs, cudaStream_t stream, bool* launched) {
-  // the planner does not know the element type: fp32 takes the largest size its fewer resident blocks hold
-  for (; cs >= 2; --cs) {
+int launch_tma_cluster_dim(const DecodeArgs& a, int cs, int least, cudaStream_t stream, bool* launched) {
+  // the planner does not know the element type: fp32 takes the largest size its fewer resident blocks hold, as long as no
+  // warp gets half as many keys again as the planner allows (us a layer at 128 dims, 15 sequences of 3,000 keys, 8 blocks
+  // offered, 6 the fewest: 30.1 with 4 blocks, 36.2 in the ordinary form; 15 of 200-2,047, 4 offered and the fewest: 35.3 with 2,
+  // 26.6; at 64 dims 50 of 300-4,096, the same: 46.8, 29.7)
+  for (; cs >= std::max((2 * least + 2) / 3, 2); --cs) {
     if (!cluster_size_ok(cs)) continue;
     int st;
     if constexpr (IsF32<T>::value) st = launch_tma_cluster_impl<T, D, false>(a, cs, stream, launched);
@@ -466,9 +469,9 @@ int launch_tma_cluster_dim(const DecodeArgs& a, int cs, cudaStream_t stream, boo
 }
 
 template <typename T>
-int launch_tma_cluster(const DecodeArgs& a, int cs, cudaStream_t stream, bool* launched) {
+int launch_tma_cluster(const DecodeArgs& a, int cs, int least, cudaStream_t stream, bool* launched) {
   *launched = false;
-  return a.head_dim == 128 ? launch_tma_cluster_dim<T, 128>(a, cs, stream, launched) : launch_tma_cluster_dim<T, 64>(a, cs, stream, launched);
+  return a.head_dim == 128 ? launch_tma_cluster_dim<T, 128>(a, cs, least, stream, launched) : launch_tma_cluster_dim<T, 64>(a, cs, least, stream, launched);
 }
 
 template <typename T, int DJ>
@@ -793,7 +796,7 @@ int decode_planned(const pkv_decode_plan* plan, const void* q, const void* kc, c
   const int cluster = a.head_dim == 128 ? plan->cluster_wide : plan->cluster;
   if (cluster >= 2 && !peers && n_shared == 0 && a.group <= 8 && tma_path<T>(a)) {
     bool launched = false;
-    st = launch_tma_cluster<T>(a, cluster, static_cast<cudaStream_t>(stream), &launched);
+    st = launch_tma_cluster<T>(a, cluster, plan->cluster_least, static_cast<cudaStream_t>(stream), &launched);
     if (st != PKV_OK || launched) return st;
   }
   // Work units, or their upper bound when the plan was made on the device.  The TMA kernel turns them into
@@ -1113,7 +1116,10 @@ static int plan_host_image(const char* fn, const int* h_token_pos, int n_tokens,
       int cs = static_cast<int>(std::min<long long>(8, resident / pairs));
       if (tuning().cluster_size >= 2 && tuning().cluster_size < cs) cs = tuning().cluster_size;
       while (cs > 2 && !cluster_size_ok(cs)) --cs;       // 8, 4, 3 or 2 blocks: what the landing areas are sized for
-      if ((max_len + 4 * cs - 1) / (4 * cs) <= max_keys) (head_dim == 64 ? plan->cluster : plan->cluster_wide) = cs;
+      if ((max_len + 4 * cs - 1) / (4 * cs) <= max_keys) {
+        (head_dim == 64 ? plan->cluster : plan->cluster_wide) = cs;
+        plan->cluster_least = (max_len + 4 * max_keys - 1) / (4 * max_keys);
+      }
     }
   }
   return PKV_OK;

@@ -65,3 +65,13 @@ def test_long_histories_without_a_workspace(pkv, orc, torch_cuda, qh, kvh, hd, k
     got = from_device(torch_cuda, orc, case.run_gpu(pkv, torch_cuda, "direct")["out"], "f32")[1].reshape(case.N, qh, hd).astype(np.float64)
     want = in_64_bits(case)
     assert np.linalg.norm(got - want) <= 1.2 * 2.0 ** -24 * np.sqrt(keys / 24) * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("keys,cluster", [(2048, False), (1000, True)])
+def test_clusters_are_not_cut_below_the_rule(pkv, orc, torch_cuda, keys, cluster):
+    """60 (token, kv head) pairs at 128 dims: four blocks each are offered and fp32 can hold two, which 2,048 keys are too
+    many for (256 a warp); those take the ordinary form."""
+    case = make(orc, pkv, 8, 4, 128, 16, [keys - 1] * 14 + [keys // 2], seed=6)
+    before = pkv.lib().pkv_debug_cluster_launches()
+    check_case(case, pkv, torch_cuda, orc, "host_plan")
+    assert pkv.lib().pkv_debug_cluster_launches() == before + (1 if cluster else 0)

@@ -161,3 +161,11 @@ def test_half_chunks_are_for_short_histories(pkv, torch_cuda, pos, chunk):
     image = plan.workspace.cpu().numpy()
     check(image, pos, 2)
     assert read(image, len(pos), 2)[0][2] == chunk
+
+
+@pytest.mark.parametrize("kvh,hd,seqs,keys,size,least", [(2, 64, 50, 4096, 4, 4), (2, 64, 50, 2049, 4, 3), (4, 128, 15, 2048, 4, 4), (4, 128, 15, 700, 4, 2),
+                                                         (2, 64, 1, 300, 8, 1)])
+def test_smallest_cluster_the_rule_allows(pkv, kvh, hd, seqs, keys, size, least):
+    """256 keys a warp (128 at 128 dims), four warps a block: what a launch may shrink the offered clusters to."""
+    plan = host_image(pkv, np.full(seqs, keys - 1, np.int32), 2 * kvh, kvh, hd)[1]
+    assert (plan.cluster if hd == 64 else plan.cluster_wide) == size and plan.cluster_least == least
