@@ -498,7 +498,11 @@ int launch_combine(const DecodeArgs& a, cudaStream_t stream) {
   long long blocks = static_cast<long long>(a.n_tokens) * a.kv_heads;
   const long long cap = static_cast<long long>(persistent_sms()) * 16;
   if (blocks > cap) blocks = cap;
-  launch_pdl(decode_combine_kernel<T, LOG2>, dim3(static_cast<unsigned>(blocks)), dim3(kCombineThreads), 0, stream, a);
+  auto kern = decode_combine_kernel<T, LOG2, false>;
+  if constexpr (LOG2) {
+    if (a.inline_min_run > 0) kern = decode_combine_kernel<T, LOG2, true>;
+  }
+  launch_pdl(kern, dim3(static_cast<unsigned>(blocks)), dim3(kCombineThreads), 0, stream, a);
   return check_launch("decode_combine_kernel");
 }
 

@@ -232,17 +232,23 @@ __device__ __forceinline__ float4 merge_partials4(const DecodeArgs& a, const Tok
   return make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
 }
 
-template <typename T, bool LOG2>
+// INLINE_PLAN: the attention kernel writes the split records (DecodeArgs::inline_min_run).
+template <typename T, bool LOG2, bool INLINE_PLAN>
 __global__ void __launch_bounds__(kCombineThreads) decode_combine_kernel(const DecodeArgs a) {
   pdl_launch_dependents();
   const int D = a.head_dim;
   const int pairs = a.n_tokens * a.kv_heads;
   // The split record of this block's first (token, kv head) is part of the plan, which was complete
-  // before the attention kernel started: fetch it while that kernel is still finishing.
+  // before the attention kernel started: fetch it while that kernel is still finishing.  (Chosen at
+  // run time instead, the two places cost 64 sequences of 256-2,048 keys 0.5 us a layer of 18.6.)
   TokSplit ts_first{0, 0};
-  if (static_cast<int>(blockIdx.x) < pairs && a.inline_min_run == 0) ts_first = a.tok_split[blockIdx.x / a.kv_heads];
+  if constexpr (!INLINE_PLAN) {
+    if (static_cast<int>(blockIdx.x) < pairs) ts_first = a.tok_split[blockIdx.x / a.kv_heads];
+  }
   pdl_wait();  // the attention kernel's partials
-  if (static_cast<int>(blockIdx.x) < pairs && a.inline_min_run > 0) ts_first = a.tok_split[blockIdx.x / a.kv_heads];
+  if constexpr (INLINE_PLAN) {
+    if (static_cast<int>(blockIdx.x) < pairs) ts_first = a.tok_split[blockIdx.x / a.kv_heads];
+  }
   for (int pr = blockIdx.x; pr < pairs; pr += gridDim.x) {
     const int token = pr / a.kv_heads, kvh = pr - token * a.kv_heads;
     const TokSplit ts = pr == static_cast<int>(blockIdx.x) ? ts_first : a.tok_split[token];
