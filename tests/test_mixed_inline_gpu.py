@@ -49,3 +49,11 @@ def test_shares_and_groups(pkv, orc, torch_cuda, qh, kvh):
 @pytest.mark.parametrize("min_run", [1, 2, 3, 1000])
 def test_run_lengths(pkv, orc, torch_cuda, min_run):
     run(pkv, orc, torch_cuda, "bf16", 14, 2, [5, 0, 63, 64, 300, 17, 90], [1, 2, 3, 40, 1, 5, 129], seed=9, min_run=min_run)
+
+
+@pytest.mark.parametrize("qh,kvh", [(14, 2), (4, 4)])
+@pytest.mark.parametrize("runs,length,min_run", [(255, 1, 1), (256, 1, 1), (257, 1, 1), (256, 2, 2), (352, 2, 2)])
+def test_run_counts(pkv, orc, torch_cuda, qh, kvh, runs, length, min_run):
+    """Around the 256 runs a block finds for itself: every run is a chunk for the prefill kernel, of one or two tokens."""
+    ctx = [int(x) for x in np.random.default_rng(runs).integers(0, 150, size=runs)]
+    run(pkv, orc, torch_cuda, "bf16", qh, kvh, ctx, [length] * runs, seed=runs + length, min_run=min_run)
