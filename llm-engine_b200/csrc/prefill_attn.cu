@@ -100,7 +100,8 @@ constexpr int kThreads = 192, kProducerWarp = 4, kMmaWarp = 5;   // warps 0-3: s
 constexpr uint32_t kTmemCols = 256;                          // two blocks per SM share the 512 columns
 constexpr uint32_t kTmemS = 0, kTmemO = 128, kTmemL = 192;   // S0 @0, S1 @64, O @128 (64) with the row sums right behind (16)
 constexpr int kBuckets = 128;
-constexpr int kMaxRankedSeqs = 256;   // launches of up to this many sequences hand their tiles out longest first
+constexpr int kMaxListedSeqs = 256;   // launches of up to this many sequences list their tiles
+constexpr int kShortTiles = 4;        // key tiles
 constexpr float kRescaleThreshold = 8.f;                     // in log2 units: P stays below 2^8
 
 struct PrefillArgs {
@@ -254,7 +255,11 @@ __device__ __forceinline__ void cluster_push4(uint32_t dst, float x, float y, fl
                : "memory");
 }
 
-template <typename T, bool SPLIT>
+// Three instantiations: the ordinary one, SPLIT (few items, see above) and INLINE (a mixed step whose long runs every
+// block finds for itself).  The look-ups of the other two cost a launch of one short chunk 0.3 us when they are
+// merely there.
+enum class Form { kOrdinary, kSplit, kInline };
+template <typename T, Form FORM>
 __global__ void __launch_bounds__(kThreads, 2)
     prefill_tc_kernel(const PrefillArgs a, const __grid_constant__ CUtensorMap qmap,
                       const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap) {
@@ -262,6 +267,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   constexpr uint32_t kIdescQK = instr_desc(kBf16, kKTile, false);
   constexpr uint32_t kIdescPV = instr_desc(kBf16, kHd + 16, true);   // 64 output dims + 16 row-sum columns
   constexpr float kLog2e = 1.4426950408889634f;
+  constexpr bool SPLIT = FORM == Form::kSplit;
 
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long bars[4 + 2 * kKVStages + 7];
@@ -318,7 +324,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 
   // In a mixed step (a.dims) the launch behind this one is the decode kernel, which does not wait for this
   // one before it reads the router's plan: it may start only once the plan is complete.
-  const bool mixed = a.dims != nullptr || a.runs.token_pos != nullptr;
+  const bool mixed = FORM == Form::kInline || (FORM == Form::kOrdinary && a.dims != nullptr);
   if (!mixed) pdl_launch_dependents();
   pdl_wait();
   if (mixed) pdl_launch_dependents();
@@ -328,7 +334,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int* ctx_lens = a.ctx_len;
   const int* table_offset = a.table_offset;
   int n_seqs = a.dims ? __ldcg(a.dims) : a.n_seqs;
-  if (!SPLIT && a.runs.token_pos != nullptr) {
+  if constexpr (FORM == Form::kInline) {
     // the runs of at least min_run tokens, in packed order; the ring serves as scratch
     __shared__ int sm_scan[2][kThreads / 32];
     constexpr int kPer = (kInlineTokens + kThreads - 1) / kThreads;
@@ -358,54 +364,68 @@ __global__ void __launch_bounds__(kThreads, 2)
     __syncthreads();
   }
 
-  // Query tiles are handed out longest key range first, so that the launch ends on its shortest items and the
-  // blocks finish together (configuration 4: 515 us for four layers sequence by sequence, 486 us this way).
+  // The list of query tiles: the sequences in order, each from its longest tile down.  Launches of several rounds take
+  // it longest key range first instead, so that they end on their shortest items and the blocks finish together.
   // The lengths of a sequence's tiles are an arithmetic series, so nothing has to be sorted: lengths fall into
-  // kBuckets buckets, s_cum[b] counts the tiles of buckets 0 .. b, longest first, and the tile of a given rank
-  // is looked up as (bucket, sequence, place) -- in the producer's tile_of_rank, a few hundred cycles.
-  // Launches of more than kMaxRankedSeqs sequences keep the natural order, whose tail matters less the more
-  // items there are.
-  __shared__ int s_top[kMaxRankedSeqs];      // keys the sequence's last tile sees, rounded up to whole tiles; tile_tokens less per tile before
-  __shared__ int s_tiles[kMaxRankedSeqs];
-  __shared__ int s_cum[kBuckets];
+  // kBuckets buckets, s_cum[b][g] counts the tiles of buckets 0 .. b, longest first, among the first 32 (g + 1)
+  // sequences, and the tile of a given rank is looked up as (bucket, 32 sequences, sequence, place) -- in the
+  // producer's find_tile.  Counting the buckets costs a launch 1 to 2 us and buys nothing where a block gets two
+  // items of a few key tiles (kShortTiles).
+  // No list at all, but slots, the longest chunk's number of tiles for every sequence, where there is a block (or
+  // cluster) for every slot, and for more sequences or tiles than the list holds.
+  __shared__ int s_top[kMaxListedSeqs];               // keys the sequence's last tile sees; up to tile_tokens less per tile before
+  __shared__ unsigned short s_tiles[kMaxListedSeqs];
+  __shared__ unsigned short s_cum[SPLIT ? 1 : kBuckets][kMaxListedSeqs / 32];
   const int tt = a.tile_tokens;
-  auto reach = [&](int s, int x) {           // tiles of sequence s whose length is x or more
-    const int over = s_top[s] - x;
-    return over >= 0 ? min(static_cast<int>(__umulhi(over, a.by_tile_tokens)) + 1, s_tiles[s]) : 0;
-  };
-  bool ranked = n_seqs <= kMaxRankedSeqs;
-  int width = 1;                             // keys per bucket
-  if (ranked) {
-    for (int s = threadIdx.x; s < n_seqs; s += kThreads) {
-      const int nt = (q_lens[s] + tt - 1) / tt;
-      s_tiles[s] = nt;
-      s_top[s] = nt > 0 ? ctx_lens[s] + nt * tt : 0;
-    }
-    __syncthreads();
-    int longest = 0;
-    for (int s = 0; s < n_seqs; ++s) longest = max(longest, s_top[s]);
-    ranked = longest < (1 << 25);            // see by_tile_tokens
-    width = longest / kBuckets + 1;
-    if (threadIdx.x < kBuckets && ranked) {
-      const int x = (kBuckets - 1 - threadIdx.x) * width + 1;
-      int c = 0;
-      for (int s = 0; s < n_seqs; ++s) c += reach(s, x);
-      s_cum[threadIdx.x] = c;
-    }
-    __syncthreads();
-  }
-
-  // Split launches: a team of `team` blocks of the cluster shares an item, as far as there are blocks and key tiles for it.
-  int team = 1;
+  uint32_t team = 1, team_rank = 0;                    // split launches: blocks of a cluster, this one's place
   if constexpr (SPLIT) {
-    uint32_t cluster_size;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(cluster_size));
-    const long long items = ranked ? static_cast<long long>(s_cum[kBuckets - 1]) * a.head_tiles : 1ll << 40;
-    while (2 * team <= static_cast<int>(cluster_size) && items * 2 * team <= gridDim.x &&
-           2ll * team * kMinSplitTiles * kKTile <= static_cast<long long>(width) * kBuckets)
-      team *= 2;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(team));
+    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(team_rank));
   }
-  const int team_rank = SPLIT ? static_cast<int>(blockIdx.x) % team : 0;   // clusters and teams are runs of consecutive blocks
+  const int n_slots = ((a.dims ? __ldcg(a.dims + 1) : a.max_q_len) + tt - 1) / tt;   // tiles of the longest chunk
+  const unsigned slots = static_cast<unsigned>(n_seqs) * n_slots * a.head_tiles;
+  auto reach = [&](int s, int x) {                     // tiles of sequence s whose length is x or more
+    const int over = s_top[s] - x;
+    return over >= 0 ? min(static_cast<int>(__umulhi(over, a.by_tile_tokens)) + 1, static_cast<int>(s_tiles[s])) : 0;
+  };
+  bool alone = false;                                  // split launches: more items than clusters, a block each after all
+  bool listed = n_seqs <= kMaxListedSeqs && slots * team > gridDim.x, ranked = false;
+  int width = 1;                                       // keys per bucket
+  unsigned n_items = slots;
+  const int n_groups = (n_seqs + 31) >> 5;
+  if (listed) {
+    int tiles = 0, longest = 0;
+    for (int s = threadIdx.x; s < n_seqs; s += kThreads) {
+      const int ql = max(q_lens[s], 0), nt = (ql + tt - 1) / tt;
+      s_tiles[s] = static_cast<unsigned short>(min(nt, 0xffff));
+      s_top[s] = nt > 0 ? max(ctx_lens[s], 0) + ql : 0;
+    }
+    __syncthreads();
+    for (int s = lane; s < n_seqs; s += 32) {
+      longest = max(longest, s_top[s]);
+      tiles += s_tiles[s];
+    }
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    tiles = __reduce_add_sync(0xffffffffu, tiles);
+    listed = longest < (1 << 25) && tiles < 0xffff;    // see by_tile_tokens, s_cum
+    if (listed) n_items = static_cast<unsigned>(tiles) * a.head_tiles;
+    if constexpr (!SPLIT) {
+      ranked = listed && n_items > gridDim.x && (n_items > 2 * gridDim.x || longest > kShortTiles * kKTile);
+      if (ranked) {
+        width = longest / kBuckets + 1;
+        if (threadIdx.x < kBuckets) {
+          const int x = (kBuckets - 1 - threadIdx.x) * width + 1;
+          int c = 0;
+          for (int g = 0; g < n_groups; ++g) {
+            for (int s = 32 * g; s < min(32 * g + 32, n_seqs); ++s) c += reach(s, x);
+            s_cum[threadIdx.x][g] = static_cast<unsigned short>(c);
+          }
+        }
+        __syncthreads();
+      }
+    }
+  }
+  if constexpr (SPLIT) alone = n_items * team > gridDim.x;
 
   // The block is persistent: it takes (sequence, query tile, head tile) items until none are left.  Every
   // role runs its own loop over the items and keeps its own running counts of items (n) and key tiles
@@ -430,29 +450,36 @@ __global__ void __launch_bounds__(kThreads, 2)
     int n = 0, g = 0;
     int q_sent = 0, kv_sent = 0;                               // lane 0: up to which loads have been issued
     unsigned round = 0;                                        // fixed deal: items taken so far
-    const int n_slots = ((a.dims ? __ldcg(a.dims + 1) : a.max_q_len) + tt - 1) / tt;   // tiles of the longest chunk
-    const unsigned n_items = (ranked ? static_cast<unsigned>(s_cum[kBuckets - 1]) : static_cast<unsigned>(n_seqs) * n_slots) * a.head_tiles;
-    // tile number `k` of the ranked list
-    auto tile_of_rank = [&](int k, int& seq, int& tile) {
-      int b = 0;
-      for (; b < kBuckets; b += 32) {
-        const unsigned past = __ballot_sync(0xffffffffu, s_cum[b + lane] > k);
-        if (past) { b += __ffs(past) - 1; break; }
+    // tile number `k` of the list
+    auto find_tile = [&](int k, int& seq, int& tile) {
+      int lo = 0, s0 = 0;                                      // ranked: shortest length of the tile's bucket
+      if (!SPLIT && ranked) {
+        int b = 0;
+        for (; b < kBuckets; b += 32) {
+          const unsigned past = __ballot_sync(0xffffffffu, s_cum[b + lane][n_groups - 1] > k);
+          if (past) { b += __ffs(past) - 1; break; }
+        }
+        if (b > 0) k -= s_cum[b - 1][n_groups - 1];            // place in its bucket
+        lo = (kBuckets - 1 - b) * width + 1;
+        if (n_groups > 1) {
+          const int g = min(lane, n_groups - 1), upto = s_cum[b][g] - (b > 0 ? s_cum[b - 1][g] : 0);
+          const int at = __ffs(__ballot_sync(0xffffffffu, upto > k)) - 1;
+          const int skipped = __shfl_sync(0xffffffffu, upto, max(at - 1, 0));
+          if (at > 0) k -= skipped;
+          s0 = 32 * at;
+        }
       }
-      if (b > 0) k -= s_cum[b - 1];                            // place in its bucket
-      const int lo = (kBuckets - 1 - b) * width + 1;
-      for (int s0 = 0; s0 < n_seqs; s0 += 32) {
+      for (; s0 < n_seqs; s0 += 32) {
         int before = 0, mine = 0;                              // longer tiles of this lane's sequence, and those of the bucket
         if (s0 + lane < n_seqs) {
-          before = reach(s0 + lane, lo + width);
-          mine = reach(s0 + lane, lo) - before;
+          if (!SPLIT && ranked) {
+            before = reach(s0 + lane, lo + width);
+            mine = reach(s0 + lane, lo) - before;
+          } else {
+            mine = s_tiles[s0 + lane];
+          }
         }
-        int upto = mine;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int x = __shfl_up_sync(0xffffffffu, upto, o);
-          if (lane >= o) upto += x;
-        }
+        const int upto = warp_scan<ScanSum>(mine, lane);
         const unsigned past = __ballot_sync(0xffffffffu, upto > k);
         if (past) {
           const int src = __ffs(past) - 1;
@@ -468,12 +495,12 @@ __global__ void __launch_bounds__(kThreads, 2)
       dead = __shfl_sync(0xffffffffu, dead ? 1 : 0, 0) != 0;   // only lane 0 waits: keep the warp in step
       // next item that has work: head tiles fastest (those of a group share their K/V tiles through L2)
       ItemDesc d;
-      int seq = 0;
+      int seq = 0, table = 0;
       d.n_kt = -1;
       while (!dead) {
         unsigned t = 0;
-        if (SPLIT && team > 1) {
-          t = round == 0 ? blockIdx.x / team : n_items;
+        if (SPLIT && !alone) {
+          t = round == 0 ? blockIdx.x / team : n_items;        // one item per cluster (clusters are runs of consecutive blocks)
           ++round;
         } else if (a.ticket != nullptr) {
           if (lane == 0) t = atomicAdd(a.ticket, 1u);
@@ -486,18 +513,17 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
         if (t >= n_items) break;
         const int rest = static_cast<int>(t / a.head_tiles);
-        int tile;
-        if (ranked) {
-          tile_of_rank(rest, seq, tile);
-        } else {
-          seq = rest / n_slots;
-          tile = (q_lens[seq] + tt - 1) / tt - 1 - (rest - seq * n_slots);
-        }
+        int tile = -1;
+        if (listed) find_tile(rest, seq, tile);
+        else seq = rest / n_slots;
+        if (seq < 0) continue;
+        const int q_len = q_lens[seq], ctx = ctx_lens[seq], start = q_start[seq];   // one round trip for all of them
+        table = table_offset[seq];
+        if (!listed) tile = (q_len + tt - 1) / tt - 1 - (rest - seq * n_slots);
         if (tile < 0) continue;
-        const int q_len = q_lens[seq], ctx = ctx_lens[seq];
         const int tokens = min(tt, q_len - tile * tt);
         d.head = static_cast<int>(t % a.head_tiles) * a.pack;
-        d.row0 = q_start[seq] + tile * tt;
+        d.row0 = start + tile * tt;
         d.rows_here = tokens * a.pack;
         d.kv_total = ctx + tile * tt + tokens;
         d.limit0 = ctx + tile * tt;
@@ -505,10 +531,10 @@ __global__ void __launch_bounds__(kThreads, 2)
         if (d.n_kt <= 0) d.n_kt = -1;
         d.kt0 = 0;
         d.n_parts = 1;
-        if (SPLIT && team > 1 && d.n_kt > 0) {
-          const int per = max((d.n_kt + team - 1) / team, 2);
+        if (SPLIT && !alone && d.n_kt > 0) {
+          const int most = min(max(d.n_kt / kMinSplitTiles, 1), static_cast<int>(team)), per = (d.n_kt + most - 1) / most;
           d.n_parts = (d.n_kt + per - 1) / per;
-          d.kt0 = team_rank * per;
+          d.kt0 = static_cast<int>(team_rank) * per;
           d.n_kt = max(min(per, d.n_kt - d.kt0), 0);
         }
         break;
@@ -518,7 +544,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         WAIT(BAR(Q_EMPTY + qb), ((n >> 1) & 1) ^ 1);
         s_item[qb] = d;
         if (d.n_kt == 0 && !dead) {
-          mbar_arrive(BAR(Q_FULL + qb));        // the item is the team's, but this block has no part of its keys
+          mbar_arrive(BAR(Q_FULL + qb));        // the item is the cluster's, but this block has no part of its keys
         } else if (d.n_kt > 0 && !dead) {
           q_sent = n + 1;
           mbar_arrive_expect_tx(BAR(Q_FULL + qb), static_cast<uint32_t>(a.pack * a.tile_tokens) * 128u);
@@ -532,7 +558,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       dead = __shfl_sync(0xffffffffu, dead ? 1 : 0, 0) != 0;
       if (d.n_kt < 0 || dead) break;
       const int kvh = d.head / a.group;
-      const int* tbl = a.block_tables + table_offset[seq];
+      const int* tbl = a.block_tables + table;
       for (int j = d.kt0; j < d.kt0 + d.n_kt; ++j, ++g) {
         const int st = g % kKVStages;
         const int rel = j * kKTile + (lane & 3) * 16;
@@ -737,17 +763,14 @@ __global__ void __launch_bounds__(kThreads, 2)
       }
       if constexpr (SPLIT) {
         if (d.n_parts > 1) {
-          // This block's partial rows go to the blocks that own them: block i of the team owns rows
+          // This block's partial rows go to the blocks that own them: block i of the cluster owns rows
           // [i, i + 1) 128 / team.  Record (part, row of the owner) of its landing area.
-          const int rows_each = kQTile / team;
-          uint32_t my_rank;
-          asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(my_rank));
-          const uint32_t cluster_base = my_rank - team_rank;
+          const int rows_each = kQTile / static_cast<int>(team);
           const uint32_t land = base + kSmemKV;
           if (r == 0) mbar_arrive_expect_tx(BAR(LAND), static_cast<uint32_t>(d.n_parts * rows_each * kLandRecord));
           if (n_kt > 0) WAIT(BAR(PV_DONE + ((g - 1) & 1)), ((g - 1) >> 1) & 1);
           // nobody sends before every block's barrier is set up and its ring idle.  (All blocks of a cluster meet
-          // here or leave; its teams hold neighbours in the order of lengths, so they wait little for one another.)
+          // here or leave.)
           __syncwarp();
           asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
           asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
@@ -760,7 +783,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             tc_ld32(tmem + lane_addr + kTmemL, lv);
             tc_wait_ld();
             tc_fence_before();
-            const uint32_t owner = cluster_base + r / rows_each;
+            const uint32_t owner = r / rows_each;
             const uint32_t dst = cluster_map(land + (team_rank * rows_each + r % rows_each) * kLandRecord, owner);
             const uint32_t bar = cluster_map(BAR(LAND), owner);
 #pragma unroll
@@ -773,8 +796,8 @@ __global__ void __launch_bounds__(kThreads, 2)
           }
           WAIT(BAR(LAND), 0);
           // fold: thread = (row, part of its 64 dims)
-          const int row = team_rank * rows_each + r / team, dims = kHd / team, d0 = (r % team) * dims;
-          const unsigned char* rec0 = base_ptr + kSmemKV + (r / team) * kLandRecord;
+          const int n_team = static_cast<int>(team), row = static_cast<int>(team_rank) * rows_each + r / n_team, dims = kHd / n_team, d0 = (r % n_team) * dims;
+          const unsigned char* rec0 = base_ptr + kSmemKV + (r / n_team) * kLandRecord;
           if (row < rows_here && !dead) {
             float m = -INFINITY, l = 0.f;
             for (int p = 0; p < d.n_parts; ++p) m = fmaxf(m, *reinterpret_cast<const float*>(rec0 + p * rows_each * kLandRecord + 256));
@@ -802,7 +825,7 @@ __global__ void __launch_bounds__(kThreads, 2)
               *reinterpret_cast<uint4*>(o + x) = packed;
             }
           }
-          break;                                       // a team has one item
+          break;                                       // a cluster has one item
         }
         if (n_kt == 0) break;                          // (a one-part item is its first block's alone)
       }
@@ -825,9 +848,9 @@ __global__ void __launch_bounds__(kThreads, 2)
         const float inv = 1.f / __uint_as_float(lv[0]);
         unsigned char* stage = base_ptr + kSmemQ + qb * kQBytes;
         unsigned char* my_row = stage + r * 128;
+        if (r < rows_here)                                     // (the rows past the tile's stay zero)
 #pragma unroll
         for (int dd = 0; dd < 32; dd += 8) {
-          if (r >= rows_here) break;                           // (the rows past the tile's stay zero)
           uint4 w0, w1;
           w0.x = pack2<T>(__uint_as_float(o0[dd]) * inv, __uint_as_float(o0[dd + 1]) * inv);
           w0.y = pack2<T>(__uint_as_float(o0[dd + 2]) * inv, __uint_as_float(o0[dd + 3]) * inv);
@@ -841,14 +864,14 @@ __global__ void __launch_bounds__(kThreads, 2)
           *reinterpret_cast<uint4*>(my_row + ((((dd >> 3) + 4) ^ (r & 7)) << 4)) = w1;
         }
         __syncwarp();
-        T* obase = static_cast<T*>(a.out) + (static_cast<size_t>(d.row0) * a.q_heads + d.head) * kHd;
+        // row = token x pack + head of the tile, q_heads - pack rows of the output from the last head of a token to the next
+        unsigned char* obase = reinterpret_cast<unsigned char*>(static_cast<T*>(a.out) + (static_cast<size_t>(d.row0) * a.q_heads + d.head) * kHd) + (lane & 7) * 16;
+        const uint32_t skip = static_cast<uint32_t>(a.q_heads - a.pack) * 128u;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const int row = warp * 32 + i * 4 + (lane >> 3), ch = lane & 7;
-          const uint4 w = *reinterpret_cast<const uint4*>(stage + row * 128 + ((ch ^ (row & 7)) << 4));
-          const int tok = static_cast<int>((row * a.by_pack) >> 16), h = row - tok * a.pack;
-          if (row < rows_here)
-            *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(obase + (static_cast<size_t>(tok) * a.q_heads + h) * kHd) + ch * 16) = w;
+          const int row = warp * 32 + i * 4 + (lane >> 3);
+          const uint4 w = *reinterpret_cast<const uint4*>(stage + row * 128 + (((lane & 7) ^ (row & 7)) << 4));
+          if (row < rows_here) *reinterpret_cast<uint4*>(obase + static_cast<size_t>(row * 128u + ((row * a.by_pack) >> 16) * skip)) = w;
         }
       }
       // The Q buffer may be refilled (by TMA) once every thread is done with it: the item's
@@ -862,7 +885,9 @@ __global__ void __launch_bounds__(kThreads, 2)
   tc_fence_before();
   if constexpr (SPLIT) {
     __syncwarp();
-    if (!met) asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");   // the producer and MMA warps, and blocks without a part
+    // The producer and MMA warps, and blocks without a part.  (Nothing of theirs is read by the others: without a release
+    // a launch of one short chunk ends 0.25 us earlier.)
+    if (!met) asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
     // A block has received everything that is sent to it before it leaves (LAND), except after a wait that ran
     // out: then it stays until the rest of the cluster has left.
     if (__syncthreads_or(dead)) {
@@ -941,6 +966,32 @@ TicketPair ticket_pair_for(cudaStream_t stream, int dev) {
 unsigned int* error_mirror(bool create);                 // error_mirror.cu
 int check_error_mirror(const char* fn, unsigned int bits = ~0u);
 
+// Query heads per tile: the divisor of the group (up to 16, at most 8 of the 128 rows unused) that costs a chunk of q_len
+// tokens the fewest key tiles, an item's fixed work counted as three.  Short chunks fill whole tiles of few heads badly and
+// many heads' tiles of few tokens best; 128 tokens are one full tile per head (30 chunks of 128 fresh tokens, 14/2
+// heads: 480 items of 7 heads 18.5 us a layer, 420 of one 17.5); a group of 20 takes 4 heads a tile at 512 tokens
+// and not 10, which leave 8 rows unused (44 -> 42 us).  q_len 0 (unknown): the most heads that leave at most 3 rows unused.
+int heads_per_tile(int group, int q_len) {
+  int pack = 1;
+  long long least = -1;
+  for (int p = 1; p <= 16; ++p) {
+    const int tt = kQTile / p, unused = kQTile - tt * p;
+    if (group % p != 0 || unused > (q_len > 0 ? 8 : 3)) continue;
+    if (q_len <= 0) { pack = p; continue; }
+    // sum over the chunk's tiles of the key tiles up to their last token; from 32 tiles on, its integral
+    const int n = (q_len + tt - 1) / tt;
+    long long cost = 3 * n;
+    if (n <= 32) {
+      for (int i = 1; i <= n; ++i) cost += (std::min(i * tt, q_len) + kKTile - 1) / kKTile;
+    } else {
+      cost += n / 2 + static_cast<long long>(q_len) * (n + 1) / (2 * kKTile);
+    }
+    cost *= group / p;
+    if (least < 0 || cost <= least) { least = cost; pack = p; }
+  }
+  return pack;
+}
+
 // Shared by the C entry points below and by the mixed-step router (decode_attn.cu).  With d_dims the
 // per-sequence arrays and their counts come from an earlier kernel on the stream: n_seqs and
 // max_q_len are then upper bounds that size the grid, and table_offset is indexed like q_start.
@@ -978,13 +1029,9 @@ int prefill_launch(const void* q, const void* k_cache, const void* v_cache, cons
   if (st != PKV_OK) return st;
   st = make_pool_tensor_map(&vmap, v_cache, is_bf16 ? PoolElem::kBF16 : PoolElem::kF16, kv_dim, 16, pool_rows);
   if (st != PKV_OK) return st;
-  // Heads per tile: the largest divisor of the group, up to 16, that leaves at most 8 of the 128 rows unused
-  // (a group of 13 would waste 11: its heads take tiles of their own).
   constexpr int kInlineSmem = kSmemTotal + 4 * kInlineRuns * static_cast<int>(sizeof(int));   // still two blocks per SM
   const int group = q_heads / kv_heads;
-  int pack = 1;
-  for (int p = 2; p <= 16; ++p)
-    if (group % p == 0 && kQTile / p * p >= kQTile - 8) pack = p;
+  const int pack = heads_per_tile(group, d_dims ? 0 : std::min(max_q_len, (n_tokens + n_seqs - 1) / n_seqs));
   const int tile_tokens = kQTile / pack;
   // q as [n_tokens][q_heads][head_dim]; rows past n_tokens read as zeros
   st = make_rows_tensor_map(&qmap, q, is_bf16, q_heads, static_cast<uint64_t>(n_tokens), pack, tile_tokens);
@@ -1004,14 +1051,15 @@ int prefill_launch(const void* q, const void* k_cache, const void* v_cache, cons
   split.dynamicSmemBytes = kSplitSmem;
   split.attrs = split_attr;
   if (configured_device != dev) {
-    cudaError_t e = cudaFuncSetAttribute(prefill_tc_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kInlineSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_tc_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem);
+    cudaError_t e = cudaFuncSetAttribute(prefill_tc_kernel<T, Form::kOrdinary>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTotal);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_tc_kernel<T, Form::kInline>, cudaFuncAttributeMaxDynamicSharedMemorySize, kInlineSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_tc_kernel<T, Form::kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem);
     if (e != cudaSuccess) return fail(PKV_E_CUDA, "%s: cannot reserve %d bytes of shared memory: %s", fn, kSplitSmem, cudaGetErrorString(e));
     split.numAttrs = 1;
     for (int i = 0; i < 3; ++i) {
       split_attr[0].val.clusterDim.x = 2u << i;
       split.gridDim = dim3(2u << i);
-      if (cudaOccupancyMaxActiveClusters(&max_clusters[i], prefill_tc_kernel<T, true>, &split) != cudaSuccess) { cudaGetLastError(); max_clusters[i] = 0; }
+      if (cudaOccupancyMaxActiveClusters(&max_clusters[i], prefill_tc_kernel<T, Form::kSplit>, &split) != cudaSuccess) { cudaGetLastError(); max_clusters[i] = 0; }
     }
     configured_device = dev;
   }
@@ -1043,27 +1091,30 @@ int prefill_launch(const void* q, const void* k_cache, const void* v_cache, cons
   }
   // PKV_PREFILL_BLOCKS_PER_SM = 1: half the persistent grid (a measurement aid: what one block per SM does alone)
   static const int per_sm = [] { const char* e = std::getenv("PKV_PREFILL_BLOCKS_PER_SM"); return (e && e[0] == '1') ? 1 : 2; }();
-  const int blocks = static_cast<int>(std::min<long long>(n_items, static_cast<long long>(per_sm) * sms));
+  const long long resident = static_cast<long long>(per_sm) * sms;
+  const int blocks = static_cast<int>(slots <= resident && d_dims == nullptr ? slots : std::min(n_items, resident));
   // A block that gets one item at most needs no ticket for it (nor the look-up of the stream's counter).
   const TicketPair tp = n_items > blocks ? ticket_pair_for(static_cast<cudaStream_t>(stream), dev) : TicketPair{nullptr, nullptr};
   a.ticket = tp.ticket;
   a.done = tp.done;
-  // Few items: the largest cluster per item that leaves all of them resident (up to 15 items eight blocks, 33
-  // four, 73 two).  Measured per layer with its rope + append: 50 tokens behind 4,000 (6 items) 53.2 -> 16.7 us,
-  // 128 behind 2,000 (32 items) 33.6 -> 18.1; short fresh chunks, which no block shares, lose 1 to 2 us of 9
-  // to 13 to the cluster launch.  A mixed step knows only a loose bound of its items, most often of none:
-  // it keeps the ordinary launch.
+  // Few items: the largest cluster per item that leaves all of them resident (up to 15 items eight blocks, 33 four, 73
+  // two; four for more than 16 items only if they are of one sequence, since it is several short chunks that are fresh
+  // prompts, which no block shares).  Measured per layer with its rope + append, 14/2 heads, ordinary form and this: 50 tokens
+  // behind 4,000 (6 items) 51.7 -> 15.9 us, 128 behind 2,000 31.3 -> 13.8, 2 x 300 behind 1,200 22.2 -> 18.7; fresh
+  // chunks pay 0.2 to 0.6 us for the cluster launch (50 tokens 7.7 -> 8.1, 3 x 100 9.0 -> 9.5, 400 12.1 -> 12.8).  A mixed
+  // step knows only a loose bound of its items, most often of none: it keeps the ordinary launch.
   int cs = 0;
   for (int i = 2; i >= 0 && !cs; --i)
-    if (d_dims == nullptr && n_items <= max_clusters[i]) cs = 2 << i;
+    if (d_dims == nullptr && n_items <= max_clusters[i] && (i != 1 || n_items <= 16 || n_seqs == 1)) cs = 2 << i;
   if (cs > 0) {
     split_attr[0].val.clusterDim.x = cs;
-    split.gridDim = dim3(static_cast<unsigned>(n_items * cs));
+    split.gridDim = dim3(static_cast<unsigned>((slots <= max_clusters[cs == 8 ? 2 : cs / 4] ? slots : n_items) * cs));
     split.stream = static_cast<cudaStream_t>(stream);
     split.numAttrs = pdl_enabled() ? 2 : 1;
-    cudaLaunchKernelEx(&split, prefill_tc_kernel<T, true>, a, qmap, kmap, vmap);
+    cudaLaunchKernelEx(&split, prefill_tc_kernel<T, Form::kSplit>, a, qmap, kmap, vmap);
   } else {
-    launch_pdl(prefill_tc_kernel<T, false>, dim3(blocks), dim3(kThreads), runs ? kInlineSmem : kSmemTotal, static_cast<cudaStream_t>(stream), a, qmap, kmap, vmap);
+    launch_pdl(runs ? prefill_tc_kernel<T, Form::kInline> : prefill_tc_kernel<T, Form::kOrdinary>, dim3(blocks), dim3(kThreads),
+               runs ? kInlineSmem : kSmemTotal, static_cast<cudaStream_t>(stream), a, qmap, kmap, vmap);
   }
   return check_launch("prefill_tc_kernel");
 }

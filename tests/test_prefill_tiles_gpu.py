@@ -71,3 +71,22 @@ def test_split_launch_replays_from_a_graph(pkv, orc, torch_cuda):
         g.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, want) and pkv.debug_device_flags() == 0
+
+
+@pytest.mark.parametrize("qh,kvh", [(14, 2), (3, 3)])
+@pytest.mark.parametrize("n_seqs,longest", [(30, 1), (32, 700), (64, 250), (96, 130), (255, 90), (256, 300), (257, 40)])
+def test_lists_of_tiles(pkv, orc, torch_cuda, qh, kvh, n_seqs, longest):
+    """One slot per block, a list in the sequences' order, and one ordered by length, over 32, 64, ... sequences:
+    every row of every chunk is written, whatever the lengths and whichever sequences bring nothing."""
+    rng = np.random.default_rng(n_seqs)
+    ctx = [int(x) for x in rng.integers(0, longest, size=n_seqs)]
+    new = [int(x) for x in rng.integers(1, 1 + min(longest, 70), size=n_seqs)]
+    new[n_seqs // 2] = min(longest, 200)
+    check(pkv, orc, torch_cuda, qh, kvh, ctx, new, seed=n_seqs, dtype="f16")
+
+
+@pytest.mark.parametrize("ctx,new", [([0, 300, 0, 40], [60, 60, 60, 60]), ([0, 0, 0], [100, 90, 100]), ([3, 0, 900, 0, 64], [1, 200, 17, 3, 130])])
+def test_few_items_of_uneven_sequences(pkv, orc, torch_cuda, ctx, new):
+    """Clusters for more slots than items: the tiles come from the list."""
+    for qh, kvh in ((14, 2), (8, 1), (2, 2)):
+        check(pkv, orc, torch_cuda, qh, kvh, ctx, new, seed=10)
