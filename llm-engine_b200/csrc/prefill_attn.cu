@@ -48,7 +48,7 @@
 // Launches with few items leave most of the chip idle and take as long as their longest item's chain of
 // key tiles.  They run as one cluster of two, four or eight blocks per item instead (SPLIT), as many as
 // are resident together: each block takes a contiguous part of the item's key tiles (at least
-// kMinSplitTiles; the longest item of the launch decides how many blocks share), and the partial rows
+// kMinSplitTiles, so short items are left to one of them), and the partial rows
 // (64 sums, maximum, sum) are sent to the block that owns the row's share of the output with st.async
 // into its K/V ring, idle by then, where they are folded.
 //
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     return over >= 0 ? min(static_cast<int>(__umulhi(over, a.by_tile_tokens)) + 1, static_cast<int>(s_tiles[s])) : 0;
   };
   bool alone = false;                                  // split launches: more items than clusters, a block each after all
-  bool listed = n_seqs <= kMaxListedSeqs && slots * team > gridDim.x, ranked = false;
+  bool listed = n_seqs <= kMaxListedSeqs && static_cast<unsigned long long>(slots) * team > gridDim.x, ranked = false;
   int width = 1;                                       // keys per bucket
   unsigned n_items = slots;
   const int n_groups = (n_seqs + 31) >> 5;
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       }
     }
   }
-  if constexpr (SPLIT) alone = n_items * team > gridDim.x;
+  if constexpr (SPLIT) alone = static_cast<unsigned long long>(n_items) * team > gridDim.x;
 
   // The block is persistent: it takes (sequence, query tile, head tile) items until none are left.  Every
   // role runs its own loop over the items and keeps its own running counts of items (n) and key tiles

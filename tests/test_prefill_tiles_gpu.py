@@ -90,3 +90,20 @@ def test_few_items_of_uneven_sequences(pkv, orc, torch_cuda, ctx, new):
     """Clusters for more slots than items: the tiles come from the list."""
     for qh, kvh in ((14, 2), (8, 1), (2, 2)):
         check(pkv, orc, torch_cuda, qh, kvh, ctx, new, seed=10)
+
+
+def test_a_generous_longest_chunk(pkv, orc, torch_cuda):
+    """max_q_len is an upper bound: 2^30 makes 2^29 slots, which eight blocks each would count past 32 bits."""
+    torch = torch_cuda
+    ctx, new = [0, 3, 64, 700, 0, 90, 5, 17], [1, 5, 2, 1, 3, 1, 4, 1]
+    case = make_case(orc, pkv, "bf16", 8, 1, 16, ctx, new, seed=11)
+    _, _, want = case.expected(orc, threads=4)
+    d = run_prefill(pkv, torch, case)
+    i32 = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.int32)).cuda()
+    d["out"].fill_(float("nan"))
+    pkv.launch_attention_prefill(d["q"], d["kc"], d["vc"], d["block_tables"], d["table_offset"], i32(np.cumsum(new) - new), i32(new), i32(ctx),
+                                 d["out"], case.N, len(new), 1 << 30, 8, 1, 64, 16, case.nb, case.scale)
+    torch.cuda.synchronize()
+    _, got = from_device(torch, orc, d["out"], "bf16")
+    e_ref, e_row = rel_errors(got.reshape(-1, 64), want.reshape(-1, 64))
+    assert e_ref <= TOL["bf16"] and e_row <= TOL["bf16"] and pkv.debug_device_flags() == 0
