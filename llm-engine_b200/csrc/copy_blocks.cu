@@ -151,7 +151,14 @@ int copy_impl(TwoPools two, void* const* pools, int n_pools, bool pools_aligned,
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (block_bytes % 16 == 0 && pools_aligned) {
     const unsigned long long pieces = (block_bytes + kBulkBytes - 1) / kBulkBytes, tasks = pieces * n_pairs * n_pools;
-    const unsigned blocks = static_cast<unsigned>(std::min<unsigned long long>(tasks, 148 * kBulkBlocksPerSm));
+    static thread_local int sms = 0;
+    if (!sms) {
+      int dev = 0;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      if (sms <= 0) sms = 148;
+    }
+    const unsigned blocks = static_cast<unsigned>(std::min<unsigned long long>(tasks, static_cast<unsigned long long>(sms) * kBulkBlocksPerSm));
     auto kern = pools ? copy_blocks_bulk_kernel<true> : copy_blocks_bulk_kernel<false>;
     launch_pdl(kern, dim3(blocks), dim3(32), kBulkStages * kBulkBytes, s, two, pools, pairs, n_pairs, block_bytes, pieces, tasks,
                error_mirror(true));

@@ -97,7 +97,7 @@ struct RouteArgs {
   int* q_len;
   int* ctx_len;
   int* tbl_off;
-  int* dims;        // [4] out: runs, tokens of the longest, tokens of none
+  int* dims;        // [2] out: runs, tokens of the longest
 };
 
 // One block: all of it is latency (a step of 600 tokens reads 5 KB), so a step of up to kPlanThreads
@@ -114,12 +114,12 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
   __shared__ int sm_scan[8][kPlanThreads / 32];
   __shared__ int sm_len[kPlanThreads];                    // run lengths of a step of up to kPlanThreads tokens
   __shared__ int sm_start[kPlanThreads + 1];              // ... and whether a run starts at a token
-  __shared__ int sm_misc[4];                              // long runs, longest of them, tokens of none, longest token
+  __shared__ int sm_misc[3];                              // long runs, longest of them, longest token
   const int tid = threadIdx.x;
   const bool small = n_tokens <= kPlanThreads;
   // the next launch on the stream is the prefill kernel, which waits for this one before it reads anything
   if constexpr (ROUTE) pdl_launch_dependents();
-  if (tid < 4) sm_misc[tid] = 0;
+  if (tid < 3) sm_misc[tid] = 0;
   for (int i = tid; i <= lim.max_shares; i += kPlanThreads) sm_first[i] = 0x7fffffff;
   if (tid == 0) sm_start[n_tokens < kPlanThreads ? n_tokens : kPlanThreads] = 1;
   __syncthreads();
@@ -161,8 +161,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
         r.tbl_off[i] = r.table_offset[seq];
         atomicMax(&sm_misc[1], len);
       }
-      const int n_dec = __syncthreads_count(my_len > 0);
-      if (tid == 0) { sm_misc[0] = tot; sm_misc[2] = n_dec; }
+      if (tid == 0) sm_misc[0] = tot;
     } else {
       // 1. running maximum of the start indices = first token of each token's run
       int carry = -1;
@@ -205,8 +204,8 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
           atomicMax(&sm_misc[1], len);
         }
         runs += tot;
-        const int n_dec = __syncthreads_count(eff > 0);
-        if (tid == 0) { sm_misc[0] = runs; sm_misc[2] += n_dec; }
+        __syncthreads();                                     // the scans' words, before the next round
+        if (tid == 0) sm_misc[0] = runs;
       }
     }
   } else {
@@ -224,7 +223,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
   int longest = my_len;
   if (small) {
     longest = __reduce_max_sync(0xffffffffu, longest);
-    if ((tid & 31) == 0) atomicMax(&sm_misc[3], longest);
+    if ((tid & 31) == 0) atomicMax(&sm_misc[2], longest);
     int tot;
     const int p = share_padded(my_len) / kShareSlab;       // scanned in slabs: 32 bits hold 2^36 keys
     my_begin = static_cast<long long>(block_scan<ScanSum, kPlanThreads / 32>(p, sm_scan[2], &tot) - p) * kShareSlab;
@@ -242,12 +241,12 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
     __shared__ long long sm_tot[kPlanThreads / 32];
     if ((tid & 31) == 0) {
       sm_tot[tid >> 5] = loc;
-      atomicMax(&sm_misc[3], longest);
+      atomicMax(&sm_misc[2], longest);
     }
     __syncthreads();
     for (int w = 0; w < kPlanThreads / 32; ++w) total += sm_tot[w];
   }
-  const ShareRule rule = share_rule(total, sm_misc[3], n_tokens, lim, !ROUTE || sm_misc[0] == 0);
+  const ShareRule rule = share_rule(total, sm_misc[2], n_tokens, lim, !ROUTE || sm_misc[0] == 0);
 
   int n_items = 0, n_parts = 0;
   long long carry_begin = 0;
@@ -317,8 +316,6 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const int* __
     if (tid == 0) {
       r.dims[0] = sm_misc[0];
       r.dims[1] = sm_misc[1];
-      r.dims[2] = sm_misc[2];
-      r.dims[3] = 0;
     }
   }
 }
@@ -807,7 +804,7 @@ int decode_planned(const pkv_decode_plan* plan, const void* q, const void* kc, c
   // resident blocks of warps itself; the kernels that give a unit a whole block (and stride over the rest) are
   // capped at four blocks per SM when the count is only a bound.  (Capping the UNITS at that number, whatever
   // the kernel, leaves a device-made plan on 148 of the 444 resident blocks of the TMA kernel: a step of 22
-  // layers over 128 sequences of 650 keys, 32 query / 4 kv heads, took 809 us that way and takes 432.)
+  // layers over 128 sequences of 650 keys, 32 query / 4 kv heads, took 809 us that way and 432 on all of them.)
   long long blocks = static_cast<long long>(plan->n_items) * plan->kv_heads;
   if (!plan->exact && !tma_path<T>(a) && blocks > persistent_grid()) blocks = persistent_grid();
   if (blocks > 0x7fffffffll) blocks = 0x7fffffffll;

@@ -97,7 +97,7 @@ struct UnitCursor { int u, item, end, kvh; };
 // A step's plan in shared memory, built by every block for itself (DecodeArgs::inline_min_run): the same cuts
 // as decode_plan_kernel makes, found through the tokens instead of a list.  A planner launch in front of the
 // attention kernel cost 4.6 us a layer, and the four dependent look-ups from its list to a unit's first load
-// 2 to 3 more; this costs every block about 1.5.
+// 2 to 3 more; this takes every block about 4 (16 us a layer without the planner launch, 19 with it, 48 sequences).
 struct InlinePlan {
   static constexpr int kPer = (kInlineTokens + 127) / 128;
   static constexpr int kBytes = kInlineTokens * (3 * 4 + 2);
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_BLOCKS)
   // Units of this warp: one item each (item, kv head) dealt round-robin, or, when the plan has shares, all the
   // items of a (share, kv head) one after the other.  The issue side and the math side walk the same list,
   // each with a cursor of its own.
-  static_assert(!INLINE_PLAN || (TOK == 1 && !FUSED_APPEND && !CLUSTER && !F32 && WARPS == 4), "mixed steps only");
+  static_assert(!INLINE_PLAN || (TOK == 1 && !FUSED_APPEND && !CLUSTER && !F32 && WARPS == 4), "16-bit calls without a plan of the caller's");
   InlinePlan ip = {};
   if constexpr (INLINE_PLAN) {
     if (!waited) {       // not behind a prefill launch that has waited for the index arrays' producers

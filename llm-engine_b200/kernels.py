@@ -69,7 +69,7 @@ def launch_store_kv(k, v, slots, k_cache, v_cache, n_tokens: int, kv_dim: int, s
     """k_cache[slots[t]] = k[t], v_cache[slots[t]] = v[t] (engine::launch_store_kv)."""
     fn, call = _fn("pkv_append_", k_cache)
     st = call(_ptr(k), _ptr(v), _ptr(slots), _ptr(k_cache), _ptr(v_cache), n_tokens, kv_dim,
-                                 _stream(stream))
+              _stream(stream))
     _lib.check(fn, st)
 
 
@@ -79,8 +79,8 @@ def launch_rope_store_kv(q, k, v, positions, cos_table, sin_table, slots, k_cach
     written to their slots (cos/sin: fp32 tables [max_positions][head_dim/2])."""
     fn, call = _fn("pkv_rope_append_", k_cache)
     st = call(_ptr(q), _ptr(k), _ptr(v), _ptr(positions), _ptr(cos_table), _ptr(sin_table),
-                                 _ptr(slots), _ptr(k_cache), _ptr(v_cache), n_tokens, q_heads, kv_heads, head_dim,
-                                 _stream(stream))
+              _ptr(slots), _ptr(k_cache), _ptr(v_cache), n_tokens, q_heads, kv_heads, head_dim,
+              _stream(stream))
     _lib.check(fn, st)
 
 
@@ -103,8 +103,8 @@ def launch_attention_decode(q, k_cache, v_cache, block_tables, table_offset, tok
     ws_ptr = _ptr(workspace)
     ws_bytes = workspace.numel() * workspace.element_size() if workspace is not None else 0
     st = call(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables), _ptr(table_offset),
-                                 _ptr(token_seq), _ptr(token_pos), _ptr(out), n_tokens, q_heads, kv_heads,
-                                 head_dim, block_size, C.c_float(scale), ws_ptr, ws_bytes, _stream(stream))
+              _ptr(token_seq), _ptr(token_pos), _ptr(out), n_tokens, q_heads, kv_heads,
+              head_dim, block_size, C.c_float(scale), ws_ptr, ws_bytes, _stream(stream))
     _lib.check(fn, st)
 
 
@@ -121,9 +121,9 @@ def launch_attention_mixed(q, k_cache, v_cache, block_tables, table_offset, toke
     the rest to the decode kernels; the split is made on the device."""
     fn, call = _fn("pkv_mixed_attn_", k_cache)
     st = call(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables), _ptr(table_offset),
-                                 _ptr(token_seq), _ptr(token_pos), _ptr(out), n_tokens, q_heads, kv_heads, head_dim,
-                                 block_size, num_blocks, C.c_float(scale), min_run, _ptr(workspace),
-                                 workspace.numel() * workspace.element_size(), _stream(stream))
+              _ptr(token_seq), _ptr(token_pos), _ptr(out), n_tokens, q_heads, kv_heads, head_dim,
+              block_size, num_blocks, C.c_float(scale), min_run, _ptr(workspace),
+              workspace.numel() * workspace.element_size(), _stream(stream))
     _lib.check(fn, st)
 
 
@@ -213,8 +213,8 @@ class DecodePlan:
         fn, call = _fn("pkv_decode_attn_planned_", k_cache)
         p, n = self._ws()
         st = call(C.byref(self.plan), _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables),
-                                     _ptr(table_offset), _ptr(token_seq), _ptr(token_pos), _ptr(out), block_size,
-                                     C.c_float(scale), p, n, _stream(stream))
+                  _ptr(table_offset), _ptr(token_seq), _ptr(token_pos), _ptr(out), block_size,
+                  C.c_float(scale), p, n, _stream(stream))
         _lib.check(fn, st)
 
     def append_attention(self, q, k, v, slots, k_cache, v_cache, block_tables, table_offset, token_seq, token_pos, out,
@@ -223,8 +223,8 @@ class DecodePlan:
         fn, call = _fn("pkv_append_decode_attn_planned_", k_cache)
         p, n = self._ws()
         st = call(C.byref(self.plan), _ptr(q), _ptr(k), _ptr(v), _ptr(slots), _ptr(k_cache), _ptr(v_cache),
-                                     _ptr(block_tables), _ptr(table_offset), _ptr(token_seq), _ptr(token_pos), _ptr(out),
-                                     block_size, C.c_float(scale), p, n, _stream(stream))
+                  _ptr(block_tables), _ptr(table_offset), _ptr(token_seq), _ptr(token_pos), _ptr(out),
+                  block_size, C.c_float(scale), p, n, _stream(stream))
         _lib.check(fn, st)
 
 
@@ -234,8 +234,8 @@ def launch_attention_prefill(q, k_cache, v_cache, block_tables, table_offset, q_
     """Causal attention of each sequence's new chunk over its cached plus new tokens."""
     fn, call = _fn("pkv_prefill_attn_", k_cache)
     st = call(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables), _ptr(table_offset),
-                                 _ptr(q_start), _ptr(q_len), _ptr(ctx_len), _ptr(out), n_tokens, n_seqs, max_q_len, q_heads,
-                                 kv_heads, head_dim, block_size, num_blocks, C.c_float(scale), _stream(stream))
+              _ptr(q_start), _ptr(q_len), _ptr(ctx_len), _ptr(out), n_tokens, n_seqs, max_q_len, q_heads,
+              kv_heads, head_dim, block_size, num_blocks, C.c_float(scale), _stream(stream))
     _lib.check(fn, st)
 
 
@@ -244,7 +244,7 @@ def launch_copy_blocks(k_cache, v_cache, src_dst_pairs, n_pairs: int, block_size
     """Copy-on-write: block pairs[2i] -> block pairs[2i+1] in both pools."""
     fn, call = _fn("pkv_copy_blocks_", k_cache)
     st = call(_ptr(k_cache), _ptr(v_cache), _ptr(src_dst_pairs), n_pairs, block_size, kv_dim,
-                                 _stream(stream))
+              _stream(stream))
     _lib.check(fn, st)
 
 
