@@ -24,7 +24,7 @@ def test_groups_and_slab_edges(pkv, orc, torch_cuda, qh, kvh, hd, bs):
 
 @pytest.mark.parametrize("hd", [64, 128])
 def test_shares(pkv, orc, torch_cuda, hd):
-    """Enough keys that the plan is cut into one share per warp; more shares than resident warps at 128 dims."""
+    """Enough keys that the plan is cut into one share per resident warp, at both head dims."""
     ctx = [int(x) for x in np.random.default_rng(2).integers(200, 9000, size=40)]
     case = make(orc, pkv, 8, 4, hd, 16, ctx, seed=3)
     for mode in ("host_plan", "device_plan"):
