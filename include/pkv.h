@@ -63,7 +63,7 @@ const char* pkv_last_error(void);
  * launch's output incomplete.  The record of it is a bit -- 1: a TMA producer never saw
  * its ring slot released; 2: a consumer never saw its tile arrive; 4: a prefill
  * pipeline wait; 8: a peer GPU's flag in the head-sharded exchange; 16: a block copy -- kept in two
- * places: a device word, and one pinned host word the kernels store to.  The attention
+ * places: a device word, and a pinned host word the kernels store to.  The attention
  * entry points (pkv_decode_attn_*, the planned, fused, peer and mixed forms,
  * pkv_prefill_attn_*) look at the host word before they enqueue anything, and so do
  * pkv_copy_blocks_* for the bit of an earlier copy: the first

@@ -160,8 +160,9 @@ int copy_impl(TwoPools two, void* const* pools, int n_pools, bool pools_aligned,
     }
     const unsigned blocks = static_cast<unsigned>(std::min<unsigned long long>(tasks, static_cast<unsigned long long>(sms) * kBulkBlocksPerSm));
     auto kern = pools ? copy_blocks_bulk_kernel<true> : copy_blocks_bulk_kernel<false>;
+    unsigned int* mirror = error_mirror(true);
     launch_pdl(kern, dim3(blocks), dim3(32), kBulkStages * kBulkBytes, s, two, pools, pairs, n_pairs, block_bytes, pieces, tasks,
-               error_mirror(true));
+               mirror ? mirror + 1 : nullptr);               // the copies' own word
     return check_launch("copy_blocks_bulk_kernel");
   }
   dim3 grid(static_cast<unsigned>((block_bytes + kCopyThreads * 8 - 1) / (kCopyThreads * 8)), n_pairs, n_pools);

@@ -16,14 +16,15 @@
 namespace pkv {
 namespace {
 std::mutex g_mu;
-unsigned int* g_mirror = nullptr;   // cudaHostAlloc'd (portable, mapped): one word, valid on every device
+unsigned int* g_mirror = nullptr;   // cudaHostAlloc'd (portable, mapped): kWords words, valid on every device
+constexpr int kWords = 2;           // the attention kernels' and the block copies': they store their bit, they do not add it
 bool g_tried = false;
 unsigned int g_plain = 0;           // what pkv_debug_set_reported_flags recorded (works without a device)
 }  // namespace
 
-// The pinned word, created on first use when `create` is set.  The one allocating call this makes
+// The pinned words, created on first use when `create` is set.  The one allocating call this makes
 // (cudaHostAlloc of 64 bytes, once per process) is kept away from callers that must not allocate:
-// they pass create = false and get the word only if somebody else made it already.
+// they pass create = false and get the words only if somebody else made them already.
 unsigned int* error_mirror(bool create) {
   std::lock_guard<std::mutex> lock(g_mu);
   if (g_mirror || !create || g_tried) return g_mirror;
@@ -45,13 +46,15 @@ unsigned int* error_mirror(bool create) {
 
 // Takes those of `bits` that are recorded.
 unsigned int take_error_mirror(unsigned int bits) {
-  // the common case -- nothing recorded -- is two plain loads, no lock and no write
+  // the common case -- nothing recorded -- is three plain loads, no lock and no write
   unsigned int* m = __atomic_load_n(&g_mirror, __ATOMIC_ACQUIRE);
-  if ((__atomic_load_n(&g_plain, __ATOMIC_RELAXED) & bits) == 0 && (!m || (__atomic_load_n(m, __ATOMIC_RELAXED) & bits) == 0)) return 0;
+  unsigned int seen = __atomic_load_n(&g_plain, __ATOMIC_RELAXED);
+  for (int i = 0; m && i < kWords; ++i) seen |= __atomic_load_n(m + i, __ATOMIC_RELAXED);
+  if ((seen & bits) == 0) return 0;
   std::lock_guard<std::mutex> lock(g_mu);
   unsigned int v = g_plain & bits;
   g_plain &= ~bits;
-  if (g_mirror) v |= __atomic_fetch_and(g_mirror, ~bits, __ATOMIC_ACQ_REL) & bits;
+  for (int i = 0; g_mirror && i < kWords; ++i) v |= __atomic_fetch_and(g_mirror + i, ~bits, __ATOMIC_ACQ_REL) & bits;
   return v;
 }
 
