@@ -239,16 +239,15 @@ __global__ void __launch_bounds__(kCombineThreads) decode_combine_kernel(const D
   const int D = a.head_dim;
   const int pairs = a.n_tokens * a.kv_heads;
   // The split record of this block's first (token, kv head) is part of the plan, which was complete
-  // before the attention kernel started: fetch it while that kernel is still finishing.  (Chosen at
-  // run time instead, the two places cost 64 sequences of 256-2,048 keys 0.5 us a layer of 18.6.)
+  // before the attention kernel started: fetch it while that kernel is still finishing.  A plan made
+  // inside the attention kernel is complete only behind the wait.  (Without the run-time test there, which
+  // is never false, the compiler's code for those is 0.2 to 0.6 us an engine step's layer slower; with it in the
+  // other instantiation, 64 sequences of 256-2,048 keys lose 0.5 us a layer of 18.6.)
   TokSplit ts_first{0, 0};
-  if constexpr (!INLINE_PLAN) {
-    if (static_cast<int>(blockIdx.x) < pairs) ts_first = a.tok_split[blockIdx.x / a.kv_heads];
-  }
+  const bool ready = !INLINE_PLAN || a.inline_min_run == 0;
+  if (static_cast<int>(blockIdx.x) < pairs && ready) ts_first = a.tok_split[blockIdx.x / a.kv_heads];
   pdl_wait();  // the attention kernel's partials
-  if constexpr (INLINE_PLAN) {
-    if (static_cast<int>(blockIdx.x) < pairs) ts_first = a.tok_split[blockIdx.x / a.kv_heads];
-  }
+  if (static_cast<int>(blockIdx.x) < pairs && !ready) ts_first = a.tok_split[blockIdx.x / a.kv_heads];
   for (int pr = blockIdx.x; pr < pairs; pr += gridDim.x) {
     const int token = pr / a.kv_heads, kvh = pr - token * a.kv_heads;
     const TokSplit ts = pr == static_cast<int>(blockIdx.x) ? ts_first : a.tok_split[token];
